@@ -67,7 +67,8 @@ extern "C" {
  *         maxwell {mu, epsilon, sigma, rho_c, chi_B, chi_D}.
  * bc_kind/bc_value: [variable][side], sides ordered left,right,bottom,top,front,back
  * (src/solver.py:36).  tile_ty: tile rows, 0 = the default shape (or the alternative
- * one that fvm_tiling reports after fvm_autotune); zchunk: planes per tile, 0 = 64. */
+ * one that fvm_tiling reports after fvm_autotune); zchunk: planes per tile, 0 = an
+ * equal run of planes for every resident block. */
 typedef struct fvm_desc {
   int physics, precision, coords;
   int nx1, nx2, nx3;
@@ -185,7 +186,8 @@ int fvm_profile_steps(fvm_handle* h, int n_steps, int dt_mode, double* stage_ker
  * afterwards.  New: the reference has no tuning. */
 int fvm_autotune(fvm_handle* h, int* best_zchunk, double* best_ms_per_step);
 /* The handle's block shape: tile rows (fvm_desc.tile_ty, or the autotuner's
- * choice) and z-march depth.  New: the reference has no tuning. */
+ * choice) and z-march depth (of the balanced split, the longest run of planes
+ * that a block marches).  New: the reference has no tuning. */
 int fvm_tiling(fvm_handle* h, int* tile_ty, int* zchunk);
 
 /* Sharp Kelvin-Helmholtz initial state written on the device (the host

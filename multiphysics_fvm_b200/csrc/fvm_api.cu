@@ -126,7 +126,7 @@ struct fvm_handle {
   unsigned extra_tx = 0;                       // test of the timeout path (fvm_set_wait_limit)
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   double max_inv_l2 = 0.0, const_rate = 0.0;
-  int zchunk = 64;
+  int zchunk = 0;   // z-march depth, 0: balanced pieces (tile_walk.cuh)
   int tile_ty = 0;  // tile rows of the stage kernel (its tensor maps are built for it)
   long long device_bytes = 0;
   fvm_closure* closure = nullptr;  // learned flux correction run inside every step
@@ -384,7 +384,6 @@ NsParams<Real> make_ns_params(fvm_handle* h, const StageDef& sd, bool rhs_only) 
   p.g2 = d.params[3];
   p.g3 = d.params[4];
   p.flat = (!rhs_only && flat_grid(h)) ? 1 : 0;
-  p.ysub = 1;
   return p;
 }
 
@@ -436,8 +435,9 @@ cudaError_t launch_stage(fvm_handle* h, const StageDef& sd, bool rhs_only, bool 
       src.p = p;
       const int nbuf = (needs_u0_host(sd) ? 1 : 0) + (sd.mode == MODE_FINAL || sd.accmode == ACC_ADD ? 1 : 0);
       return launch_mx_strip(kernel_limiter(d), d.coords, src, h->tile_ty, nbuf, h->stream, nsm);
+    } else {
+      return launch_maxwell<Real>(kernel_limiter(d), d.riemann, d.coords, h->tmap[sd.in], p, h->stream, nsm);
     }
-    return launch_maxwell<Real>(kernel_limiter(d), d.riemann, d.coords, h->tmap[sd.in], p, h->stream, nsm);
   }
   const bool visc = d.params[1] != 0.0;
   if constexpr (std::is_same<Real, float>::value) {
@@ -626,7 +626,7 @@ int fvm_create(const fvm_desc* desc, fvm_handle** out) {
   L.pitch = (row + 31) / 32 * 32;
   L.plane = L.pitch * (L.ny + 2);
   L.var_stride = (L.plane * (L.nz + 2) + 63) / 64 * 64;
-  h->zchunk = d.zchunk > 0 ? d.zchunk : 64;
+  h->zchunk = d.zchunk > 0 ? d.zchunk : 0;
   auto cleanup = [&](int code) { fvm_destroy(h); return code; };
 #define FVM_CKC(x)                                                                                         \
   do {                                                                                                     \
@@ -1179,8 +1179,9 @@ struct fvm_batch {
     std::vector<int> members;
     std::vector<void*> prm;           // device params array per stage
     std::vector<CUtensorMap*> maps;   // device tensor-map array per stage
-    int* tile_start = nullptr;
-    long long ntiles = 0;
+    long long* starts = nullptr;      // prefix sums over the members (tile_walk.cuh)
+    long long ntiles = 0;             // units or pieces of the launch
+    int bal = 1;
   };
   std::vector<Group> groups;
   BatchAux* aux = nullptr;
@@ -1203,34 +1204,42 @@ namespace {
 int build_mixed_arrays(fvm_batch* b, fvm_batch::Group& g) {
   const std::vector<StageDef> st = stage_table(b->integrator);
   for (void* x : g.prm) cudaFree(x);
-  if (g.tile_start) cudaFree(g.tile_start);
+  if (g.starts) cudaFree(g.starts);
   g.prm.clear();
   g.nbuf.clear();
-  g.tile_start = nullptr;
-  std::vector<int> starts(1, 0);
+  g.starts = nullptr;
+  g.ntiles = 0;
+  g.bal = b->h[g.members[0]]->zchunk == 0;
+  std::vector<long long> starts(1, 0);
   for (size_t si = 0; si < st.size(); ++si) {
     std::vector<MixedInst> mi(g.members.size());
     for (size_t k = 0; k < g.members.size(); ++k) {
       fvm_handle* h = b->h[g.members[k]];
       MixedInst& m = mi[k];
       m.tmap = h->tmap[st[si].in];
-      int tiles = 0;
       if (h->d.physics == FVM_NAVIER_STOKES) {
         m.kind = 0;
         m.u0map = h->smap;
         m.accmap = h->amap;
         m.ns = make_ns_params<float>(h, st[si], false);
-        ns_strip_tiles(m.ns, MIX_NS_TY);
-        tiles = m.ns.ntx * m.ns.nty * m.ns.nzc;
+        set_tiles(m.ns, MIX_NS_TY, m.ns.flat != 0);
+        m.ncol = m.ns.ncol;
+        m.nunit = m.ns.nunit;
+        m.zchunk = m.ns.zchunk;
+        m.weight = MIX_NS_COST;
       } else {
         m.kind = 1;
         m.heat = make_heat_params<float>(h, st[si], false);
-        m.heat.ntx = (h->lay.nx + 31) / 32;
-        m.heat.nty = (h->lay.ny + g.heat_ty - 1) / g.heat_ty;
-        m.heat.nzc = (h->lay.nz + m.heat.zchunk - 1) / m.heat.zchunk;
-        tiles = m.heat.ntx * m.heat.nty * m.heat.nzc;
+        set_tiles(m.heat, g.heat_ty);
+        m.ncol = m.heat.ncol;
+        m.nunit = m.heat.nunit;
+        m.zchunk = m.heat.zchunk;
+        m.weight = g.heat_ty == MIX_HEAT_TY ? MIX_HEAT_COST : MIX_HEAT_COST_ALT;
       }
-      if (si == 0) starts.push_back(starts.back() + tiles);
+      if (si == 0) {
+        g.ntiles += tile_total(m);
+        starts.push_back(starts.back() + tile_total(m) * (g.bal ? m.weight : 1));
+      }
     }
     void* dev = nullptr;
     FVM_CK(cudaMalloc(&dev, mi.size() * sizeof(MixedInst)));
@@ -1238,9 +1247,8 @@ int build_mixed_arrays(fvm_batch* b, fvm_batch::Group& g) {
     g.prm.push_back(dev);
     g.nbuf.push_back((needs_u0_host(st[si]) ? 1 : 0) + (st[si].mode == MODE_FINAL || st[si].accmode == ACC_ADD ? 1 : 0));
   }
-  g.ntiles = starts.back();
-  FVM_CK(cudaMalloc(&g.tile_start, starts.size() * sizeof(int)));
-  FVM_CK(cudaMemcpy(g.tile_start, starts.data(), starts.size() * sizeof(int), cudaMemcpyHostToDevice));
+  FVM_CK(cudaMalloc(&g.starts, starts.size() * sizeof(long long)));
+  FVM_CK(cudaMemcpy(g.starts, starts.data(), starts.size() * sizeof(long long), cudaMemcpyHostToDevice));
   return FVM_OK;
 }
 
@@ -1250,11 +1258,13 @@ int build_group_arrays(fvm_batch* b, fvm_batch::Group& g) {
   const std::vector<StageDef> st = stage_table(b->integrator);
   for (void* x : g.prm) cudaFree(x);
   for (CUtensorMap* x : g.maps) cudaFree(x);
-  if (g.tile_start) cudaFree(g.tile_start);
+  if (g.starts) cudaFree(g.starts);
   g.prm.clear();
   g.maps.clear();
-  g.tile_start = nullptr;
-  std::vector<int> starts(1, 0);
+  g.starts = nullptr;
+  g.ntiles = 0;
+  g.bal = b->h[g.members[0]]->zchunk == 0;
+  std::vector<long long> starts(1, 0);
   for (size_t si = 0; si < st.size(); ++si) {
     std::vector<CUtensorMap> maps;
     void* dev = nullptr;
@@ -1262,11 +1272,10 @@ int build_group_arrays(fvm_batch* b, fvm_batch::Group& g) {
       std::vector<NsParams<Real>> ps;
       for (int i : g.members) {
         NsParams<Real> p = make_ns_params<Real>(b->h[i], st[si], false);
-        if (g.visc) ns_tile_counts<Real, true>(p);
-        else ns_tile_counts<Real, false>(p);
+        set_tiles(p, g.visc ? ns_tile_ty<Real, true>() : ns_tile_ty<Real, false>());
         ps.push_back(p);
         maps.push_back(b->h[i]->tmap[st[si].in]);
-        if (si == 0) starts.push_back(starts.back() + p.ntx * p.nty * p.nzc);
+        if (si == 0) starts.push_back(g.ntiles += tile_total(p));
       }
       FVM_CK(cudaMalloc(&dev, ps.size() * sizeof(ps[0])));
       FVM_CK(cudaMemcpy(dev, ps.data(), ps.size() * sizeof(ps[0]), cudaMemcpyHostToDevice));
@@ -1274,10 +1283,10 @@ int build_group_arrays(fvm_batch* b, fvm_batch::Group& g) {
       std::vector<HeatParams<Real>> ps;
       for (int i : g.members) {
         HeatParams<Real> p = make_heat_params<Real>(b->h[i], st[si], false);
-        heat_tile_counts(p);
+        set_tiles(p, HEAT_TY);
         ps.push_back(p);
         maps.push_back(b->h[i]->tmap[st[si].in]);
-        if (si == 0) starts.push_back(starts.back() + p.ntx * p.nty * p.nzc);
+        if (si == 0) starts.push_back(g.ntiles += tile_total(p));
       }
       FVM_CK(cudaMalloc(&dev, ps.size() * sizeof(ps[0])));
       FVM_CK(cudaMemcpy(dev, ps.data(), ps.size() * sizeof(ps[0]), cudaMemcpyHostToDevice));
@@ -1288,9 +1297,8 @@ int build_group_arrays(fvm_batch* b, fvm_batch::Group& g) {
     FVM_CK(cudaMemcpy(dm, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
     g.maps.push_back(dm);
   }
-  g.ntiles = starts.back();
-  FVM_CK(cudaMalloc(&g.tile_start, starts.size() * sizeof(int)));
-  FVM_CK(cudaMemcpy(g.tile_start, starts.data(), starts.size() * sizeof(int), cudaMemcpyHostToDevice));
+  FVM_CK(cudaMalloc(&g.starts, starts.size() * sizeof(long long)));
+  FVM_CK(cudaMemcpy(g.starts, starts.data(), starts.size() * sizeof(long long), cudaMemcpyHostToDevice));
   return FVM_OK;
 }
 
@@ -1298,17 +1306,17 @@ template <typename Real>
 cudaError_t launch_group_stage(fvm_batch* b, fvm_batch::Group& g, int si, int nsm) {
   if (g.mixed) {
     const int nbuf = g.nbuf[si];
-    const MixedSource src{static_cast<const MixedInst*>(g.prm[si]), g.tile_start, (int)g.members.size(),
+    const MixedSource src{static_cast<const MixedInst*>(g.prm[si]), g.starts, (int)g.members.size(), g.bal,
                           mixed_bar_offset(nbuf)};
     return launch_mixed(g.lim, g.riem, g.coords, g.heat_ty, src, g.ntiles, nbuf, b->stream, nsm);
   }
   if (g.physics == FVM_NAVIER_STOKES) {
-    BatchSource<NsParams<Real>> src{static_cast<const NsParams<Real>*>(g.prm[si]), g.maps[si], g.tile_start,
-                                    (int)g.members.size()};
+    BatchSource<NsParams<Real>> src{static_cast<const NsParams<Real>*>(g.prm[si]), g.maps[si], g.starts,
+                                    (int)g.members.size(), g.bal};
     return launch_ns_batch<Real>(g.lim, g.riem, g.coords, g.visc, src, g.ntiles, b->stream, nsm);
   }
-  BatchSource<HeatParams<Real>> src{static_cast<const HeatParams<Real>*>(g.prm[si]), g.maps[si], g.tile_start,
-                                    (int)g.members.size()};
+  BatchSource<HeatParams<Real>> src{static_cast<const HeatParams<Real>*>(g.prm[si]), g.maps[si], g.starts,
+                                    (int)g.members.size(), g.bal};
   return launch_heat_batch<Real>(g.lim, g.coords, src, g.ntiles, b->stream, nsm);
 }
 
@@ -1392,7 +1400,7 @@ int fvm_batch_destroy(fvm_batch* b) {
   for (auto& g : b->groups) {
     for (void* x : g.prm) cudaFree(x);
     for (CUtensorMap* x : g.maps) cudaFree(x);
-    if (g.tile_start) cudaFree(g.tile_start);
+    if (g.starts) cudaFree(g.starts);
   }
   for (auto& dg : b->dtg) {
     if (dg.d) cudaFree(dg.d);
@@ -1621,12 +1629,14 @@ int fvm_batch_time_steps(fvm_batch* b, int n_steps, int dt_mode, double* ms) {
 // of the coalesced 128-byte rows are fixed per kernel specialisation.
 namespace {
 
-// Depths: a fixed ladder plus ceil(nz / c) for every chunk count c (equal
-// chunks).  The persistent grid deals tiles round-robin, so a launch takes
-// ceil(tiles / resident blocks) tile times; some chunk count puts the tile
-// count just under a whole number of waves, and timing finds it.
+// Depths: balanced pieces (0, tile_walk.cuh), a fixed ladder, and ceil(nz / c)
+// for every chunk count c (equal chunks).  Fixed-depth pieces are dealt
+// round-robin, so a launch takes ceil(pieces / resident blocks) piece times;
+// some chunk count puts the piece count just under a whole number of waves,
+// and timing finds it.
 std::vector<int> zchunk_candidates(int nz) {
   std::vector<int> c;
+  c.push_back(0);  // balanced pieces
   for (int z : {8, 16, 32, 48, 64, 96, 128, 192, 256})
     if (z < nz) c.push_back(z);
   c.push_back(nz);
@@ -1634,6 +1644,18 @@ std::vector<int> zchunk_candidates(int nz) {
   std::sort(c.begin(), c.end());
   c.erase(std::unique(c.begin(), c.end()), c.end());
   return c;
+}
+
+// The z-march depth a handle reports: its fixed one, or the longest run of
+// planes that the balanced split gives a block.
+int reported_depth(fvm_handle* h) {
+  if (h->zchunk > 0) return h->zchunk;
+  StageDef sd{0, 1, MODE_RHS, ACC_NONE, 0, 0, 0};
+  const cudaError_t e = h->f64 ? launch_stage<double>(h, sd, true, true) : launch_stage<float>(h, sd, true, true);
+  if (e != cudaSuccess) return h->d.nx3;
+  const long long units = (long long)((h->lay.nx + 31) / 32) * ((h->lay.ny + h->tile_ty - 1) / h->tile_ty) * h->lay.nz;
+  const long long blocks = std::max(1LL, std::min(units, (long long)prepared_blocks * h->nsm));
+  return (int)std::min<long long>(h->d.nx3, (units + blocks - 1) / blocks);
 }
 
 struct Saved {
@@ -1703,7 +1725,7 @@ int fvm_autotune(fvm_handle* h, int* best_zchunk, double* best_ms) {
   if (rc) return rc;
   if (rr) return rr;
   if (rt) return rt;
-  if (best_zchunk) *best_zchunk = best;
+  if (best_zchunk) *best_zchunk = reported_depth(h);
   if (best_ms) *best_ms = bt / 3.0;
   return FVM_OK;
 }
@@ -1711,7 +1733,7 @@ int fvm_autotune(fvm_handle* h, int* best_zchunk, double* best_ms) {
 int fvm_tiling(fvm_handle* h, int* tile_ty, int* zchunk) {
   if (!h) return fail(FVM_E_INVALID, "null handle");
   if (tile_ty) *tile_ty = h->tile_ty;
-  if (zchunk) *zchunk = h->zchunk;
+  if (zchunk) *zchunk = reported_depth(h);
   return FVM_OK;
 }
 
@@ -1769,7 +1791,7 @@ int fvm_batch_autotune(fvm_batch* b, int* best_zchunk, double* best_ms) {
   if (rc) return rc;
   if (rr) return rr;
   if (ra) return ra;
-  if (best_zchunk) *best_zchunk = best;
+  if (best_zchunk) *best_zchunk = best ? best : nzmax;
   if (best_ms) *best_ms = bt / 3.0;
   return FVM_OK;
 }

@@ -2,9 +2,7 @@
 #include "launch.cuh"
 namespace fvm {
 cudaError_t launch_heat_pc(int coord, const CUtensorMap& map, HeatParams<float> p, cudaStream_t s, int nsm, int ty) {
-  p.ntx = (p.lay.nx + 31) / 32;
-  p.nty = (p.lay.ny + ty - 1) / ty;
-  p.nzc = (p.lay.nz + p.zchunk - 1) / p.zchunk;
+  set_tiles(p, ty);
 #define FVM_HEAT_PC_CASE(CO)                                                                     \
   if (coord == CO)                                                                               \
     return ty == HEAT_PC_TY_ALT    ? launch_heat_pc_ty<CO, HEAT_PC_TY_ALT>(map, p, s, nsm)     \

@@ -2,10 +2,7 @@
 #include "launch.cuh"
 namespace fvm {
 cudaError_t launch_mx_strip(int lim, int coord, MxStripSource& src, int ty, int nbuf, cudaStream_t s, int nsm) {
-  MaxwellParams<float>& p = src.p;
-  p.ntx = (p.lay.nx + 31) / 32;
-  p.nty = (p.lay.ny + ty - 1) / ty;
-  p.nzc = (p.lay.nz + p.zchunk - 1) / p.zchunk;
+  set_tiles(src.p, ty);
 #define FVM_MX_CASE(L, CO)                                                                          \
   if (lim == L && coord == CO)                                                                      \
     return ty == MX_STRIP_TY_ALT ? launch_mx_strip_ty<L, CO, MX_STRIP_TY_ALT>(src, nbuf, s, nsm)   \

@@ -29,6 +29,10 @@ constexpr int ns_min_blocks() {
 }
 constexpr int HEAT_TY = 8, HEAT_TY_ALT = 4;
 
+// Resident blocks per SM of the kernel that prepare_kernel last looked at on
+// this thread (of a kernel with several shared-memory sizes, its largest).
+inline thread_local int prepared_blocks = 0;
+
 template <typename K>
 static cudaError_t prepare_kernel(K kern, int threads, int bytes, int* blocks_per_sm) {
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
@@ -40,6 +44,7 @@ static cudaError_t prepare_kernel(K kern, int threads, int bytes, int* blocks_pe
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kern, threads, bytes);
   if (e != cudaSuccess) return e;
   if (*blocks_per_sm < 1) return cudaErrorInvalidConfiguration;
+  prepared_blocks = *blocks_per_sm;
   return cudaSuccess;
 }
 
@@ -61,13 +66,6 @@ cudaError_t launch_ns_src(const Src& src, long long ntiles, cudaStream_t s, int 
   return cudaGetLastError();
 }
 
-template <typename Real, bool VISC>
-void ns_tile_counts(NsParams<Real>& p, int ty = ns_tile_ty<Real, VISC>()) {
-  p.ntx = (p.lay.nx + 31) / 32;
-  p.nty = (p.lay.ny + ty - 1) / ty;
-  p.nzc = p.flat ? 1 : (p.lay.nz + p.zchunk - 1) / p.zchunk;
-}
-
 // ty: tile rows of the handle (its tensor maps were built for it).
 template <typename Real, int LIM, int RIEM, int COORD, bool VISC>
 cudaError_t launch_ns_one(const CUtensorMap& map, NsParams<Real> p, cudaStream_t s, int nsm, int ty) {
@@ -76,15 +74,15 @@ cudaError_t launch_ns_one(const CUtensorMap& map, NsParams<Real> p, cudaStream_t
   src.tmap = map;
   if constexpr (TA != TD) {
     if (ty == TA) {
-      ns_tile_counts<Real, VISC>(p, TA);
+      set_tiles(p, TA);
       src.p = p;
       return launch_ns_src<Real, LIM, RIEM, COORD, VISC, SingleSource<NsParams<Real>>, TA>(
-          src, (long long)p.ntx * p.nty * p.nzc, s, nsm);
+          src, tile_total(p), s, nsm);
     }
   }
-  ns_tile_counts<Real, VISC>(p, TD);
+  set_tiles(p, TD);
   src.p = p;
-  return launch_ns_src<Real, LIM, RIEM, COORD, VISC>(src, (long long)p.ntx * p.nty * p.nzc, s, nsm);
+  return launch_ns_src<Real, LIM, RIEM, COORD, VISC>(src, tile_total(p), s, nsm);
 }
 
 template <typename Real, int COORD>
@@ -176,27 +174,17 @@ cudaError_t launch_ns_strip_ty(const NsStripSource& src, int nbuf, cudaStream_t 
     }
   }
   if (nsm < 0) return cudaSuccess;
-  const long long ntiles = (long long)src.p.ntx * src.p.nty * src.p.nzc;
+  const long long ntiles = tile_total(src.p);
   if (ntiles <= 0) return cudaSuccess;
   const int grid = (int)(ntiles < (long long)bps[nbuf] * nsm ? ntiles : (long long)bps[nbuf] * nsm);
   kern<<<grid, C::NT, C::bytes(nbuf), s>>>(src);
   return cudaGetLastError();
 }
 
-// Row tiles a flat tile marches over along x2 (stage_ns_strip.cuh).
-constexpr int NS_FLAT_YSUB = 4;
-// Tile counts of the register-blocked kernel for block rows ty.
-inline void ns_strip_tiles(NsParams<float>& p, int ty) {
-  p.ntx = (p.lay.nx + 31) / 32;
-  p.ysub = p.flat ? NS_FLAT_YSUB : 1;
-  p.nty = ((p.lay.ny + ty - 1) / ty + p.ysub - 1) / p.ysub;
-  p.nzc = (p.lay.nz + p.zchunk - 1) / p.zchunk;
-}
-
 template <int LIM, int RIEM>
 cudaError_t launch_ns_strip_lr(NsStripSource& src, int ty, int nbuf, cudaStream_t s, int nsm) {
   NsParams<float>& p = src.p;
-  ns_strip_tiles(p, ty);
+  set_tiles(p, ty, p.flat != 0);
   if (ty == NS_STRIP_TY_ALT) return launch_ns_strip_ty<LIM, RIEM, NS_STRIP_TY_ALT>(src, nbuf, s, nsm);
   return launch_ns_strip_ty<LIM, RIEM, NS_STRIP_TY>(src, nbuf, s, nsm);
 }
@@ -224,7 +212,7 @@ cudaError_t launch_ns_strip_visc_ty(const NsStripSource& src, int nbuf, cudaStre
     }
   }
   if (nsm < 0) return cudaSuccess;
-  const long long ntiles = (long long)src.p.ntx * src.p.nty * src.p.nzc;
+  const long long ntiles = tile_total(src.p);
   if (ntiles <= 0) return cudaSuccess;
   const int grid = (int)(ntiles < (long long)bps[nbuf] * nsm ? ntiles : (long long)bps[nbuf] * nsm);
   kern<<<grid, C::NT, C::bytes(nbuf), s>>>(src);
@@ -234,10 +222,7 @@ cudaError_t launch_ns_strip_visc_ty(const NsStripSource& src, int nbuf, cudaStre
 template <int LIM, int RIEM>
 cudaError_t launch_ns_strip_visc_lr(NsStripSource& src, int ty, int nbuf, cudaStream_t s, int nsm) {
   NsParams<float>& p = src.p;
-  p.ntx = (p.lay.nx + 31) / 32;
-  p.nty = (p.lay.ny + ty - 1) / ty;
-  p.nzc = (p.lay.nz + p.zchunk - 1) / p.zchunk;
-  (void)ty;
+  set_tiles(p, ty);
   return launch_ns_strip_visc_ty<LIM, RIEM, NS_STRIP_VISC_TY>(src, nbuf, s, nsm);
 }
 
@@ -257,13 +242,6 @@ cudaError_t launch_heat_src(const Src& src, long long ntiles, cudaStream_t s, in
   const int grid = (int)(ntiles < (long long)bps * nsm ? ntiles : (long long)bps * nsm);
   kern<<<grid, C::NT, C::BYTES, s>>>(src);
   return cudaGetLastError();
-}
-
-template <typename Real>
-void heat_tile_counts(HeatParams<Real>& p, int ty = HEAT_TY) {
-  p.ntx = (p.lay.nx + 31) / 32;
-  p.nty = (p.lay.ny + ty - 1) / ty;
-  p.nzc = (p.lay.nz + p.zchunk - 1) / p.zchunk;
 }
 
 template <typename Real, class Src, int TY = HEAT_TY>
@@ -298,7 +276,7 @@ cudaError_t launch_heat_pc_ty(const CUtensorMap& map, const HeatParams<float>& p
     if (e != cudaSuccess) return e;
   }
   if (nsm < 0) return cudaSuccess;
-  const long long ntiles = (long long)p.ntx * p.nty * p.nzc;
+  const long long ntiles = tile_total(p);
   if (ntiles <= 0) return cudaSuccess;
   const int grid = (int)(ntiles < (long long)bps * nsm ? ntiles : (long long)bps * nsm);
   kern<<<grid, C::NT, C::BYTES, s>>>(map, p);
@@ -343,15 +321,15 @@ cudaError_t launch_heat(int lim, int coord, const CUtensorMap& map, const HeatPa
   src.tmap = map;
   if constexpr (std::is_same<Real, float>::value) {
     if (ty == HEAT_TY_ALT) {
-      heat_tile_counts(p, HEAT_TY_ALT);
+      set_tiles(p, HEAT_TY_ALT);
       src.p = p;
       return launch_heat_any<Real, SingleSource<HeatParams<Real>>, HEAT_TY_ALT>(
-          lim, coord, src, (long long)p.ntx * p.nty * p.nzc, s, nsm);
+          lim, coord, src, tile_total(p), s, nsm);
     }
   }
-  heat_tile_counts(p);
+  set_tiles(p, HEAT_TY);
   src.p = p;
-  return launch_heat_any<Real>(lim, coord, src, (long long)p.ntx * p.nty * p.nzc, s, nsm);
+  return launch_heat_any<Real>(lim, coord, src, tile_total(p), s, nsm);
 }
 template <typename Real>
 cudaError_t launch_heat_batch(int lim, int coord, const BatchSource<HeatParams<Real>>& src, long long ntiles,
@@ -383,10 +361,8 @@ cudaError_t launch_maxwell_one(const CUtensorMap& map, MaxwellParams<Real> p, cu
     if (e != cudaSuccess) return e;
   }
   if (nsm < 0) return cudaSuccess;
-  p.ntx = (p.lay.nx + C::TX - 1) / C::TX;
-  p.nty = (p.lay.ny + TY - 1) / TY;
-  p.nzc = (p.lay.nz + p.zchunk - 1) / p.zchunk;
-  const long long ntiles = (long long)p.ntx * p.nty * p.nzc;
+  set_tiles(p, TY);
+  const long long ntiles = tile_total(p);
   const int grid = (int)(ntiles < (long long)bps * nsm ? ntiles : (long long)bps * nsm);
   kern<<<grid, C::NT, C::BYTES, s>>>(map, p);
   return cudaGetLastError();
@@ -408,9 +384,6 @@ cudaError_t launch_maxwell_coord(int lim, int riem, const CUtensorMap& map, cons
 #define FVM_DECLARE_MX(REAL, COORD)                                                                      \
   extern template cudaError_t launch_maxwell_coord<REAL, COORD>(int, int, const CUtensorMap&,           \
                                                                const MaxwellParams<REAL>&, cudaStream_t, int);
-FVM_DECLARE_MX(float, COORD_CART)
-FVM_DECLARE_MX(float, COORD_CYL)
-FVM_DECLARE_MX(float, COORD_SPH)
 FVM_DECLARE_MX(double, COORD_CART)
 FVM_DECLARE_MX(double, COORD_CYL)
 FVM_DECLARE_MX(double, COORD_SPH)
@@ -440,7 +413,7 @@ cudaError_t launch_mx_strip_ty(const MxStripSource& src, int nbuf, cudaStream_t 
     }
   }
   if (nsm < 0) return cudaSuccess;
-  const long long ntiles = (long long)src.p.ntx * src.p.nty * src.p.nzc;
+  const long long ntiles = tile_total(src.p);
   if (ntiles <= 0) return cudaSuccess;
   const int grid = (int)(ntiles < (long long)bps[nbuf] * nsm ? ntiles : (long long)bps[nbuf] * nsm);
   kern<<<grid, C::NT, C::bytes(nbuf), s>>>(src);

@@ -19,6 +19,11 @@ constexpr int MIX_NS_R = 2, MIX_NS_NW = 4;  // Navier-Stokes: 2-row strips, 8-ro
 constexpr int MIX_HEAT_NW = 5;              // heat: 4-row strips (20-row tiles) or 2-row (10-row tiles)
 constexpr int MIX_NT = 160;
 constexpr int MIX_NBAR = 7;
+// Relative cost of a unit in the balanced split of the launch: a Navier-Stokes
+// plane (or row tile) of 32 x 8 cells against a heat plane of 32 x 20 (or 32 x
+// 10).  Step of 64 + 32 grids (12,275 and 40,085 units) at 1:1, 3:2, 2:1, 5:2,
+// 3:1 and 4:1: 2112, 1731, 1533, 1484, 1560 and 1728 us.
+constexpr int MIX_NS_COST = 5, MIX_HEAT_COST = 2, MIX_HEAT_COST_ALT = 1;
 constexpr int MIX_NS_TY = MIX_NS_R * MIX_NS_NW, MIX_HEAT_TY = 4 * MIX_HEAT_NW, MIX_HEAT_TY_ALT = 2 * MIX_HEAT_NW;
 static_assert(NsStripCfg<MIX_NS_R, MIX_NS_NW>::NT == MIX_NT && HeatPcCfg<4, MIX_HEAT_NW>::NT == MIX_NT,
               "both bodies run on the same block");
@@ -40,13 +45,21 @@ struct alignas(64) MixedInst {
   NsParams<float> ns;
   HeatParams<float> heat;
   int kind;  // 0 Navier-Stokes, 1 heat
+  int ncol, nunit, zchunk, weight;  // tile_walk.cuh; weight: relative cost of a unit
 };
 
 struct MixedSource {
-  const MixedInst* inst;  // per grid, this stage
-  const int* tile_start;  // ninst + 1 prefix sums of tiles
+  const MixedInst* inst;    // per grid, this stage
+  const long long* starts;  // ninst + 1 prefix sums of unit costs (or pieces)
   int ninst;
-  int bar_off;            // byte offset of the barriers in shared memory
+  int bal;                  // the launch is balanced (depth 0)
+  int bar_off;              // byte offset of the barriers in shared memory
+  __device__ __forceinline__ bool balanced() const { return bal != 0; }
+  __device__ __forceinline__ long long total() const { return __ldg(starts + ninst); }
+  __device__ __forceinline__ int instance(long long pos) const { return find_instance(starts, ninst, pos); }
+  __device__ __forceinline__ long long start(int i) const { return __ldg(starts + i); }
+  __device__ __forceinline__ const MixedInst& params(int i) const { return inst[i]; }
+  __device__ __forceinline__ int weight(int i) const { return inst[i].weight; }
 };
 
 // HR: heat rows per strip (4: 20-row heat tiles, 2: 10-row).
@@ -68,30 +81,19 @@ __global__ void __launch_bounds__(MIX_NT, 3) batch_mixed_kernel(const __grid_con
   }
   __syncthreads();
   unsigned phase_bits = 0, pending = 0;
-  const int ntiles = __ldg(src.tile_start + src.ninst);
+  TileWalk<MixedSource> walk(src);
+  Piece pc;
+  int inst;
   bool ok = true;
-  for (int gtile = blockIdx.x; gtile < ntiles; gtile += gridDim.x) {
-    int lo = 0, hi = src.ninst - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (__ldg(src.tile_start + mid) <= gtile) lo = mid;
-      else hi = mid - 1;
-    }
-    const MixedInst& in = src.inst[lo];
-    const int tile = gtile - __ldg(src.tile_start + lo);
+  while (ok && walk.next(src, inst, pc)) {
+    const MixedInst& in = src.inst[inst];
     if (in.kind == 0) {
       if (in.ns.active && !*in.ns.active) continue;  // this grid's clock passed t_end
-      if (!ns_strip_tile<LIM, RIEM, MIX_NS_R, MIX_NS_NW>(in.ns, &in.tmap, &in.u0map, &in.accmap, tile, smem_raw,
-                                                         bars, bars + 6, 6, phase_bits, pending)) {
-        ok = false;
-        break;
-      }
+      ok = ns_strip_tile<LIM, RIEM, MIX_NS_R, MIX_NS_NW>(in.ns, &in.tmap, &in.u0map, &in.accmap, pc, smem_raw, bars,
+                                                         bars + 6, 6, phase_bits, pending);
     } else {
       if (in.heat.active && !*in.heat.active) continue;
-      if (!heat_pc_tile<HCOORD, HR, MIX_HEAT_NW, true>(in.heat, &in.tmap, tile, smem_raw, bars, phase_bits, pending)) {
-        ok = false;
-        break;
-      }
+      ok = heat_pc_tile<HCOORD, HR, MIX_HEAT_NW, true>(in.heat, &in.tmap, pc, smem_raw, bars, phase_bits, pending);
     }
   }
   // On a timeout, wait (bounded) for every copy this block may still have in flight.

@@ -25,7 +25,8 @@ struct HeatParams {
   StageCoef coef;
   double rho_cp, k, q, inv_rho_cp;
   unsigned* status;
-  int zchunk, ntx, nty, nzc;
+  int zchunk, ntx, nty;  // zchunk 0: balanced pieces (tile_walk.cuh)
+  int ncol, nunit;
   unsigned long long wait_ns;  // limit of each wait for a TMA plane (ns)
   unsigned long long drain_ns;  // limit of the wait for copies in flight after a timeout (ns)
   unsigned extra_tx;  // test of the timeout path: bytes a ring copy never delivers (0 normally)
@@ -89,22 +90,21 @@ __global__ void __launch_bounds__(HeatCfg<Real, LIM, TY>::NT, 1)
 
   const bool is_out = tid < TX * TY;
   const int otx = tid % TX, oty = tid / TX;
-  const int ntiles = src.total();
+  TileWalk<Src> walk(src);
+  Piece pc;
+  int inst;
   bool ok = true;
-  for (int gtile = blockIdx.x; gtile < ntiles && ok; gtile += gridDim.x) {
-    const int inst = src.instance(gtile);
+  while (ok && walk.next(src, inst, pc)) {
     const HeatParams<Real>& p = src.params(inst);
     if (p.active && !*p.active) continue;  // this grid's clock passed t_end
     const CUtensorMap* tmap = src.map(inst);
-    const int tile = src.local(gtile, inst);
     const Layout& L = p.lay;
     const int nx = L.nx, ny = L.ny, nz = L.nz;
     const Real rcp = Real(p.rho_cp), kk = Real(p.k), qsrc = Real(p.q), ircp = Real(p.inv_rho_cp);
     const Real dt = Real(*p.dt);
     if (tid == 0) tma_prefetch_desc(tmap);
-    const int x0 = (tile % p.ntx) * TX, y0 = ((tile / p.ntx) % p.nty) * TY;
-    const int Z0 = 1 + (tile / (p.ntx * p.nty)) * p.zchunk;
-    const int Zl = min(Z0 + p.zchunk - 1, nz);
+    const int x0 = (pc.col % p.ntx) * TX, y0 = (pc.col / p.ntx) * TY;
+    const int Z0 = 1 + pc.u0, Zl = pc.u1;
     const int Pfirst = Z0 - HH, Plast = Zl + HH, Kfirst = Z0 - 2 * HH;
     const int oi = x0 + otx, oj = y0 + oty;
     const bool out_valid = is_out && oi < nx && oj < ny;

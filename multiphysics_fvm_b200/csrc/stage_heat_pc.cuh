@@ -33,7 +33,7 @@ struct HeatPcCfg {
   static_assert((SLOT * 4) % 128 == 0, "TMA destinations need 128-byte alignment");
 };
 
-// One tile of the stage (all planes of its z-chunk) with the ring barriers
+// One piece of the stage (a run of planes of one tile column) with the ring barriers
 // `bars` (phase bits 0..5); `phase_bits` and `pending` carry over from tile to
 // tile.  Returns false when a wait ran out: the block must stop and drain.
 // MERGED: the two warm-up steps of the z-march (phi3 of planes Z0-1 and Z0)
@@ -41,7 +41,7 @@ struct HeatPcCfg {
 // batched launch); a single-grid launch of one wave of long chunks ran 2 %
 // slower with it.
 template <int COORD, int R, int NW, bool MERGED = false>
-__device__ __forceinline__ bool heat_pc_tile(const HeatParams<float>& p, const CUtensorMap* tmap, int tile,
+__device__ __forceinline__ bool heat_pc_tile(const HeatParams<float>& p, const CUtensorMap* tmap, const Piece& pc,
                                              unsigned char* smem_raw, uint64_t* bars, unsigned& phase_bits,
                                              unsigned& pending) {
   using C = HeatPcCfg<R, NW>;
@@ -58,9 +58,8 @@ __device__ __forceinline__ bool heat_pc_tile(const HeatParams<float>& p, const C
   const bool need_acc = needs_acc(p.coef);
   const int w = tid >> 5, lane = tid & 31;
   {
-    const int x0 = (tile % p.ntx) * TX, y0 = ((tile / p.ntx) % p.nty) * TY;
-    const int Z0 = 1 + (tile / (p.ntx * p.nty)) * p.zchunk;
-    const int Zl = min(Z0 + p.zchunk - 1, nz);
+    const int x0 = (pc.col % p.ntx) * TX, y0 = (pc.col / p.ntx) * TY;
+    const int Z0 = 1 + pc.u0, Zl = pc.u1;
     const int Kfirst = Z0 - 2, Plast = Zl + 2;
     const int i = x0 + lane, jb = y0 + w * R;
     const bool icol = i < nx;
@@ -256,13 +255,12 @@ __global__ void __launch_bounds__(HeatPcCfg<R, NW>::NT)
   }
   __syncthreads();
   unsigned phase_bits = 0, pending = 0;
-  const int ntiles = p.ntx * p.nty * p.nzc;
+  const OneGrid<HeatParams<float>> grid{p};
+  TileWalk<OneGrid<HeatParams<float>>> walk(grid);
+  Piece pc;
+  int inst;
   bool ok = true;
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
-    if (!heat_pc_tile<COORD, R, NW>(p, &tmap, tile, smem_raw, bars, phase_bits, pending)) {
-      ok = false;
-      break;
-    }
+  while (ok && walk.next(grid, inst, pc)) ok = heat_pc_tile<COORD, R, NW>(p, &tmap, pc, smem_raw, bars, phase_bits, pending);
   if (!ok && tid == 0)
     for (int s = 0; s < C::NSLOT; ++s)
       if ((pending >> s) & 1u) mbar_wait_bounded(&bars[s], (phase_bits >> s) & 1u, p.drain_ns);

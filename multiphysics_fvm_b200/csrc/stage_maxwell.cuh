@@ -27,7 +27,8 @@ struct MaxwellParams {
   StageCoef coef;
   double mu, ep, sigma, rho_c, chi_b, chi_d, c;
   unsigned* status;
-  int zchunk, ntx, nty, nzc;
+  int zchunk, ntx, nty;  // zchunk 0: balanced pieces (tile_walk.cuh)
+  int ncol, nunit;
   unsigned long long wait_ns;  // limit of each wait for a TMA plane (ns)
   unsigned long long drain_ns;  // limit of the wait for copies in flight after a timeout (ns)
   unsigned extra_tx;  // test of the timeout path: bytes a ring copy never delivers (0 normally)
@@ -146,12 +147,14 @@ __global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, MINB)
 
   const bool is_out = tid < TX * TY;
   const int otx = tid % TX, oty = tid / TX;
-  const int ntiles = p.ntx * p.nty * p.nzc;
+  const OneGrid<MaxwellParams<Real>> grid{p};
+  TileWalk<OneGrid<MaxwellParams<Real>>> walk(grid);
+  Piece pc;
+  int inst;
   bool ok = true;
-  for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-    const int x0 = (tile % p.ntx) * TX, y0 = ((tile / p.ntx) % p.nty) * TY;
-    const int Z0 = 1 + (tile / (p.ntx * p.nty)) * p.zchunk;
-    const int Zl = min(Z0 + p.zchunk - 1, nz);
+  while (ok && walk.next(grid, inst, pc)) {
+    const int x0 = (pc.col % p.ntx) * TX, y0 = (pc.col / p.ntx) * TY;
+    const int Z0 = 1 + pc.u0, Zl = pc.u1;
     const int Pfirst = Z0 - HH, Plast = Zl + HH, Kfirst = Z0 - 2 * HH;
     const int oi = x0 + otx, oj = y0 + oty;
     const bool out_valid = is_out && oi < nx && oj < ny;

@@ -173,12 +173,14 @@ __global__ void __launch_bounds__(MxStripCfg<R, NW>::NT, MINB)
     }
   };
 
-  const int ntiles = p.ntx * p.nty * p.nzc;
+  const OneGrid<MaxwellParams<float>> grid{p};
+  TileWalk<OneGrid<MaxwellParams<float>>> walk(grid);
+  Piece pc;
+  int inst;
   bool ok = true;
-  for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-    const int x0 = (tile % p.ntx) * TX, y0 = ((tile / p.ntx) % p.nty) * TY;
-    const int Z0 = 1 + (tile / (p.ntx * p.nty)) * p.zchunk;
-    const int Zl = min(Z0 + p.zchunk - 1, nz);
+  while (ok && walk.next(grid, inst, pc)) {
+    const int x0 = (pc.col % p.ntx) * TX, y0 = (pc.col / p.ntx) * TY;
+    const int Z0 = 1 + pc.u0, Zl = pc.u1;
     const int Kfirst = Z0 - 2, Plast = Zl + HH;
     const int i = x0 + lane, jb = y0 + w * R;
     const int ic = min(i, nx - 1);

@@ -17,6 +17,7 @@
 // HH = 3 with viscosity (tau at K+2 needs v at K+3), 2 without.
 #pragma once
 #include "fvm_common.cuh"
+#include "tile_walk.cuh"
 
 namespace fvm {
 
@@ -32,45 +33,12 @@ struct NsParams {
   StageCoef coef;
   double gamma, mu, g1, g2, g3;
   unsigned* status;
-  int zchunk, ntx, nty, nzc;
+  int zchunk, ntx, nty;  // zchunk 0: balanced pieces (tile_walk.cuh)
+  int ncol, nunit;
   int flat;  // nx3 == 1 with x3 ghosts equal to the plane: x3 fluxes cancel, no z-march
-  int ysub;  // register-blocked kernel, flat grids: row tiles a tile marches over along x2
   unsigned long long wait_ns;  // limit of each wait for a TMA plane (ns)
   unsigned long long drain_ns;  // limit of the wait for copies in flight after a timeout (ns)
   unsigned extra_tx;  // test of the timeout path: bytes a ring copy never delivers (0 normally)
-};
-
-// Tile sources: one grid (params + tensor map in kernel parameter space) or a
-// batch of independent grids (per-instance params and maps in global memory,
-// one flat tile list, instance found by binary search over tile offsets).
-template <class P>
-struct SingleSource {
-  CUtensorMap tmap;
-  P p;
-  __device__ __forceinline__ int total() const { return p.ntx * p.nty * p.nzc; }
-  __device__ __forceinline__ int instance(int) const { return 0; }
-  __device__ __forceinline__ const P& params(int) const { return p; }
-  __device__ __forceinline__ const CUtensorMap* map(int) const { return &tmap; }
-  __device__ __forceinline__ int local(int g, int) const { return g; }
-};
-template <class P>
-struct BatchSource {
-  const P* prm;             // per instance (this stage)
-  const CUtensorMap* maps;  // per instance: map of this stage's input buffer
-  const int* tile_start;    // ninst+1 prefix sums of tiles
-  int ninst;
-  __device__ __forceinline__ int total() const { return __ldg(tile_start + ninst); }
-  __device__ __forceinline__ int instance(int g) const {
-    int lo = 0, hi = ninst - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (__ldg(tile_start + mid) <= g) lo = mid; else hi = mid - 1;
-    }
-    return lo;
-  }
-  __device__ __forceinline__ const P& params(int i) const { return prm[i]; }
-  __device__ __forceinline__ const CUtensorMap* map(int i) const { return maps + i; }
-  __device__ __forceinline__ int local(int g, int i) const { return g - __ldg(tile_start + i); }
 };
 
 constexpr int cmax(int a, int b) { return a > b ? a : b; }
@@ -229,26 +197,22 @@ __global__ void __launch_bounds__(NsCfg<Real, VISC, TY>::NT, MINB)
   const bool is_out = tid < TX * TY;
   const int otx = tid % TX, oty = tid / TX;
 
-  const int ntiles = src.total();
+  TileWalk<Src> walk(src);
+  Piece pc;
+  int inst;
   bool ok = true;
-  for (int gtile = blockIdx.x; gtile < ntiles && ok; gtile += gridDim.x) {
-    const int inst = src.instance(gtile);
+  while (ok && walk.next(src, inst, pc)) {
     const NsParams<Real>& p = src.params(inst);
     if (p.active && !*p.active) continue;  // this grid's clock passed t_end
     const CUtensorMap* tmap = src.map(inst);
-    const int tile = src.local(gtile, inst);
     const Layout& L = p.lay;
     const int nx = L.nx, ny = L.ny, nz = L.nz;
     const Real gam = Real(p.gamma), mu = Real(p.mu);
     const Real dt = Real(*p.dt);
     const bool flat = p.flat != 0;
     if (tid == 0) tma_prefetch_desc(tmap);
-    const int tx_i = tile % p.ntx;
-    const int ty_i = (tile / p.ntx) % p.nty;
-    const int zc_i = tile / (p.ntx * p.nty);
-    const int x0 = tx_i * TX, y0 = ty_i * TY;
-    const int Z0 = 1 + zc_i * p.zchunk;         // first ghosted output plane
-    const int Zl = min(Z0 + p.zchunk - 1, nz);  // last ghosted output plane
+    const int x0 = (pc.col % p.ntx) * TX, y0 = (pc.col / p.ntx) * TY;
+    const int Z0 = 1 + pc.u0, Zl = pc.u1;  // first and last ghosted output plane
     // flat grids: only plane 1, no x3 pipeline
     const int Pfirst = flat ? Z0 : Z0 - HH, Plast = flat ? Zl : Zl + HH;
     const int Kfirst = flat ? Z0 : Z0 - 4;  // first step: P (and tau) of plane Z0-2

@@ -127,13 +127,14 @@ __device__ __forceinline__ float strip_pressure(const float* u, int PL, float gm
   return gm1 * (E - ke);
 }
 
-// One tile of the stage (all planes of its z-chunk).  `bars` holds the ring
+// One piece of the stage (a run of planes of one tile column, or of row tiles
+// of a flat grid).  `bars` holds the ring
 // barriers (indices 0..2, phase bits 0..2), `gbar` the staged-tile barrier with
 // phase bit `gbit`; `phase_bits` and `pending` carry over from tile to tile.
 // Returns false when a wait ran out: the block must stop and drain.
 template <int LIM, int RIEM, int R, int NW>
 __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CUtensorMap* tmap,
-                                              const CUtensorMap* u0map, const CUtensorMap* accmap, int tile,
+                                              const CUtensorMap* u0map, const CUtensorMap* accmap, const Piece& pc,
                                               unsigned char* smem_raw, uint64_t* bars, uint64_t* gbar, int gbit,
                                               unsigned& phase_bits, unsigned& pending) {
   using C = NsStripCfg<R, NW>;
@@ -159,20 +160,16 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
   const int w = tid >> 5, lane = tid & 31;
   const bool is_out = w < NW;
   {
-    const int tx_i = tile % p.ntx;
-    const int ty_i = (tile / p.ntx) % p.nty;
-    const int zc_i = tile / (p.ntx * p.nty);
-    const int Z0 = 1 + zc_i * p.zchunk;         // first ghosted output plane
-    const int Zl = min(Z0 + p.zchunk - 1, nz);  // last ghosted output plane
     // A one-plane grid whose x3 ghosts copy the plane ("flat") has x3 fluxes
-    // that cancel exactly: plane 1 alone, no x3 pipeline.  Its tile marches
-    // instead over p.ysub row tiles along x2 (the steps of the march), each
-    // step's plane copy issued one step ahead into the next ring slot.
+    // that cancel exactly: plane 1 alone, no x3 pipeline.  Its piece marches
+    // instead over row tiles along x2 (the steps of the march), each step's
+    // plane copy issued one step ahead into the next ring slot.
     const bool flat = p.flat != 0;
-    const int ysub = flat ? p.ysub : 1;
-    const int x0 = tx_i * TX, ybase = ty_i * ysub * TY;
+    const int Z0 = flat ? 1 : 1 + pc.u0;  // first ghosted output plane
+    const int Zl = flat ? 1 : pc.u1;      // last ghosted output plane
+    const int x0 = (pc.col % p.ntx) * TX, ybase = flat ? pc.u0 * TY : (pc.col / p.ntx) * TY;
     int y0 = ybase;  // the current step's first row
-    const int nsteps = flat ? min(ysub, (ny + TY - 1) / TY - ty_i * ysub) : 0;
+    const int nsteps = pc.u1 - pc.u0;
     const int Kfirst = flat ? Z0 : Z0 - 2, Plast = flat ? Zl : Zl + HH;
     const int i = x0 + lane;
     const float idx = (is_out && i < nx) ? __ldg(p.met.inv_dx1 + i) : 0.f;
@@ -554,14 +551,14 @@ __global__ void __launch_bounds__(NsStripCfg<R, NW>::NT, MINB)
   __syncthreads();
   unsigned phase_bits = 0;  // expected parity per barrier (identical in the threads that wait)
   unsigned pending = 0;     // barriers with a copy in flight (thread 0)
-  const int ntiles = p.ntx * p.nty * p.nzc;
+  const OneGrid<NsParams<float>> grid{p};
+  TileWalk<OneGrid<NsParams<float>>> walk(grid);
+  Piece pc;
+  int inst;
   bool ok = true;
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
-    if (!ns_strip_tile<LIM, RIEM, R, NW>(p, &src.tmap, &src.u0map, &src.accmap, tile, smem_raw, bars,
-                                         bars + C::NSLOT, C::NSLOT, phase_bits, pending)) {
-      ok = false;
-      break;
-    }
+  while (ok && walk.next(grid, inst, pc))
+    ok = ns_strip_tile<LIM, RIEM, R, NW>(p, &src.tmap, &src.u0map, &src.accmap, pc, smem_raw, bars, bars + C::NSLOT,
+                                         C::NSLOT, phase_bits, pending);
   // On a timeout, wait (bounded) for every copy this block may still have in flight.
   if (!ok && tid == 0) {
     for (int s = 0; s < C::NBAR; ++s)

@@ -160,12 +160,14 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
     if (need_u0) tma_prefetch_desc(&src.u0map);
     if (need_acc) tma_prefetch_desc(&src.accmap);
   }
-  const int ntiles = p.ntx * p.nty * p.nzc;
+  const OneGrid<NsParams<float>> grid{p};
+  TileWalk<OneGrid<NsParams<float>>> walk(grid);
+  Piece pc;
+  int inst;
   bool ok = true;
-  for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-    const int x0 = (tile % p.ntx) * TX, y0 = ((tile / p.ntx) % p.nty) * TY;
-    const int Z0 = 1 + (tile / (p.ntx * p.nty)) * p.zchunk;
-    const int Zl = min(Z0 + p.zchunk - 1, nz);
+  while (ok && walk.next(grid, inst, pc)) {
+    const int x0 = (pc.col % p.ntx) * TX, y0 = (pc.col / p.ntx) * TY;
+    const int Z0 = 1 + pc.u0, Zl = pc.u1;
     const int Kfirst = Z0 - 3, Plast = Zl + HH;
     const int i = x0 + lane;
     const float idx = (is_out && i < nx) ? __ldg(m.inv_dx1 + i) : 0.f;
