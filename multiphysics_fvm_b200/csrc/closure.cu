@@ -1,5 +1,6 @@
 // Learned flux-correction closure: host side of the C ABI (include/fvm_closure.h)
 // and the launch sequences for inference, training and the solver hook.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -324,7 +325,17 @@ cudaError_t launch_box_filter(const float* u, const Layout& lay, int nv, int f, 
 }
 cudaError_t launch_dense_copy(float* u, const Layout& lay, int nv, float* dense, int to_state, int nsm,
                               cudaStream_t s) {
-  dense_copy_kernel<float><<<4 * nsm, 256, 0, s>>>(u, lay, nv, dense, to_state);
+  // 16-byte elements need dense rows of whole float4 from an aligned base (the
+  // state's first interior column is 16-byte aligned by its layout)
+  const bool wide = lay.nx % 4 == 0 && reinterpret_cast<uintptr_t>(dense) % 16 == 0;
+  const int n = wide ? lay.nx / 4 : lay.nx;
+  int gsh = 0;  // lanes per row: the power of two that covers it, at most a warp
+  while (gsh < 5 && (1 << gsh) < n) ++gsh;
+  const long long lanes = ((long long)lay.ny * lay.nz) << gsh;
+  const long long want = (lanes + 256ll * DC_ROWS - 1) / (256ll * DC_ROWS);
+  const dim3 grid((unsigned)std::min(want, 4ll * nsm), (unsigned)nv);
+  if (wide) dense_copy_kernel<float4><<<grid, 256, 0, s>>>(u, lay, dense, to_state, gsh);
+  else dense_copy_kernel<float><<<grid, 256, 0, s>>>(u, lay, dense, to_state, gsh);
   return cudaGetLastError();
 }
 cudaError_t enqueue_fix(fvm_closure* c, const float* uin, float* uout, const Layout& lay, float gamma, float coef,

@@ -763,18 +763,40 @@ __global__ void box_filter_kernel(const float* u, Layout lay, int nv, int f, flo
   }
 }
 
-// Interior copy between a solver-layout state and a dense [q][k][j][i] array.
-template <typename Real>
-__global__ void dense_copy_kernel(Real* u, Layout lay, int nv, Real* dense, int to_state) {
-  const long long n = (long long)lay.nx * lay.ny * lay.nz;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n * nv;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int q = (int)(e / n);
-    const long long p = e % n;
-    const int i = (int)(p % lay.nx), j = (int)((p / lay.nx) % lay.ny), k = (int)(p / ((long long)lay.nx * lay.ny));
-    const long long s = lay.idx(q, k + 1, j + 1, i + 1);
-    if (to_state) u[s] = dense[e];
-    else dense[e] = u[s];
+// Interior copy between a solver-layout state and a dense [q][k][j][i] array,
+// bound by HBM: one lane group (2^gsh lanes, gsh <= 5) per x1 row, V elements
+// (16 bytes where rows and pointers allow) along it, DC_ROWS rows in flight
+// before their stores; blockIdx.y is the variable.  One element per thread with
+// 64-bit divisions for its cell took 571 us at 5 x 256^3 (1.2 TB/s), this
+// takes 118 us (5.7 TB/s).
+constexpr int DC_ROWS = 4;
+template <typename V>
+__global__ void __launch_bounds__(256) dense_copy_kernel(float* u, Layout lay, float* dense, int to_state, int gsh) {
+  const int n = lay.nx / (int)(sizeof(V) / sizeof(float)), rows = lay.ny * lay.nz;
+  const int lane = threadIdx.x & ((1 << gsh) - 1);
+  const long long ngrp = ((long long)gridDim.x * blockDim.x) >> gsh;
+  const long long grp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> gsh;
+  for (long long r0 = grp; r0 < rows; r0 += DC_ROWS * ngrp) {
+    V* s[DC_ROWS];
+    V* d[DC_ROWS];
+    bool in[DC_ROWS];
+#pragma unroll
+    for (int m = 0; m < DC_ROWS; ++m) {
+      const long long row = r0 + m * ngrp;
+      in[m] = row < rows;
+      const int r = in[m] ? (int)row : 0, k = r / lay.ny, j = r - k * lay.ny;
+      s[m] = reinterpret_cast<V*>(u + lay.idx(blockIdx.y, k + 1, j + 1, 1));
+      d[m] = reinterpret_cast<V*>(dense + ((long long)blockIdx.y * rows + r) * lay.nx);
+    }
+    for (int x = lane; x < n; x += 1 << gsh) {
+      V v[DC_ROWS];
+#pragma unroll
+      for (int m = 0; m < DC_ROWS; ++m)
+        if (in[m]) v[m] = to_state ? d[m][x] : s[m][x];
+#pragma unroll
+      for (int m = 0; m < DC_ROWS; ++m)
+        if (in[m]) (to_state ? s[m] : d[m])[x] = v[m];
+    }
   }
 }
 
