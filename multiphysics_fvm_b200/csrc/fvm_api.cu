@@ -362,11 +362,11 @@ void fill_common(fvm_handle* h, const StageDef& sd, bool rhs_only, P& p) {
 }
 
 // x3 fluxes cancel exactly on a one-plane grid whose x3 ghosts copy the plane
-// (periodic or Neumann for every variable): the float32 inviscid path then
-// skips the x3 pipeline ("flat").
+// (periodic or Neumann for every variable): the inviscid kernels then skip the
+// x3 pipeline ("flat").
 bool flat_grid(const fvm_handle* h) {
   const fvm_desc& d = h->d;
-  if (h->f64 || d.nx3 != 1 || d.physics != FVM_NAVIER_STOKES || d.params[1] != 0.0) return false;
+  if (d.nx3 != 1 || d.physics != FVM_NAVIER_STOKES || d.params[1] != 0.0) return false;
   for (int q = 0; q < h->nv; ++q)
     for (int s = 4; s < 6; ++s)
       if (d.bc_kind[q][s] != FVM_BC_PERIODIC && d.bc_kind[q][s] != FVM_BC_NEUMANN) return false;
@@ -1851,7 +1851,6 @@ int fvm_filter_state(fvm_handle* h, int factor, float* coarse_dense_dev) {
 static int dense_copy(fvm_handle* h, float* dense, int to_state) {
   if (!h || !dense) return fail(FVM_E_INVALID, "null argument");
   if (h->f64) return fail(FVM_E_INVALID, "dense copy: float32 handles only");
-  FVM_CK(cudaStreamSynchronize(h->stream));
   FVM_CK(closure::launch_dense_copy(static_cast<float*>(h->U[0]), h->lay, h->nv, dense, to_state, h->nsm, h->stream));
   FVM_CK(cudaStreamSynchronize(h->stream));
   return FVM_OK;

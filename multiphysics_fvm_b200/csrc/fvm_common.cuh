@@ -154,33 +154,29 @@ __device__ __forceinline__ void lame_at(const Metric<Real>& m, int i, int j, Lam
 }
 
 // ------------------------------------------------------------ limiters ----
-template <typename R>
-__device__ __forceinline__ R sgn(R x) { return x > R(0) ? R(1) : (x < R(0) ? R(-1) : R(0)); }
+__device__ __forceinline__ float sgn(float x) { return x > 0.f ? 1.f : (x < 0.f ? -1.f : 0.f); }
 
+// The float64 limiters give the reference's values without its float64 sign
+// sums: where the signs of a and b agree (sign bits, an integer operation) the
+// sign factor is +-1 or, for the three-sign test, +-1 too.
+__device__ __forceinline__ bool same_sign(double a, double b) { return (__double2hiint(a) ^ __double2hiint(b)) >= 0; }
+__device__ __forceinline__ double abs_min(double a, double b) { return fabs(a) < fabs(b) ? a : b; }
 // slope_limiters.py:13-39
-template <typename R>
-__device__ __forceinline__ R lim_minmod(R a, R b) {
-  R ss = (sgn(a) + sgn(b)) / R(2);
-  return ss * fmin(fabs(a), fabs(b));
-}
-// slope_limiters.py:42-73 (three-sign test divided by 3, nonzero for opposite signs)
-template <typename R>
-__device__ __forceinline__ R lim_mc(R a, R b) {
-  R c = R(0.5) * (a + b);
-  R a2 = R(2) * a, b2 = R(2) * b;
-  R ss = ((sgn(c) + sgn(a2)) + sgn(b2)) / R(3);
-  return ss * fmin(fabs(c), fmin(fabs(a2), fabs(b2)));
+__device__ __forceinline__ double lim_minmod(double a, double b) { return same_sign(a, b) ? abs_min(a, b) : 0.0; }
+// slope_limiters.py:42-73 (three-sign test divided by 3: opposite slopes keep
+// a third of the sign of their sum)
+__device__ __forceinline__ double lim_mc(double a, double b) {
+  const double c = 0.5 * (a + b);
+  const double m = fabs(abs_min(c, 2.0 * abs_min(a, b)));
+  return copysign(same_sign(a, b) ? m : (1.0 / 3.0) * m, c);
 }
 // slope_limiters.py:76-105
-template <typename R>
-__device__ __forceinline__ R lim_vanleer(R a, R b) {
-  R ss = (sgn(a) + sgn(b)) / R(2);
-  R den = fabs(a) + fabs(b);
-  R hm = den > R(0) ? ((R(2) * a) * b) / den : R(0);
-  return ss * hm;
+__device__ __forceinline__ double lim_vanleer(double a, double b) {
+  const double ab = (2.0 * a) * b, den = fabs(a) + fabs(b);
+  return same_sign(a, b) && den > 0.0 ? copysign(ab / den, a) : 0.0;
 }
-template <int LIM, typename R>
-__device__ __forceinline__ R limiter(R a, R b) {
+template <int LIM>
+__device__ __forceinline__ double limiter(double a, double b) {
   if constexpr (LIM == LIM_MINMOD) return lim_minmod(a, b);
   else if constexpr (LIM == LIM_MC) return lim_mc(a, b);
   else return lim_vanleer(a, b);
@@ -204,6 +200,25 @@ __device__ __forceinline__ R recip(R x) {
   if constexpr (sizeof(R) == 4) return rcp_approx(x);
   else return R(1) / x;
 }
+// Quotients x / y by one y.  float32: the approximate reciprocal.  float64: the
+// correctly rounded reciprocal r once, then per x the product q = x r and one
+// residual correction q + (x - q y) r with fused multiply-adds (Markstein 1990),
+// which rounds to the quotient itself: three operations in place of a division
+// of about 25 instructions.  (x or 1/y infinite gives NaN where the division
+// gives infinity; such a state is already flagged.)  The float64 viscous stage
+// divided 120 times per cell and 26 times by a shared denominator.
+template <typename R>
+struct Quot {
+  R y, r;
+  __device__ __forceinline__ explicit Quot(R y_) : y(y_), r(recip(y_)) {}
+  __device__ __forceinline__ R operator()(R x) const {
+    if constexpr (sizeof(R) == 4) return x * r;
+    else {
+      const R q = x * r;
+      return __fma_rn(__fma_rn(-q, y, x), r, q);
+    }
+  }
+};
 // Limiters are positively homogeneous of degree one, so limiter(a/L, b/L)*L
 // equals limiter(a, b); the float32 path evaluates that form directly.
 __device__ __forceinline__ float flim_minmod(float a, float b) {
@@ -221,7 +236,7 @@ __device__ __forceinline__ float flim_mc(float a, float b) {
 
 // MUSCL slope of a cell (reconstructors.py:120-132): limiter(bwd/L, fwd/L)*L.
 template <int LIM, typename R>
-__device__ __forceinline__ R muscl_slope(R fm, R f0, R fp, R L) {
+__device__ __forceinline__ R muscl_slope(R fm, R f0, R fp, const Quot<R>& L) {
   if constexpr (LIM == LIM_PC) return R(0);
   else if constexpr (sizeof(R) == 4) {
     const float a = f0 - fm, b = fp - f0;
@@ -229,7 +244,7 @@ __device__ __forceinline__ R muscl_slope(R fm, R f0, R fp, R L) {
     else if constexpr (LIM == LIM_MC) return flim_mc(a, b);
     else return flim_vanleer(a, b);
   } else {
-    return limiter<LIM>((f0 - fm) / L, (fp - f0) / L) * L;
+    return limiter<LIM>(L(f0 - fm), L(fp - f0)) * L.y;
   }
 }
 

@@ -150,9 +150,10 @@ __global__ void __launch_bounds__(HeatCfg<Real, LIM, TY>::NT, 1)
         const int pl = K + HH;
         const Real* ub = uring + pmod(pl, C::NSLOT) * C::SLOT;
         Real* tb = tring + pmod(pl, 3) * PL;
+        const Quot<Real> by_rcp(rcp);
         for (int it = tid; it < C::ROWS * (TX + 6); it += NT) {
           const int o = (it / (TX + 6)) * W + 1 + it % (TX + 6);
-          tb[o] = ub[o] / rcp;
+          tb[o] = by_rcp(ub[o]);
         }
         __syncthreads();
       }
@@ -198,7 +199,7 @@ __global__ void __launch_bounds__(HeatCfg<Real, LIM, TY>::NT, 1)
         if constexpr (LIM != LIM_PC) {
           const bool ghost = (K + 1 <= 0 || K + 1 >= nz + 1);
           if (!ghost && out_valid)
-            zn = muscl_slope<LIM>(Ph(K, 2, r, c), Ph(K + 1, 2, r, c), Ph(K + 2, 2, r, c), G::L3(p.met, oi, oj, K));
+            zn = muscl_slope<LIM>(Ph(K, 2, r, c), Ph(K + 1, 2, r, c), Ph(K + 2, 2, r, c), Quot<Real>(G::L3(p.met, oi, oj, K)));
         }
         if (K >= Z0 - 1) {
           const Real fl = Ph(K, 2, r, c) + zs / Real(2);
@@ -242,7 +243,7 @@ __global__ void __launch_bounds__(HeatCfg<Real, LIM, TY>::NT, 1)
         const Real f0 = Ph(K, 0, r, c);
         Real s = Real(0);
         if constexpr (LIM != LIM_PC) {
-          if (i >= 0 && i < nx && j < ny) s = muscl_slope<LIM>(Ph(K, 0, r, c - 1), f0, Ph(K, 0, r, c + 1), G::L1(p.met, i, j, kK));
+          if (i >= 0 && i < nx && j < ny) s = muscl_slope<LIM>(Ph(K, 0, r, c - 1), f0, Ph(K, 0, r, c + 1), Quot<Real>(G::L1(p.met, i, j, kK)));
         }
         const int o = ty * (TX + 2) + tx + 1;
         fL[o] = f0 + s / Real(2);
@@ -268,7 +269,7 @@ __global__ void __launch_bounds__(HeatCfg<Real, LIM, TY>::NT, 1)
         const Real f0 = Ph(K, 1, r, c);
         Real s = Real(0);
         if constexpr (LIM != LIM_PC) {
-          if (i < nx && j >= 0 && j < ny) s = muscl_slope<LIM>(Ph(K, 1, r - 1, c), f0, Ph(K, 1, r + 1, c), G::L2(p.met, i, j, kK));
+          if (i < nx && j >= 0 && j < ny) s = muscl_slope<LIM>(Ph(K, 1, r - 1, c), f0, Ph(K, 1, r + 1, c), Quot<Real>(G::L2(p.met, i, j, kK)));
         }
         const int o = (ty + 1) * TX + tx;
         fL[o] = f0 + s / Real(2);

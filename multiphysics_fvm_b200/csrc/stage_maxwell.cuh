@@ -67,16 +67,9 @@ struct MaxwellCfg {
 // F_B[c] = FB[c][D], F_D[c] = FD[c][D] with FB12 = E3, FB13 = -E2, FB23 = E1,
 // FD12 = -H3, FD13 = H2, FD23 = -H1 and antisymmetry (maxwell.py:145-165).
 template <typename R, int D>
-__device__ __forceinline__ void maxwell_face(const R* q, R mu, R ep, R F[6]) {
-  R H0, H1, H2, E0, E1, E2;
-  if constexpr (sizeof(R) == 4) {
-    const R imu = rcp_approx(mu), iep = rcp_approx(ep);
-    H0 = q[0] * imu; H1 = q[1] * imu; H2 = q[2] * imu;
-    E0 = q[3] * iep; E1 = q[4] * iep; E2 = q[5] * iep;
-  } else {
-    H0 = q[0] / mu; H1 = q[1] / mu; H2 = q[2] / mu;
-    E0 = q[3] / ep; E1 = q[4] / ep; E2 = q[5] / ep;
-  }
+__device__ __forceinline__ void maxwell_face(const R* q, const Quot<R>& mu, const Quot<R>& ep, R F[6]) {
+  const R H0 = mu(q[0]), H1 = mu(q[1]), H2 = mu(q[2]);
+  const R E0 = ep(q[3]), E1 = ep(q[4]), E2 = ep(q[5]);
   if constexpr (D == 0) {
     F[0] = R(0); F[1] = -E2; F[2] = E1;
     F[3] = R(0); F[4] = H2; F[5] = -H1;
@@ -90,7 +83,7 @@ __device__ __forceinline__ void maxwell_face(const R* q, R mu, R ep, R F[6]) {
 }
 
 template <typename R, int D, int RIEM>
-__device__ __forceinline__ void maxwell_flux(const R* qL, const R* qR, R mu, R ep, R c, R F[6]) {
+__device__ __forceinline__ void maxwell_flux(const R* qL, const R* qR, const Quot<R>& mu, const Quot<R>& ep, const Quot<R>& c2, R c, R F[6]) {
   R FL[6], FR[6];
   maxwell_face<R, D>(qL, mu, ep, FL);
   maxwell_face<R, D>(qR, mu, ep, FR);
@@ -99,8 +92,7 @@ __device__ __forceinline__ void maxwell_flux(const R* qL, const R* qR, R mu, R e
     if constexpr (RIEM == RIEM_HLL) {
       const R smin = -c, smax = c;
       const R num = ((smax * FL[v]) - (smin * FR[v])) + ((smin * smax) * (qR[v] - qL[v]));
-      if constexpr (sizeof(R) == 4) F[v] = num * (0.5f * rcp_approx(c));
-      else F[v] = num / (smax - smin);
+      F[v] = c2(num);
     } else {
       F[v] = ((FL[v] + FR[v]) / R(2)) - ((c * (qR[v] - qL[v])) / R(2));
     }
@@ -133,7 +125,8 @@ __global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, MINB)
   const int tid = threadIdx.x;
   const Layout& L = p.lay;
   const int nx = L.nx, ny = L.ny, nz = L.nz;
-  const Real mu = Real(p.mu), ep = Real(p.ep), cl = Real(p.c);
+  const Quot<Real> mu(Real(p.mu)), ep(Real(p.ep)), c2(Real(p.c) + Real(p.c));
+  const Real cl = Real(p.c);
   const Real dt = Real(*p.dt);
   if (tid == 0) {
     tma_prefetch_desc(&tmap);
@@ -219,6 +212,8 @@ __global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, MINB)
             const int i = x0 + c - 4, j = y0 + r - HH;
             if (i < 0 || i >= nx || j < 0 || j >= ny) continue;
             Real div[2];
+            const Quot<Real> by1(Real(2) * G::L1(p.met, i, j, k)), by2(Real(2) * G::L2(p.met, i, j, k));
+            const Quot<Real> by3(Real(2) * G::L3(p.met, i, j, k));
             Lame<Real> lm;
             if constexpr (COORD != COORD_CART) lame_at<Real, COORD>(p.met, i, j, lm);
 #pragma unroll
@@ -230,10 +225,9 @@ __global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, MINB)
                 d2 = (UA(uK1, q0 + 1, r + 1, c) - UA(uK1, q0 + 1, r - 1, c)) * (0.5f * inv_len<Real, COORD, 1>(p.met, i, j, k));
                 d3 = (UA(uK2, q0 + 2, r, c) - UA(uK, q0 + 2, r, c)) * (0.5f * inv_len<Real, COORD, 2>(p.met, i, j, k));
               } else {
-                const Real l1 = G::L1(p.met, i, j, k), l2 = G::L2(p.met, i, j, k), l3 = G::L3(p.met, i, j, k);
-                d1 = (UA(uK1, q0, r, c + 1) - UA(uK1, q0, r, c - 1)) / (Real(2) * l1);
-                d2 = (UA(uK1, q0 + 1, r + 1, c) - UA(uK1, q0 + 1, r - 1, c)) / (Real(2) * l2);
-                d3 = (UA(uK2, q0 + 2, r, c) - UA(uK, q0 + 2, r, c)) / (Real(2) * l3);
+                d1 = by1(UA(uK1, q0, r, c + 1) - UA(uK1, q0, r, c - 1));
+                d2 = by2(UA(uK1, q0 + 1, r + 1, c) - UA(uK1, q0 + 1, r - 1, c));
+                d3 = by3(UA(uK2, q0 + 2, r, c) - UA(uK, q0 + 2, r, c));
               }
               Real dv = (d1 + d2) + d3;
               if constexpr (COORD != COORD_CART) {
@@ -265,7 +259,7 @@ __global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, MINB)
 #pragma unroll
           for (int v = 0; v < NV; ++v) zn[v] = Real(0);
         } else {
-          const Real l3 = G::L3(p.met, oi, oj, K);
+          const Quot<Real> l3(G::L3(p.met, oi, oj, K));
 #pragma unroll
           for (int v = 0; v < NV; ++v) zn[v] = muscl_slope<LIM>(qm[v], q0[v], qp[v], l3);
         }
@@ -273,7 +267,7 @@ __global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, MINB)
           Real qL[NV], qR[NV], F[NV];
 #pragma unroll
           for (int v = 0; v < NV; ++v) { qL[v] = qm[v] + zs[v] / Real(2); qR[v] = q0[v] - zn[v] / Real(2); }
-          maxwell_flux<Real, 2, RIEM>(qL, qR, mu, ep, cl, F);
+          maxwell_flux<Real, 2, RIEM>(qL, qR, mu, ep, c2, cl, F);
 #pragma unroll
           for (int v = 0; v < NV; ++v) { Fzp[v] = Fzn[v]; Fzn[v] = F[v] * S3c; }
         }
@@ -288,7 +282,7 @@ __global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, MINB)
         const int ty = it / (TX + 2), tx = it % (TX + 2) - 1;
         const int r = ty + HH, c = tx + 4, i = x0 + tx, j = y0 + ty;
         const bool interior = i >= 0 && i < nx && j < ny;
-        const Real l1 = interior ? G::L1(p.met, i, j, kK) : Real(1);
+        const Quot<Real> l1(interior ? G::L1(p.met, i, j, kK) : Real(1));
         const int o = ty * (TX + 2) + tx + 1;
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
@@ -309,7 +303,7 @@ __global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, MINB)
           const int o = ty * (TX + 2) + fx;
 #pragma unroll
           for (int v = 0; v < NV; ++v) { qL[v] = fL[v * C::XB + o]; qR[v] = fR[v * C::XB + o + 1]; }
-          maxwell_flux<Real, 0, RIEM>(qL, qR, mu, ep, cl, F);
+          maxwell_flux<Real, 0, RIEM>(qL, qR, mu, ep, c2, cl, F);
           const Real s1 = G::S1(p.met, fi, j, kK);
 #pragma unroll
           for (int v = 0; v < NV; ++v) F[v] = F[v] * s1;
@@ -331,7 +325,7 @@ __global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, MINB)
         const int ty = it / TX - 1, tx = it % TX;
         const int r = ty + HH, c = tx + 4, i = x0 + tx, j = y0 + ty;
         const bool interior = i < nx && j >= 0 && j < ny;
-        const Real l2 = interior ? G::L2(p.met, i, j, kK) : Real(1);
+        const Quot<Real> l2(interior ? G::L2(p.met, i, j, kK) : Real(1));
         const int o = (ty + 1) * TX + tx;
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
@@ -352,7 +346,7 @@ __global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, MINB)
           const int o = fy * TX + tx;
 #pragma unroll
           for (int v = 0; v < NV; ++v) { qL[v] = fL[v * C::XB + o]; qR[v] = fR[v * C::XB + o + TX]; }
-          maxwell_flux<Real, 1, RIEM>(qL, qR, mu, ep, cl, F);
+          maxwell_flux<Real, 1, RIEM>(qL, qR, mu, ep, c2, cl, F);
           const Real s2 = G::S2(p.met, i, fj, kK);
 #pragma unroll
           for (int v = 0; v < NV; ++v) F[v] = F[v] * s2;
@@ -373,8 +367,8 @@ __global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, MINB)
         if constexpr (COORD != COORD_CART) {
           Lame<Real> lm;
           lame_at<Real, COORD>(p.met, oi, oj, lm);
-          const Real H0 = q[0] / mu, H1 = q[1] / mu, H2 = q[2] / mu;
-          const Real E0 = q[3] / ep, E1 = q[4] / ep, E2 = q[5] / ep;
+          const Real H0 = mu(q[0]), H1 = mu(q[1]), H2 = mu(q[2]);
+          const Real E0 = ep(q[3]), E1 = ep(q[4]), E2 = ep(q[5]);
           Real FB[3][3], FD[3][3];
           FB[0][1] = E2; FB[0][2] = -E1; FB[1][2] = E0;
           FD[0][1] = -H2; FD[0][2] = H1; FD[1][2] = -H0;
@@ -419,7 +413,7 @@ __global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, MINB)
           sc[3 * f + 1] = (-chi) * g2;
           sc[3 * f + 2] = (-chi) * g3;
         }
-        const Real Vc = G::V(p.met, oi, oj, kK);
+        const Quot<Real> by_V(G::V(p.met, oi, oj, kK));
         const long long gidx = L.idx(0, K, oj + 1, oi + 1);
         // residual of each variable first (the flux registers die), then
         // every global load of the cell before its first store: the stores
@@ -430,9 +424,8 @@ __global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, MINB)
         for (int v = 0; v < NV; ++v) {
           const Real Fym = fb[v * C::FB + oty * TX + otx], Fyp = fb[v * C::FB + (oty + 1) * TX + otx];
           const Real sum = ((((Fxp[v] - Fxm[v]) + Fyp) - Fym) + Fzn[v]) - Fzp[v];
-          const Real sp = v < 3 ? Real(0) : (-Real(p.sigma)) * (q[v] / ep);
-          if constexpr (sizeof(Real) == 4) kv[v] = (-sum) * rcp_approx(Vc) + ((sg[v] + sp) + sc[v]);
-          else kv[v] = (-sum) / Vc + ((sg[v] + sp) + sc[v]);
+          const Real sp = v < 3 ? Real(0) : (-Real(p.sigma)) * ep(q[v]);
+          kv[v] = by_V(-sum) + ((sg[v] + sp) + sc[v]);
         }
         Real u0v[NV], accv[NV];
         if constexpr (STAGED) cp_async_wait_all();

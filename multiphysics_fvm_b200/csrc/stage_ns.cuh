@@ -88,13 +88,8 @@ struct NsCfg {
 template <typename R, int D, bool VISC>
 __device__ __forceinline__ void ns_face(const R* q, R gam, R Fc[5], R Fd[5], R& vn, R& cs) {
   const R rho = q[0];
-  R v0, v1, v2, E, ir = R(0);
-  if constexpr (sizeof(R) == 4) {
-    ir = rcp_approx(rho);
-    v0 = q[1] * ir; v1 = q[2] * ir; v2 = q[3] * ir; E = q[4] * ir;
-  } else {
-    v0 = q[1] / rho; v1 = q[2] / rho; v2 = q[3] / rho; E = q[4] / rho;
-  }
+  const Quot<R> by_rho(rho);
+  const R v0 = by_rho(q[1]), v1 = by_rho(q[2]), v2 = by_rho(q[3]), E = by_rho(q[4]);
   const R P = q[5];
   const R va = D == 0 ? v0 : (D == 1 ? v1 : v2);
   Fc[0] = rho * va;
@@ -110,8 +105,8 @@ __device__ __forceinline__ void ns_face(const R* q, R gam, R Fc[5], R Fd[5], R& 
     Fd[3] = -q[8];
     Fd[4] = (((-q[6]) * v0) - (q[7] * v1)) - (q[8] * v2);
   }
-  if constexpr (sizeof(R) == 4) cs = sqrt_approx((gam * P) * ir);
-  else cs = sqrt((gam * P) / rho);
+  if constexpr (sizeof(R) == 4) cs = sqrt_approx(by_rho(gam * P));
+  else cs = sqrt(by_rho(gam * P));
   vn = va;
 }
 
@@ -124,15 +119,11 @@ __device__ __forceinline__ void ns_flux(const R* qL, const R* qR, R gam, R F[5])
   if constexpr (RIEM == RIEM_HLL) {
     const R smin = fmin(vnL - csL, vnR - csR);
     const R smax = fmax(vnL + csL, vnR + csR);
-    const R den = smax - smin;
-    const R rden = recip(den);
+    const Quot<R> by_den(smax - smin);
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
       const R num = ((smax * FcL[v]) - (smin * FcR[v])) + ((smin * smax) * (qR[v] - qL[v]));
-      R mid;
-      if constexpr (sizeof(R) == 4) mid = num * rden;
-      else mid = num / den;
-      F[v] = smin >= R(0) ? FcL[v] : (smax <= R(0) ? FcR[v] : mid);
+      F[v] = smin >= R(0) ? FcL[v] : (smax <= R(0) ? FcR[v] : by_den(num));
     }
   } else {
     const R vs = fmax(fabs(vnL) + csL, fabs(vnR) + csR);
@@ -319,17 +310,10 @@ __global__ void __launch_bounds__(NsCfg<Real, VISC, TY>::NT, MINB)
           for (int it = tid; it < C::ROWS * (TX + 6); it += NT) {
             const int r = it / (TX + 6), c = 1 + it % (TX + 6);
             const int o = r * W + c;
-            const Real rho = ub[o];
-            if constexpr (F32) {
-              const Real ir = rcp_approx(rho);
-              vb[o] = ub[PL + o] * ir;
-              vb[PL + o] = ub[2 * PL + o] * ir;
-              vb[2 * PL + o] = ub[3 * PL + o] * ir;
-            } else {
-              vb[o] = ub[PL + o] / rho;
-              vb[PL + o] = ub[2 * PL + o] / rho;
-              vb[2 * PL + o] = ub[3 * PL + o] / rho;
-            }
+            const Quot<Real> by_rho(ub[o]);
+            vb[o] = by_rho(ub[PL + o]);
+            vb[PL + o] = by_rho(ub[2 * PL + o]);
+            vb[2 * PL + o] = by_rho(ub[3 * PL + o]);
           }
         }
       }
@@ -342,15 +326,8 @@ __global__ void __launch_bounds__(NsCfg<Real, VISC, TY>::NT, MINB)
         const int r2 = it / W2, c2 = it % W2;
         const Real* u = usrc + (r2 + HH - 2) * W + c2 + 2;
         const Real rho = u[0];
-        Real v0, v1, v2, E;
-        if constexpr (F32) {
-          const Real ir = rcp_approx(rho);
-          v0 = u[PL] * ir; v1 = u[2 * PL] * ir; v2 = u[3 * PL] * ir;
-          E = u[4 * PL] * ir;
-        } else {
-          v0 = u[PL] / rho; v1 = u[2 * PL] / rho; v2 = u[3 * PL] / rho;
-          E = u[4 * PL] / rho;
-        }
+        const Quot<Real> by_rho(rho);
+        const Real v0 = by_rho(u[PL]), v1 = by_rho(u[2 * PL]), v2 = by_rho(u[3 * PL]), E = by_rho(u[4 * PL]);
         pw[it] = ((gam - Real(1)) * rho) * (E - (((v0 * v0) + (v1 * v1)) + (v2 * v2)) / Real(2));
       };
       if constexpr (!VISC) {
@@ -391,13 +368,14 @@ __global__ void __launch_bounds__(NsCfg<Real, VISC, TY>::NT, MINB)
                 g[cc][2] = (vp[o] - vm[o]) * h3;
               }
             } else {
-              const Real l1 = G::L1(p.met, i, j, k), l2 = G::L2(p.met, i, j, k), l3 = G::L3(p.met, i, j, k);
+              const Quot<Real> by1(Real(2) * G::L1(p.met, i, j, k)), by2(Real(2) * G::L2(p.met, i, j, k));
+              const Quot<Real> by3(Real(2) * G::L3(p.met, i, j, k));
 #pragma unroll
               for (int cc = 0; cc < 3; ++cc) {
                 const int o = cc * PL + r * W + c;
-                g[cc][0] = (v0p[o + 1] - v0p[o - 1]) / (Real(2) * l1);
-                g[cc][1] = (v0p[o + W] - v0p[o - W]) / (Real(2) * l2);
-                g[cc][2] = (vp[o] - vm[o]) / (Real(2) * l3);
+                g[cc][0] = by1(v0p[o + 1] - v0p[o - 1]);
+                g[cc][1] = by2(v0p[o + W] - v0p[o - W]);
+                g[cc][2] = by3(vp[o] - vm[o]);
               }
             }
             const Real tt = Real(2.0 / 3.0);
@@ -449,7 +427,7 @@ __global__ void __launch_bounds__(NsCfg<Real, VISC, TY>::NT, MINB)
 #pragma unroll
           for (int f = 0; f < NREC; ++f) zn[f] = Real(0);
         } else {
-          const Real l3 = F32 ? Real(1) : G::L3(p.met, oi, oj, kk);
+          const Quot<Real> l3(F32 ? Real(1) : G::L3(p.met, oi, oj, kk));
 #pragma unroll
           for (int f = 0; f < NREC; ++f) zn[f] = muscl_slope<LIM>(qm[f], q0[f], qp[f], l3);
         }
@@ -484,7 +462,7 @@ __global__ void __launch_bounds__(NsCfg<Real, VISC, TY>::NT, MINB)
           if (hh < 32) {
             const int i = x0 - 1;
             const bool in = i >= 0 && j < ny;  // i < nx as x0 < nx
-            const Real l1 = (F32 || !in) ? Real(1) : G::L1(p.met, i, j, kh);
+            const Quot<Real> l1((F32 || !in) ? Real(1) : G::L1(p.met, i, j, kh));
 #pragma unroll
             for (int f = 0; f < NREC; ++f)
               hl[(par * NREC + f) * TY + row] =
@@ -496,8 +474,8 @@ __global__ void __launch_bounds__(NsCfg<Real, VISC, TY>::NT, MINB)
             Real F[5] = {Real(0), Real(0), Real(0), Real(0), Real(0)};
             if (i <= nx && j < ny) {
               const bool in0 = i < nx;  // cell i-1 is interior here
-              const Real l1m = F32 ? Real(1) : G::L1(p.met, i - 1, j, kh);
-              const Real l1 = (F32 || !in0) ? Real(1) : G::L1(p.met, i, j, kh);
+              const Quot<Real> l1m(F32 ? Real(1) : G::L1(p.met, i - 1, j, kh));
+              const Quot<Real> l1((F32 || !in0) ? Real(1) : G::L1(p.met, i, j, kh));
               Real qL[NREC], qR[NREC];
 #pragma unroll
               for (int f = 0; f < NREC; ++f) {
@@ -535,7 +513,7 @@ __global__ void __launch_bounds__(NsCfg<Real, VISC, TY>::NT, MINB)
         const int tx = otx, ty = oty, par = K & 1;
         const int i = x0 + tx, j = y0 + ty;
         const bool in0 = i < nx && j < ny;  // this cell (i >= 0)
-        const Real l1 = (F32 || !in0) ? Real(1) : G::L1(p.met, i, j, kK);
+        const Quot<Real> l1((F32 || !in0) ? Real(1) : G::L1(p.met, i, j, kK));
         Real qL[NREC], qR[NREC];
 #pragma unroll
         for (int f = 0; f < NREC; ++f) {
@@ -571,7 +549,7 @@ __global__ void __launch_bounds__(NsCfg<Real, VISC, TY>::NT, MINB)
           const int ty = it / TX - 1, tx = it % TX;
           const int i = x0 + tx, j = y0 + ty;
           const bool interior = i < nx && j >= 0 && j < ny;
-          const Real l2 = (F32 || !interior) ? Real(1) : G::L2(p.met, i, j, kK);
+          const Quot<Real> l2((F32 || !interior) ? Real(1) : G::L2(p.met, i, j, kK));
 #pragma unroll
           for (int f = 0; f < NREC; ++f) {
             const Real s = interior ? muscl_slope<LIM>(field(uK, pK, tK, ti, f, tx, ty - 1), field(uK, pK, tK, ti, f, tx, ty),
@@ -614,13 +592,8 @@ __global__ void __launch_bounds__(NsCfg<Real, VISC, TY>::NT, MINB)
 #pragma unroll
         for (int v = 0; v < 5; ++v) q[v] = uK[v * PL + r * W + c];
         const Real rho = q[0];
-        Real v0, v1, v2;
-        if constexpr (F32) {
-          const Real ir = rcp_approx(rho);
-          v0 = q[1] * ir; v1 = q[2] * ir; v2 = q[3] * ir;
-        } else {
-          v0 = q[1] / rho; v1 = q[2] / rho; v2 = q[3] / rho;
-        }
+        const Quot<Real> by_rho(rho);
+        const Real v0 = by_rho(q[1]), v1 = by_rho(q[2]), v2 = by_rho(q[3]);
         // sources: geometric (navier_stokes.py:437-452) + gravity (:499-504)
         Real src[5];
         const Real gx = Real(p.g1), gy = Real(p.g2), gz = Real(p.g3);
@@ -661,9 +634,22 @@ __global__ void __launch_bounds__(NsCfg<Real, VISC, TY>::NT, MINB)
             src[1 + cc] = (sgc + sgd) + src[1 + cc];
           }
         }
-        const Real Vc = G::V(p.met, oi, oj, kK);
-        const Real iV = recip(Vc);
+        const Quot<Real> by_V(G::V(p.met, oi, oj, kK));
         const long long gidx = L.idx(0, K, oj + 1, oi + 1);
+        if constexpr (!F32 && !VISC) {
+          // a flat grid's two x3 faces carry the flux of the cell's own state
+          // (the ghost planes equal it); the reference adds one and subtracts
+          // the other, and float64 keeps that rounding
+          if (flat) {
+            Real qz[6], F[5];
+#pragma unroll
+            for (int v = 0; v < 5; ++v) qz[v] = q[v];
+            qz[5] = pK[(oty + 2) * W2 + otx + 2];
+            ns_flux<Real, 2, RIEM, false>(qz, qz, gam, F);
+#pragma unroll
+            for (int v = 0; v < 5; ++v) Fzp[v] = Fzn[v] = F[v] * S3c;
+          }
+        }
         // residual of each variable first (the flux registers die), then
         // every global load of the cell before its first store: the stores
         // may alias later loads as far as the compiler knows, which would
@@ -674,8 +660,7 @@ __global__ void __launch_bounds__(NsCfg<Real, VISC, TY>::NT, MINB)
           const Real Fym = fb[v * C::FB + oty * TX + otx];
           const Real Fyp = fb[v * C::FB + (oty + 1) * TX + otx];
           const Real sum = ((((Fxp[v] - Fxm[v]) + Fyp) - Fym) + Fzn[v]) - Fzp[v];
-          if constexpr (F32) kv[v] = (-sum) * iV + src[v];
-          else kv[v] = (-sum) / Vc + src[v];
+          kv[v] = by_V(-sum) + src[v];
         }
         Real u0v[5], accv[5];
         if constexpr (STAGED) cp_async_wait_all();
