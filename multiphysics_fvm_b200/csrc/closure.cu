@@ -45,6 +45,8 @@ struct fvm_closure {
   long long npos = 0;
   int nsm = 148;
   cudaStream_t stream = nullptr;
+  cudaStream_t side = nullptr;  // bias gradients, forked from and joined to `stream` by the two events
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   // workspace
   __nv_bfloat16 *x0 = nullptr, *a1 = nullptr, *a2 = nullptr, *g3 = nullptr, *g2 = nullptr, *g1 = nullptr;
   float *z3 = nullptr, *e = nullptr;
@@ -52,7 +54,8 @@ struct fvm_closure {
   float *w[NLAYER] = {}, *b[NLAYER] = {}, *mw[NLAYER] = {}, *vw[NLAYER] = {}, *mb[NLAYER] = {}, *vb[NLAYER] = {};
   float *gw[NLAYER] = {}, *gb[NLAYER] = {};
   __nv_bfloat16 *pf[NLAYER] = {}, *pb[NLAYER] = {};
-  float* partial = nullptr;  // wgrad / bias partial sums
+  float* partial = nullptr;    // weight-gradient partial sums
+  float* bias_part = nullptr;  // bias-gradient partial sums
   size_t partial_elems = 0;
   double* loss_part = nullptr;
   double* loss_dev = nullptr;
@@ -62,7 +65,7 @@ struct fvm_closure {
   float gamma = 1.4f;
   float in_mean[5] = {0, 0, 0, 0, 0}, in_inv_scale[5] = {1, 1, 1, 1, 1};
   float out_scale[5] = {1, 1, 1, 1, 1}, loss_w[5] = {1, 1, 1, 1, 1};
-  int zc_conv = 1, zc_wg = 1;
+  int zc_wg = 1;               // planes of a weight-gradient chunk
   unsigned* status = nullptr;  // ST_TMA_TIMEOUT when a tensor-core wait gave up
   int fct = 0;                 // 1: flux-corrected transport bound on the corrections
   float* ratio = nullptr;      // FCT fractions [10][cells]
@@ -70,14 +73,9 @@ struct fvm_closure {
 
 namespace {
 
-size_t wcount(int l) { return (size_t)27 * LCOUT[l] * LCIN[l]; }
+int wgrad_chunks(const fvm_closure* c) { return (c->n1 / 16) * (c->n2 / 8) * (c->n3 / c->zc_wg); }
 
-template <int CIN, int COUT>
-constexpr int wgrad_smem() {
-  // One CTA per SM: the accumulator block takes up to all of an SM's tensor
-  // memory, so the launch asks for more than half of its shared memory.
-  return WgCfg<CIN, COUT>::BYTES > 120 * 1024 ? WgCfg<CIN, COUT>::BYTES : 120 * 1024;
-}
+size_t wcount(int l) { return (size_t)27 * LCOUT[l] * LCIN[l]; }
 
 // Opt every tensor-core kernel into its dynamic shared memory once per
 // process (before any graph capture).
@@ -90,9 +88,9 @@ cudaError_t set_attributes() {
   CL_RET(cudaFuncSetAttribute(conv3_kernel<C_HID, C_OUT, EPI_LIN_F32>, A, ConvCfg<C_HID, C_OUT>::BYTES));
   CL_RET(cudaFuncSetAttribute(conv3_kernel<C_OUT, C_HID, EPI_MASK_BF16>, A, ConvCfg<C_OUT, C_HID>::BYTES));
   CL_RET(cudaFuncSetAttribute(conv3_kernel<C_HID, C_HID, EPI_MASK_BF16>, A, ConvCfg<C_HID, C_HID>::BYTES));
-  CL_RET(cudaFuncSetAttribute(wgrad_kernel<C_HID, C_OUT>, A, wgrad_smem<C_HID, C_OUT>()));
-  CL_RET(cudaFuncSetAttribute(wgrad_kernel<C_HID, C_HID>, A, wgrad_smem<C_HID, C_HID>()));
-  CL_RET(cudaFuncSetAttribute(wgrad_kernel<C_IN0, C_HID>, A, wgrad_smem<C_IN0, C_HID>()));
+  CL_RET(cudaFuncSetAttribute(wgrad_kernel<C_HID, C_OUT>, A, WgCfg<C_HID, C_OUT>::BYTES));
+  CL_RET(cudaFuncSetAttribute(wgrad_kernel<C_HID, C_HID>, A, WgCfg<C_HID, C_HID>::BYTES));
+  CL_RET(cudaFuncSetAttribute(wgrad_kernel<C_IN0, C_HID>, A, WgCfg<C_IN0, C_HID>::BYTES));
   done = true;
   return cudaSuccess;
 }
@@ -101,31 +99,41 @@ template <int CIN, int COUT, int EPI>
 cudaError_t conv(fvm_closure* c, const __nv_bfloat16* x, const __nv_bfloat16* wpack, const float* bias, void* y,
                  const __nv_bfloat16* mask, cudaStream_t s) {
   using C = ConvCfg<CIN, COUT>;
-  const ConvArgs a{x, wpack, bias, y, mask, c->n1, c->n2, c->n3, c->zc_conv, c->status};
-  const dim3 grid(c->n1 / 8, c->n2 / 16, c->n3 / c->zc_conv);
-  conv3_kernel<CIN, COUT, EPI><<<grid, 128, C::BYTES, s>>>(a);
+  const ConvArgs a{x, wpack, bias, y, mask, c->n1, c->n2, c->n3, c->status};
+  const long long planes = (long long)(c->n1 / 8) * (c->n2 / 16) * c->n3;
+  const int grid = (int)std::min(planes, 2ll * c->nsm);
+  conv3_kernel<CIN, COUT, EPI><<<grid, C::NT, C::BYTES, s>>>(a);
   return cudaGetLastError();
 }
 
 template <int CIN, int COUT>
-cudaError_t wgrad(fvm_closure* c, const __nv_bfloat16* x, const __nv_bfloat16* g, float* dw, float* db,
-                  cudaStream_t s) {
+cudaError_t wgrad(fvm_closure* c, const __nv_bfloat16* x, const __nv_bfloat16* g, float* dw, cudaStream_t s) {
   using C = WgCfg<CIN, COUT>;
-  const dim3 grid(c->n1 / C::TX, c->n2 / C::TY, c->n3 / c->zc_wg);
-  const int nblk = grid.x * grid.y * grid.z;
+  const int nchunk = wgrad_chunks(c);
   const WgradArgs a{x, g, c->partial, c->n1, c->n2, c->n3, c->zc_wg, c->status};
-  wgrad_kernel<CIN, COUT><<<grid, 128, wgrad_smem<CIN, COUT>(), s>>>(a);
+  wgrad_kernel<CIN, COUT><<<std::min(nchunk, C::CTAS * c->nsm), C::NT, C::BYTES, s>>>(a);
   CL_RET(cudaGetLastError());
   const int n = 27 * COUT * CIN;
-  reduce_partials_kernel<<<(n + 255) / 256, 256, 0, s>>>(c->partial, nblk, n, dw);
-  CL_RET(cudaGetLastError());
-  // bias gradient
-  const int cblk = 2 * c->nsm;
-  float* cpart = c->partial + (size_t)nblk * n;
-  channel_sum_kernel<COUT><<<cblk, 256, 0, s>>>(g, c->npos, cpart);
-  CL_RET(cudaGetLastError());
-  reduce_partials_kernel<<<1, 64, 0, s>>>(cpart, cblk, COUT, db);
+  reduce_partials_kernel<<<(n + 63) / 64, 256, 0, s>>>(c->partial, nchunk, n, dw);
   return cudaGetLastError();
+}
+
+// Bias gradient of a layer whose output gradient g the stream s has just
+// written: a memory-bound pass on the side stream, under the tensor-core kernels
+// that follow on s (join_side orders the two again).
+template <int COUT>
+cudaError_t bias_grad(fvm_closure* c, const __nv_bfloat16* g, float* db, cudaStream_t s) {
+  CL_RET(cudaEventRecord(c->ev_fork, s));
+  CL_RET(cudaStreamWaitEvent(c->side, c->ev_fork, 0));
+  const int cblk = 2 * c->nsm;
+  channel_sum_kernel<COUT><<<cblk, 256, 0, c->side>>>(g, c->npos, c->bias_part);
+  CL_RET(cudaGetLastError());
+  reduce_partials_kernel<<<1, 256, 0, c->side>>>(c->bias_part, cblk, COUT, db);
+  return cudaGetLastError();
+}
+cudaError_t join_side(fvm_closure* c, cudaStream_t s) {
+  CL_RET(cudaEventRecord(c->ev_join, c->side));
+  return cudaStreamWaitEvent(s, c->ev_join, 0);
 }
 
 cudaError_t forward(fvm_closure* c, cudaStream_t s) {
@@ -162,13 +170,17 @@ cudaError_t backward(fvm_closure* c, const float* d, double dt, const double h[3
   loss_grad_kernel<<<4 * c->nsm, 256, 0, s>>>(la);
   CL_RET(cudaGetLastError());
   // layer 3: X = A2 (32), G = G3 (16)
-  CL_RET((wgrad<C_HID, C_OUT>(c, c->a2, c->g3, c->gw[2], c->gb[2], s)));
+  CL_RET(bias_grad<C_OUT>(c, c->g3, c->gb[2], s));
+  CL_RET((wgrad<C_HID, C_OUT>(c, c->a2, c->g3, c->gw[2], s)));
   CL_RET((conv<C_OUT, C_HID, EPI_MASK_BF16>(c, c->g3, c->pb[2], nullptr, c->g2, c->a2, s)));
   // layer 2
-  CL_RET((wgrad<C_HID, C_HID>(c, c->a1, c->g2, c->gw[1], c->gb[1], s)));
+  CL_RET(bias_grad<C_HID>(c, c->g2, c->gb[1], s));
+  CL_RET((wgrad<C_HID, C_HID>(c, c->a1, c->g2, c->gw[1], s)));
   CL_RET((conv<C_HID, C_HID, EPI_MASK_BF16>(c, c->g2, c->pb[1], nullptr, c->g1, c->a1, s)));
   // layer 1
-  return wgrad<C_IN0, C_HID>(c, c->x0, c->g1, c->gw[0], c->gb[0], s);
+  CL_RET(bias_grad<C_HID>(c, c->g1, c->gb[0], s));
+  CL_RET((wgrad<C_IN0, C_HID>(c, c->x0, c->g1, c->gw[0], s)));
+  return join_side(c, s);
 }
 
 cudaError_t adam_all(fvm_closure* c, bool update, float lr, float b1, float b2, float eps, cudaStream_t s) {
@@ -364,12 +376,8 @@ int fvm_closure_create(int n1, int n2, int n3, unsigned long long seed, fvm_clos
   c->n3 = n3;
   c->npos = (long long)n1 * n2 * n3;
   cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, dev);
-  // conv CTAs are serial load -> MMA -> epilogue chains: aim for about four
-  // resident per SM (shared memory allows 3-4) so their waits overlap
-  c->zc_conv = largest_zc(n3, (long long)(n1 / 8) * (n2 / 16), 4ll * c->nsm);
   c->zc_wg = largest_zc(n3, (long long)(n1 / 16) * (n2 / 8), 2ll * c->nsm);
-  const long long wg_blocks = (long long)(n1 / 16) * (n2 / 8) * (n3 / c->zc_wg);
-  c->partial_elems = (size_t)wg_blocks * 27 * C_HID * C_HID + (size_t)2 * c->nsm * C_HID;
+  c->partial_elems = (size_t)wgrad_chunks(c) * 27 * C_HID * C_HID;
   c->loss_blocks = 4 * c->nsm;
   int rc = FVM_OK;
   const size_t np = (size_t)c->npos;
@@ -383,6 +391,7 @@ int fvm_closure_create(int n1, int n2, int n3, unsigned long long seed, fvm_clos
   if (!rc) rc = dalloc(&c->e, np * 5);
   if (!rc) rc = dalloc(&c->ratio, np * 10);
   if (!rc) rc = dalloc(&c->partial, c->partial_elems);
+  if (!rc) rc = dalloc(&c->bias_part, (size_t)2 * c->nsm * C_HID);
   if (!rc) rc = dalloc(&c->loss_part, (size_t)c->loss_blocks);
   if (!rc) rc = dalloc(&c->loss_dev, 1);
   if (!rc) rc = dalloc(&c->status, 1);
@@ -400,7 +409,10 @@ int fvm_closure_create(int n1, int n2, int n3, unsigned long long seed, fvm_clos
     if (!rc) rc = dalloc(&c->pf[l], nw);
     if (!rc) rc = dalloc(&c->pb[l], nw);
   }
-  if (!rc && cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess)
+  if (!rc && (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
+              cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) != cudaSuccess ||
+              cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
+              cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess))
     rc = set_error(FVM_E_CUDA, "closure: stream creation failed");
   if (rc) {
     fvm_closure_destroy(c);
@@ -428,8 +440,10 @@ int fvm_closure_create(int n1, int n2, int n3, unsigned long long seed, fvm_clos
 int fvm_closure_destroy(fvm_closure* c) {
   if (!c) return FVM_OK;
   if (c->stream) cudaStreamSynchronize(c->stream);
+  if (c->side) cudaStreamSynchronize(c->side);
   void* ptrs[] = {c->x0,      c->a1,        c->a2,       c->z3,      c->g3,    c->g2,
-                  c->g1,      c->e,         c->partial,  c->loss_part, c->loss_dev, c->status, c->ratio};
+                  c->g1,      c->e,         c->partial,  c->loss_part, c->loss_dev, c->status, c->ratio,
+                  c->bias_part};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (int l = 0; l < NLAYER; ++l) {
@@ -437,6 +451,9 @@ int fvm_closure_destroy(fvm_closure* c) {
     for (void* p : lp)
       if (p) cudaFree(p);
   }
+  if (c->ev_fork) cudaEventDestroy(c->ev_fork);
+  if (c->ev_join) cudaEventDestroy(c->ev_join);
+  if (c->side) cudaStreamDestroy(c->side);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return FVM_OK;
