@@ -119,7 +119,7 @@ struct fvm_handle {
   cudaStream_t s_in = nullptr, s_out = nullptr;
   cudaEvent_t ev_in_ready = nullptr, ev_in_free = nullptr, ev_out_ready = nullptr, ev_out_free = nullptr;
   CUtensorMap tmap[3];
-  CUtensorMap smap{}, amap{};  // staged U0 / accumulator tiles of the float32 cartesian NS kernel
+  CUtensorMap smap{}, amap{};  // staged U0 / accumulator tiles (staged_kernel)
   bool legacy = false;         // batch member: runs the batched (tile-list) kernels
   unsigned long long wait_ns = 2000000000ull;  // limit of each wait for a TMA plane
   unsigned long long drain_ns = 1000000000ull; // limit of the wait for copies in flight after a timeout
@@ -140,12 +140,12 @@ int default_tile_ty(const fvm_desc& d);
 int alt_tile_ty(const fvm_desc& d);
 int tile_halo(const fvm_desc& d);
 
-// float32 cartesian Navier-Stokes grids run the register-blocked stage
-// kernels (stage_ns_strip.cuh, stage_ns_strip_visc.cuh) and float32
+// float32 Navier-Stokes grids run the register-blocked stage kernels
+// (stage_ns_strip.cuh, stage_ns_strip_visc.cuh) and float32
 // piecewise-constant heat grids stage_heat_pc.cuh; batch members keep the
 // tile-list kernels.
 bool strip_desc(const fvm_desc& d) {
-  return d.precision == FVM_FP32 && d.physics == FVM_NAVIER_STOKES && d.coords == FVM_CARTESIAN;
+  return d.precision == FVM_FP32 && d.physics == FVM_NAVIER_STOKES;
 }
 // viscous grids run it when the handle's block shape is the strip kernel's
 // (their default); the autotuner's second viscous shape is the general kernel's
@@ -213,7 +213,7 @@ int make_stage_tmap(fvm_handle* h, CUtensorMap* m, void* base, int rows) {
 }
 
 // Tensor maps of the three state buffers for the handle's tile rows (and the
-// staged-tile maps of the float32 cartesian NS kernel).
+// staged-tile maps).
 int make_tmaps(fvm_handle* h) {
   const int rows = h->tile_ty + 2 * tile_halo(h->d);
   for (int b = 0; b < 3; ++b)
@@ -265,16 +265,14 @@ int default_tile_ty(const fvm_desc& d) {
   if (heat_pc_desc(d)) return HEAT_PC_TY;
   if (d.physics == FVM_HEAT) return HEAT_TY;
   if (d.physics == FVM_MAXWELL) return f64 ? maxwell_tile_ty<double>() : MX_STRIP_TY;
-  if (f64) return visc ? ns_tile_ty<double, true>() : ns_tile_ty<double, false>();
-  return visc ? ns_tile_ty<float, true>() : ns_tile_ty<float, false>();
+  return visc ? ns_tile_ty<double, true>() : ns_tile_ty<double, false>();
 }
 int alt_tile_ty(const fvm_desc& d) {
   if (mx_strip_desc(d)) return MX_STRIP_TY_ALT;
   if (d.precision == FVM_FP64 || d.physics == FVM_MAXWELL) return default_tile_ty(d);
   if (heat_pc_desc(d)) return HEAT_PC_TY_ALT;
   if (d.physics == FVM_HEAT) return HEAT_TY_ALT;
-  if (strip_desc(d)) return d.params[1] != 0.0 ? ns_tile_ty<float, true>() : NS_STRIP_TY_ALT;
-  return d.params[1] != 0.0 ? ns_tile_ty_alt<float, true>() : ns_tile_ty_alt<float, false>();
+  return d.params[1] != 0.0 ? ns_tile_ty<float, true>() : NS_STRIP_TY_ALT;
 }
 // Halo rows staged on each side of a tile (TMA box height = rows + 2*halo).
 int tile_halo(const fvm_desc& d) {
@@ -448,12 +446,12 @@ cudaError_t launch_stage(fvm_handle* h, const StageDef& sd, bool rhs_only, bool 
       src.accmap = h->amap;
       src.p = make_ns_params<float>(h, sd, rhs_only);
       const int nbuf = (needs_u0_host(sd) ? 1 : 0) + (sd.mode == MODE_FINAL || sd.accmode == ACC_ADD ? 1 : 0);
-      return visc ? launch_ns_strip_visc(kernel_limiter(d), d.riemann, src, h->tile_ty, nbuf, h->stream, nsm)
-                  : launch_ns_strip(kernel_limiter(d), d.riemann, src, h->tile_ty, nbuf, h->stream, nsm);
+      return visc ? launch_ns_strip_visc(kernel_limiter(d), d.riemann, d.coords, src, h->tile_ty, nbuf, h->stream, nsm)
+                  : launch_ns_strip(kernel_limiter(d), d.riemann, d.coords, src, h->tile_ty, nbuf, h->stream, nsm);
     }
   }
   return launch_ns<Real>(kernel_limiter(d), d.riemann, d.coords, visc, h->tmap[sd.in],
-                         make_ns_params<Real>(h, sd, rhs_only), h->stream, nsm, h->tile_ty);
+                         make_ns_params<Real>(h, sd, rhs_only), h->stream, nsm);
 }
 
 // Ghost fill of state buffer b; `ck` (optional) also closes the step's clock.
@@ -1444,7 +1442,7 @@ int fvm_batch_create(const fvm_desc* descs, int n, fvm_batch** out) {
   int mheat_ty = 0;
   for (int i = 0; i < n && mixed; ++i) {
     const fvm_desc& d = descs[i];
-    if (strip_desc(d) && d.params[1] == 0.0) {
+    if (strip_desc(d) && d.coords == FVM_CARTESIAN && d.params[1] == 0.0) {
       if (mlim < 0) { mlim = kernel_limiter(d); mriem = d.riemann; }
       mixed = kernel_limiter(d) == mlim && d.riemann == mriem;
     } else if (heat_pc_desc(d)) {

@@ -153,6 +153,66 @@ __device__ __forceinline__ void lame_at(const Metric<Real>& m, int i, int j, Lam
   }
 }
 
+// The float32 build trades IEEE division/sqrt for the approximate SFU
+// instructions (<= 2 ulp); the float64 build keeps the reference's exact
+// operation sequence.
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// float32 metric factors of a cell for the register-blocked kernels, as
+// products of one per-column value c1 and table entries: the divergence takes
+// face areas over the cell volume, S_a / V (the x3 length cancels in S1 / V and
+// S2 / V), and the curvilinear terms the three non-zero d_a ln h_b / h_a of the
+// supported coordinates, la = dl01/h0, lb = dl02/h0, lc = dl12/h1.
+template <int COORD>
+struct ColMetric {
+  float a1p, a1m;  // S1 / V of the upper and lower x1 face
+  float c1;        // cylindrical dx1 / a1, spherical a1 / b1
+  float ir;        // 1 / r
+  __device__ __forceinline__ void load(const Metric<float>& m, int i) {
+    if constexpr (COORD == COORD_CART) {
+      a1p = a1m = __ldg(m.inv_dx1 + i);
+      c1 = ir = 0.f;
+    } else if constexpr (COORD == COORD_CYL) {
+      const float ia = rcp_approx(__ldg(m.a1 + i));
+      a1p = __ldg(m.r_f + i + 1) * ia;
+      a1m = __ldg(m.r_f + i) * ia;
+      c1 = __ldg(m.dx1 + i) * ia;
+      ir = __ldg(m.inv_r + i);
+    } else {
+      const float ib = rcp_approx(__ldg(m.b1 + i));
+      a1p = __ldg(m.r_f2 + i + 1) * ib;
+      a1m = __ldg(m.r_f2 + i) * ib;
+      c1 = __ldg(m.a1 + i) * ib;
+      ir = __ldg(m.inv_r + i);
+    }
+  }
+  // S2 / V of cell row j at its face fj (j or j + 1)
+  __device__ __forceinline__ float a2(const Metric<float>& m, int j, int fj) const {
+    if constexpr (COORD == COORD_CART) return __ldg(m.inv_dx2 + j);
+    else if constexpr (COORD == COORD_CYL) return c1 * __ldg(m.inv_dx2 + j);
+    else return (c1 * __ldg(m.sin_f2 + fj)) * rcp_approx(__ldg(m.c2 + j));
+  }
+  // S3 / V at a plane with inverse length idz
+  __device__ __forceinline__ float a3(const Metric<float>& m, int j, float idz) const {
+    if constexpr (COORD == COORD_SPH) return ((c1 * __ldg(m.dx2 + j)) * rcp_approx(__ldg(m.c2 + j))) * idz;
+    else return idz;
+  }
+  __device__ __forceinline__ float la() const { return ir; }
+  __device__ __forceinline__ float lb() const { return COORD == COORD_SPH ? ir : 0.f; }
+  __device__ __forceinline__ float lc(const Metric<float>& m, int j) const {
+    return COORD == COORD_SPH ? ir * __ldg(m.cot_c2 + j) : 0.f;
+  }
+};
+
 // ------------------------------------------------------------ limiters ----
 __device__ __forceinline__ float sgn(float x) { return x > 0.f ? 1.f : (x < 0.f ? -1.f : 0.f); }
 
@@ -182,19 +242,6 @@ __device__ __forceinline__ double limiter(double a, double b) {
   else return lim_vanleer(a, b);
 }
 // ------------------------------------------- float32 fast arithmetic ----
-// The float32 build trades IEEE division/sqrt for the approximate SFU
-// instructions (<= 2 ulp); the float64 build keeps the reference's exact
-// operation sequence.
-__device__ __forceinline__ float rcp_approx(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ float sqrt_approx(float x) {
-  float y;
-  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 template <typename R>
 __device__ __forceinline__ R recip(R x) {
   if constexpr (sizeof(R) == 4) return rcp_approx(x);

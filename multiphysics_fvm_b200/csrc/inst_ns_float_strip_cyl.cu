@@ -1,0 +1,5 @@
+// Explicit instantiation: register-blocked float32 inviscid Navier-Stokes stage kernels, COORD_CYL.
+#include "launch.cuh"
+namespace fvm {
+template cudaError_t launch_ns_strip_coord<COORD_CYL>(int, int, NsStripSource&, int, int, cudaStream_t, int);
+}

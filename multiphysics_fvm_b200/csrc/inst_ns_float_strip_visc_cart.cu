@@ -1,0 +1,5 @@
+// Explicit instantiation: register-blocked float32 viscous Navier-Stokes stage kernels, COORD_CART.
+#include "launch.cuh"
+namespace fvm {
+template cudaError_t launch_ns_strip_visc_coord<COORD_CART>(int, int, NsStripSource&, int, int, cudaStream_t, int);
+}

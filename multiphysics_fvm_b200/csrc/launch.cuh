@@ -18,15 +18,8 @@ namespace fvm {
 // float32 inviscid 8 rows (2 blocks), float64 viscous 4 rows, inviscid 8.
 template <typename Real, bool VISC>
 constexpr int ns_tile_ty() { return std::is_same<Real, double>::value ? (VISC ? 4 : 8) : (VISC ? 6 : 8); }
-// The float32 kernels also come with 4-row tiles (a second block shape for
-// the autotuner: fewer threads and less shared memory per block, more halo
-// per cell); float64 has the default shape only.
 template <typename Real, bool VISC>
-constexpr int ns_tile_ty_alt() { return std::is_same<Real, double>::value ? ns_tile_ty<Real, VISC>() : 4; }
-template <typename Real, bool VISC, int TY = ns_tile_ty<Real, VISC>()>
-constexpr int ns_min_blocks() {
-  return std::is_same<Real, double>::value ? 1 : (VISC ? 2 : (TY == 8 ? 3 : 4));
-}
+constexpr int ns_min_blocks() { return std::is_same<Real, double>::value ? 1 : (VISC ? 2 : 3); }
 constexpr int HEAT_TY = 8, HEAT_TY_ALT = 4;
 
 // Resident blocks per SM of the kernel that prepare_kernel last looked at on
@@ -50,10 +43,11 @@ static cudaError_t prepare_kernel(K kern, int threads, int bytes, int* blocks_pe
 
 // nsm < 0: only set the kernel's shared-memory attribute and query its
 // occupancy (done once, outside any stream capture).
-template <typename Real, int LIM, int RIEM, int COORD, bool VISC, class Src, int TY = ns_tile_ty<Real, VISC>()>
+template <typename Real, int LIM, int RIEM, int COORD, bool VISC, class Src>
 cudaError_t launch_ns_src(const Src& src, long long ntiles, cudaStream_t s, int nsm) {
+  constexpr int TY = ns_tile_ty<Real, VISC>();
   using C = NsCfg<Real, VISC, TY>;
-  auto kern = ns_stage_kernel<Real, LIM, RIEM, COORD, VISC, TY, ns_min_blocks<Real, VISC, TY>(), Src>;
+  auto kern = ns_stage_kernel<Real, LIM, RIEM, COORD, VISC, TY, ns_min_blocks<Real, VISC>(), Src>;
   static int bps = 0;
   if (bps == 0 || nsm < 0) {
     cudaError_t e = prepare_kernel(kern, C::NT, C::BYTES, &bps);
@@ -66,32 +60,28 @@ cudaError_t launch_ns_src(const Src& src, long long ntiles, cudaStream_t s, int 
   return cudaGetLastError();
 }
 
-// ty: tile rows of the handle (its tensor maps were built for it).
+// One grid: float64, and the viscous float32 grids' second block shape
+// (inviscid float32 grids always run the register-blocked kernel).
 template <typename Real, int LIM, int RIEM, int COORD, bool VISC>
-cudaError_t launch_ns_one(const CUtensorMap& map, NsParams<Real> p, cudaStream_t s, int nsm, int ty) {
-  constexpr int TD = ns_tile_ty<Real, VISC>(), TA = ns_tile_ty_alt<Real, VISC>();
-  SingleSource<NsParams<Real>> src;
-  src.tmap = map;
-  if constexpr (TA != TD) {
-    if (ty == TA) {
-      set_tiles(p, TA);
-      src.p = p;
-      return launch_ns_src<Real, LIM, RIEM, COORD, VISC, SingleSource<NsParams<Real>>, TA>(
-          src, tile_total(p), s, nsm);
-    }
+cudaError_t launch_ns_one(const CUtensorMap& map, NsParams<Real> p, cudaStream_t s, int nsm) {
+  if constexpr (std::is_same<Real, float>::value && !VISC) {
+    return cudaErrorInvalidValue;
+  } else {
+    SingleSource<NsParams<Real>> src;
+    src.tmap = map;
+    set_tiles(p, ns_tile_ty<Real, VISC>());
+    src.p = p;
+    return launch_ns_src<Real, LIM, RIEM, COORD, VISC>(src, tile_total(p), s, nsm);
   }
-  set_tiles(p, TD);
-  src.p = p;
-  return launch_ns_src<Real, LIM, RIEM, COORD, VISC>(src, tile_total(p), s, nsm);
 }
 
 template <typename Real, int COORD>
 cudaError_t launch_ns_coord(int lim, int riem, bool visc, const CUtensorMap& map, const NsParams<Real>& p,
-                            cudaStream_t s, int nsm, int ty) {
+                            cudaStream_t s, int nsm) {
 #define FVM_NS_CASE(L, R)                                                          \
   if (lim == L && riem == R)                                                       \
-    return visc ? launch_ns_one<Real, L, R, COORD, true>(map, p, s, nsm, ty)       \
-                : launch_ns_one<Real, L, R, COORD, false>(map, p, s, nsm, ty);
+    return visc ? launch_ns_one<Real, L, R, COORD, true>(map, p, s, nsm)           \
+                : launch_ns_one<Real, L, R, COORD, false>(map, p, s, nsm);
   FVM_NS_CASE(LIM_PC, RIEM_RUSANOV)
   FVM_NS_CASE(LIM_PC, RIEM_HLL)
   FVM_NS_CASE(LIM_MINMOD, RIEM_RUSANOV)
@@ -128,7 +118,7 @@ cudaError_t launch_ns_batch_coord(int lim, int riem, bool visc, const BatchSourc
 // Declarations of the per-(precision, coordinate) instantiations.
 #define FVM_DECLARE_NS(REAL, COORD)                                                                      \
   extern template cudaError_t launch_ns_coord<REAL, COORD>(int, int, bool, const CUtensorMap&,          \
-                                                          const NsParams<REAL>&, cudaStream_t, int, int); \
+                                                          const NsParams<REAL>&, cudaStream_t, int);    \
   extern template cudaError_t launch_ns_batch_coord<REAL, COORD>(                                        \
       int, int, bool, const BatchSource<NsParams<REAL>>&, long long, cudaStream_t, int);
 FVM_DECLARE_NS(float, COORD_CART)
@@ -148,23 +138,23 @@ cudaError_t launch_ns_batch(int lim, int riem, int coord, bool visc, const Batch
 
 template <typename Real>
 cudaError_t launch_ns(int lim, int riem, int coord, bool visc, const CUtensorMap& map, const NsParams<Real>& p,
-                      cudaStream_t s, int nsm, int ty) {
-  if (coord == COORD_CART) return launch_ns_coord<Real, COORD_CART>(lim, riem, visc, map, p, s, nsm, ty);
-  if (coord == COORD_CYL) return launch_ns_coord<Real, COORD_CYL>(lim, riem, visc, map, p, s, nsm, ty);
-  return launch_ns_coord<Real, COORD_SPH>(lim, riem, visc, map, p, s, nsm, ty);
+                      cudaStream_t s, int nsm) {
+  if (coord == COORD_CART) return launch_ns_coord<Real, COORD_CART>(lim, riem, visc, map, p, s, nsm);
+  if (coord == COORD_CYL) return launch_ns_coord<Real, COORD_CYL>(lim, riem, visc, map, p, s, nsm);
+  return launch_ns_coord<Real, COORD_SPH>(lim, riem, visc, map, p, s, nsm);
 }
 
-// ------------------------------------------------ float32 cartesian NS ----
+// ---------------------------------------------------------- float32 NS ----
 // Register-blocked stage kernel (stage_ns_strip.cuh) for float32 inviscid
-// cartesian grids, 2 rows per thread: TY = 8 (4 output warps, 3 blocks/SM at
+// grids, 2 rows per thread: TY = 8 (4 output warps, 3 blocks/SM at
 // 128 registers) or 16 (8 output warps, 2 blocks/SM).
 constexpr int NS_STRIP_TY = 8, NS_STRIP_TY_ALT = 16;
 
-template <int LIM, int RIEM, int TY>
+template <int LIM, int RIEM, int COORD, int TY>
 cudaError_t launch_ns_strip_ty(const NsStripSource& src, int nbuf, cudaStream_t s, int nsm) {
   constexpr int R = 2, NW = TY / R;
   using C = NsStripCfg<R, NW>;
-  auto kern = ns_strip_kernel<LIM, RIEM, R, NW, TY == 8 ? 3 : 2>;
+  auto kern = ns_strip_kernel<LIM, RIEM, R, NW, TY == 8 ? 3 : 2, COORD>;
   static int bps[3] = {0, 0, 0};
   if (bps[0] == 0 || nsm < 0) {
     // occupancy with 0, 1 and 2 staged tiles; the attribute ends at the largest
@@ -181,17 +171,40 @@ cudaError_t launch_ns_strip_ty(const NsStripSource& src, int nbuf, cudaStream_t 
   return cudaGetLastError();
 }
 
-template <int LIM, int RIEM>
+template <int LIM, int RIEM, int COORD>
 cudaError_t launch_ns_strip_lr(NsStripSource& src, int ty, int nbuf, cudaStream_t s, int nsm) {
   NsParams<float>& p = src.p;
   set_tiles(p, ty, p.flat != 0);
-  if (ty == NS_STRIP_TY_ALT) return launch_ns_strip_ty<LIM, RIEM, NS_STRIP_TY_ALT>(src, nbuf, s, nsm);
-  return launch_ns_strip_ty<LIM, RIEM, NS_STRIP_TY>(src, nbuf, s, nsm);
+  if (ty == NS_STRIP_TY_ALT) return launch_ns_strip_ty<LIM, RIEM, COORD, NS_STRIP_TY_ALT>(src, nbuf, s, nsm);
+  return launch_ns_strip_ty<LIM, RIEM, COORD, NS_STRIP_TY>(src, nbuf, s, nsm);
 }
 
-cudaError_t launch_ns_strip(int lim, int riem, NsStripSource& src, int ty, int nbuf, cudaStream_t s, int nsm);
+template <int COORD>
+cudaError_t launch_ns_strip_coord(int lim, int riem, NsStripSource& src, int ty, int nbuf, cudaStream_t s, int nsm) {
+#define FVM_STRIP_CASE(L, R) \
+  if (lim == L && riem == R) return launch_ns_strip_lr<L, R, COORD>(src, ty, nbuf, s, nsm);
+  FVM_STRIP_CASE(LIM_PC, RIEM_RUSANOV)
+  FVM_STRIP_CASE(LIM_PC, RIEM_HLL)
+  FVM_STRIP_CASE(LIM_MINMOD, RIEM_RUSANOV)
+  FVM_STRIP_CASE(LIM_MINMOD, RIEM_HLL)
+  FVM_STRIP_CASE(LIM_MC, RIEM_RUSANOV)
+  FVM_STRIP_CASE(LIM_MC, RIEM_HLL)
+  FVM_STRIP_CASE(LIM_VANLEER, RIEM_RUSANOV)
+  FVM_STRIP_CASE(LIM_VANLEER, RIEM_HLL)
+#undef FVM_STRIP_CASE
+  return cudaErrorInvalidValue;
+}
+extern template cudaError_t launch_ns_strip_coord<COORD_CART>(int, int, NsStripSource&, int, int, cudaStream_t, int);
+extern template cudaError_t launch_ns_strip_coord<COORD_CYL>(int, int, NsStripSource&, int, int, cudaStream_t, int);
+extern template cudaError_t launch_ns_strip_coord<COORD_SPH>(int, int, NsStripSource&, int, int, cudaStream_t, int);
+inline cudaError_t launch_ns_strip(int lim, int riem, int coord, NsStripSource& src, int ty, int nbuf, cudaStream_t s,
+                                   int nsm) {
+  return coord == COORD_CART  ? launch_ns_strip_coord<COORD_CART>(lim, riem, src, ty, nbuf, s, nsm)
+         : coord == COORD_CYL ? launch_ns_strip_coord<COORD_CYL>(lim, riem, src, ty, nbuf, s, nsm)
+                              : launch_ns_strip_coord<COORD_SPH>(lim, riem, src, ty, nbuf, s, nsm);
+}
 
-// Viscous float32 cartesian grids (stage_ns_strip_visc.cuh): 1 row per
+// Viscous float32 grids (stage_ns_strip_visc.cuh): 1 row per
 // thread, TY = 7 (7 output warps + the halo warp, 2 blocks/SM: 16 warps per SM,
 // 4 per scheduler, fit 128 registers without spills; 8 output warps left 96
 // registers and spilled, 2-row strips held 168 and ran 8 warps per SM).  It is
@@ -199,11 +212,11 @@ cudaError_t launch_ns_strip(int lim, int riem, NsStripSource& src, int ty, int n
 // (stage_ns.cuh).
 constexpr int NS_STRIP_VISC_TY = 7;
 
-template <int LIM, int RIEM, int TY>
+template <int LIM, int RIEM, int COORD, int TY>
 cudaError_t launch_ns_strip_visc_ty(const NsStripSource& src, int nbuf, cudaStream_t s, int nsm) {
   constexpr int R = 1, NW = TY / R;
   using C = NsStripViscCfg<R, NW>;
-  auto kern = ns_strip_visc_kernel<LIM, RIEM, R, NW, 2>;
+  auto kern = ns_strip_visc_kernel<LIM, RIEM, R, NW, 2, COORD>;
   static int bps[3] = {0, 0, 0};
   if (bps[0] == 0 || nsm < 0) {
     for (int nb = 0; nb < 3; ++nb) {
@@ -219,14 +232,37 @@ cudaError_t launch_ns_strip_visc_ty(const NsStripSource& src, int nbuf, cudaStre
   return cudaGetLastError();
 }
 
-template <int LIM, int RIEM>
+template <int LIM, int RIEM, int COORD>
 cudaError_t launch_ns_strip_visc_lr(NsStripSource& src, int ty, int nbuf, cudaStream_t s, int nsm) {
   NsParams<float>& p = src.p;
   set_tiles(p, ty);
-  return launch_ns_strip_visc_ty<LIM, RIEM, NS_STRIP_VISC_TY>(src, nbuf, s, nsm);
+  return launch_ns_strip_visc_ty<LIM, RIEM, COORD, NS_STRIP_VISC_TY>(src, nbuf, s, nsm);
 }
 
-cudaError_t launch_ns_strip_visc(int lim, int riem, NsStripSource& src, int ty, int nbuf, cudaStream_t s, int nsm);
+template <int COORD>
+cudaError_t launch_ns_strip_visc_coord(int lim, int riem, NsStripSource& src, int ty, int nbuf, cudaStream_t s, int nsm) {
+#define FVM_STRIP_CASE(L, R) \
+  if (lim == L && riem == R) return launch_ns_strip_visc_lr<L, R, COORD>(src, ty, nbuf, s, nsm);
+  FVM_STRIP_CASE(LIM_PC, RIEM_RUSANOV)
+  FVM_STRIP_CASE(LIM_PC, RIEM_HLL)
+  FVM_STRIP_CASE(LIM_MINMOD, RIEM_RUSANOV)
+  FVM_STRIP_CASE(LIM_MINMOD, RIEM_HLL)
+  FVM_STRIP_CASE(LIM_MC, RIEM_RUSANOV)
+  FVM_STRIP_CASE(LIM_MC, RIEM_HLL)
+  FVM_STRIP_CASE(LIM_VANLEER, RIEM_RUSANOV)
+  FVM_STRIP_CASE(LIM_VANLEER, RIEM_HLL)
+#undef FVM_STRIP_CASE
+  return cudaErrorInvalidValue;
+}
+extern template cudaError_t launch_ns_strip_visc_coord<COORD_CART>(int, int, NsStripSource&, int, int, cudaStream_t, int);
+extern template cudaError_t launch_ns_strip_visc_coord<COORD_CYL>(int, int, NsStripSource&, int, int, cudaStream_t, int);
+extern template cudaError_t launch_ns_strip_visc_coord<COORD_SPH>(int, int, NsStripSource&, int, int, cudaStream_t, int);
+inline cudaError_t launch_ns_strip_visc(int lim, int riem, int coord, NsStripSource& src, int ty, int nbuf,
+                                        cudaStream_t s, int nsm) {
+  return coord == COORD_CART  ? launch_ns_strip_visc_coord<COORD_CART>(lim, riem, src, ty, nbuf, s, nsm)
+         : coord == COORD_CYL ? launch_ns_strip_visc_coord<COORD_CYL>(lim, riem, src, ty, nbuf, s, nsm)
+                              : launch_ns_strip_visc_coord<COORD_SPH>(lim, riem, src, ty, nbuf, s, nsm);
+}
 
 // ---------------------------------------------------------------- heat ----
 template <typename Real, int LIM, int COORD, class Src, int TY = HEAT_TY>

@@ -1,4 +1,5 @@
-// Float32 cartesian Navier-Stokes stage kernel with register-blocked columns:
+// Float32 Navier-Stokes stage kernel with register-blocked columns, for every
+// coordinate system:
 // residual (navier_stokes.py:588-711) + Runge-Kutta stage combination in one
 // pass, built to issue few instructions per cell.
 //
@@ -24,7 +25,8 @@
 //      cells by the halo warp (navier_stokes.py:94-100);
 //   5. x3: slope of plane K+1 at the thread's cells and the face flux at
 //      K+1/2; the left state and the flux at K-1/2 are carried in registers;
-//   6. divergence with the inverse cell lengths, gravity, stage combination
+//   6. divergence with the face areas over the cell volume (cartesian: the
+//      inverse cell lengths), gravity and curvilinear sources, stage combination
 //      with U0 / acc from shared memory, coalesced stores;
 //   7. one block barrier per step (after it, plane K's slot is free).
 // Face values are the reference's: MUSCL slopes limiter(f_i - f_i-1,
@@ -127,12 +129,39 @@ __device__ __forceinline__ float strip_pressure(const float* u, int PL, float gm
   return gm1 * (E - ke);
 }
 
+// Geometric source of a cell (navier_stokes.py:437-452), added to s[1..3]: q =
+// {rho, m1, m2, m3, E}, pressure P and, with viscosity, the stress components
+// {t11, t22, t33, t12, t13, t23} tau[0], tau[stride], ... .
+template <int COORD>
+__device__ __forceinline__ void curvilinear_source(const ColMetric<COORD>& cm, const Metric<float>& m, int j,
+                                                   const float* q, float P, const float* tau, float* s,
+                                                   int stride = 0) {
+  const float ir = rcp_approx(q[0]), la = cm.la(), lb = cm.lb(), lc = cm.lc(m, j);
+  const float v1 = q[1] * ir, v2 = q[2] * ir, v3 = q[3] * ir;
+  float n2 = fmaf(q[2], v2, P), n3 = fmaf(q[3], v3, P), s12 = q[1] * v2, s13 = q[1] * v3, s23 = q[2] * v3;
+  (void)v1;
+  if (tau) {
+    n2 -= tau[stride];
+    n3 -= tau[2 * stride];
+    s12 -= tau[3 * stride];
+    s13 -= tau[4 * stride];
+    s23 -= tau[5 * stride];
+  }
+  s[1] = fmaf(n2, la, s[1]);
+  s[2] = fmaf(-s12, la, s[2]);
+  if constexpr (COORD == COORD_SPH) {
+    s[1] = fmaf(n3, lb, s[1]);
+    s[2] = fmaf(n3, lc, s[2]);
+    s[3] = fmaf(-s13, lb, fmaf(-s23, lc, s[3]));
+  }
+}
+
 // One piece of the stage (a run of planes of one tile column, or of row tiles
 // of a flat grid).  `bars` holds the ring
 // barriers (indices 0..2, phase bits 0..2), `gbar` the staged-tile barrier with
 // phase bit `gbit`; `phase_bits` and `pending` carry over from tile to tile.
 // Returns false when a wait ran out: the block must stop and drain.
-template <int LIM, int RIEM, int R, int NW>
+template <int LIM, int RIEM, int R, int NW, int COORD = COORD_CART>
 __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CUtensorMap* tmap,
                                               const CUtensorMap* u0map, const CUtensorMap* accmap, const Piece& pc,
                                               unsigned char* smem_raw, uint64_t* bars, uint64_t* gbar, int gbit,
@@ -172,7 +201,8 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
     const int nsteps = pc.u1 - pc.u0;
     const int Kfirst = flat ? Z0 : Z0 - 2, Plast = flat ? Zl : Zl + HH;
     const int i = x0 + lane;
-    const float idx = (is_out && i < nx) ? __ldg(p.met.inv_dx1 + i) : 0.f;
+    ColMetric<COORD> cm;
+    cm.load(p.met, min(i, nx - 1));
 
     // plane pl of the rows from yrow - HH into ring slot s
     auto issue_at = [&](int pl, int s, int yrow) {
@@ -357,12 +387,14 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
               for (int f = 0; f < NF; ++f) qr[f] = fmaf(-0.5f, s[f], fb[f]);
               strip_flux<1, RIEM>(ql, qr, gam, F);
               if (t >= 2) {
-                const float idym = __ldg(p.met.inv_dx2 + min(max(j - 1, 0), ny - 1));
+                const int jc = min(max(j - 1, 0), ny - 1);
+                const float idym = cm.a2(p.met, jc, jc + 1);
 #pragma unroll
                 for (int v = 0; v < 5; ++v) kv[t - 2][v] = fmaf(F[v], idym, kv[t - 2][v]);
               }
               if (t <= R) {
-                const float idy = __ldg(p.met.inv_dx2 + min(j, ny - 1));
+                const int jc = min(j, ny - 1);
+                const float idy = cm.a2(p.met, jc, jc);
 #pragma unroll
                 for (int v = 0; v < 5; ++v) kv[t - 1][v] = fmaf(-F[v], idy, kv[t - 1][v]);
               }
@@ -390,7 +422,8 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
               for (int v = 0; v < 5; ++v) {
                 const float fd = __shfl_down_sync(0xffffffffu, F[v], 1);
                 const float fe = lane == 31 ? fr[(par * 5 + v) * TY + ty] : fd;
-                kv[r][v] = fmaf(fe - F[v], idx, kv[r][v]);
+                if constexpr (COORD == COORD_CART) kv[r][v] = fmaf(fe - F[v], cm.a1p, kv[r][v]);
+                else kv[r][v] = fmaf(fe, cm.a1p, fmaf(-F[v], cm.a1m, kv[r][v]));
               }
             }
 #pragma unroll
@@ -459,9 +492,10 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
             if (zface) {
               float F[5];
               strip_flux<2, RIEM>(qlz[r], qr, gam, F);
+              const float a3 = cm.a3(p.met, min(y0 + ty, ny - 1), idz);
 #pragma unroll
               for (int v = 0; v < 5; ++v) {
-                kv[r][v] = fmaf(F[v] - fzp[r][v], idz, kv[r][v]);
+                kv[r][v] = fmaf(F[v] - fzp[r][v], a3, kv[r][v]);
                 fzp[r][v] = F[v];
               }
             }
@@ -491,7 +525,9 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
 #pragma unroll
               for (int v = 0; v < 5; ++v) q[v] = uK[v * PL + o];
               // gravity (navier_stokes.py:499-504): rho g and rho g.v = g.m
-              const float sg[5] = {0.f, q[0] * gx, q[0] * gy, q[0] * gz, fmaf(gx, q[1], fmaf(gy, q[2], gz * q[3]))};
+              float sg[5] = {0.f, q[0] * gx, q[0] * gy, q[0] * gz, fmaf(gx, q[1], fmaf(gy, q[2], gz * q[3]))};
+              if constexpr (COORD != COORD_CART)
+                curvilinear_source<COORD>(cm, p.met, j, q, pK[(ty + 2) * W2 + lane + 2], nullptr, sg);
               const long long g = L.idx(0, K, j + 1, i + 1);
               const int so = ty * TX + lane;
 #pragma unroll
@@ -528,7 +564,7 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
   return true;
 }
 
-template <int LIM, int RIEM, int R, int NW, int MINB>
+template <int LIM, int RIEM, int R, int NW, int MINB, int COORD>
 __global__ void __launch_bounds__(NsStripCfg<R, NW>::NT, MINB)
     ns_strip_kernel(const __grid_constant__ NsStripSource src) {
   using C = NsStripCfg<R, NW>;
@@ -557,8 +593,8 @@ __global__ void __launch_bounds__(NsStripCfg<R, NW>::NT, MINB)
   int inst;
   bool ok = true;
   while (ok && walk.next(grid, inst, pc))
-    ok = ns_strip_tile<LIM, RIEM, R, NW>(p, &src.tmap, &src.u0map, &src.accmap, pc, smem_raw, bars, bars + C::NSLOT,
-                                         C::NSLOT, phase_bits, pending);
+    ok = ns_strip_tile<LIM, RIEM, R, NW, COORD>(p, &src.tmap, &src.u0map, &src.accmap, pc, smem_raw, bars,
+                                                bars + C::NSLOT, C::NSLOT, phase_bits, pending);
   // On a timeout, wait (bounded) for every copy this block may still have in flight.
   if (!ok && tid == 0) {
     for (int s = 0; s < C::NBAR; ++s)

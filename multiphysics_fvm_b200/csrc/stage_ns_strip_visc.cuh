@@ -1,5 +1,5 @@
-// Float32 cartesian viscous Navier-Stokes stage kernel with register-blocked
-// columns: the layout of stage_ns_strip.cuh plus the Stokes stress
+// Float32 viscous Navier-Stokes stage kernel with register-blocked columns, for
+// every coordinate system: the layout of stage_ns_strip.cuh plus the Stokes stress
 // (navier_stokes.py:102-142, zero in ghost cells) reconstructed with U and P
 // (9 fields per face direction) and the centred diffusive flux
 // (diffusive_solvers.py:11-30, navier_stokes.py:217-277).
@@ -111,7 +111,7 @@ __device__ __forceinline__ void strip_flux_visc(const float* qL, const float* qR
   F[4] -= 0.5f * (eL + eR);
 }
 
-template <int LIM, int RIEM, int R, int NW, int MINB>
+template <int LIM, int RIEM, int R, int NW, int MINB, int COORD>
 __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
     ns_strip_visc_kernel(const __grid_constant__ NsStripSource src) {
   using C = NsStripViscCfg<R, NW>;
@@ -170,7 +170,8 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
     const int Z0 = 1 + pc.u0, Zl = pc.u1;
     const int Kfirst = Z0 - 3, Plast = Zl + HH;
     const int i = x0 + lane;
-    const float idx = (is_out && i < nx) ? __ldg(m.inv_dx1 + i) : 0.f;
+    ColMetric<COORD> cm;
+    cm.load(m, min(i, nx - 1));
 
     auto issue = [&](int pl) {
       const int s = pmod(pl, C::NSLOT);
@@ -207,8 +208,8 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
         const float* vm = vring + pmod(pl - 1, 3) * 3 * PL;
         const float* v0 = vring + pmod(pl, 3) * 3 * PL;
         const float* vp = vring + pmod(pl + 1, 3) * 3 * PL;
-        const float h1 = 0.5f * __ldg(m.inv_dx1 + ii), h2 = 0.5f * __ldg(m.inv_dx2 + jj);
-        const float h3 = 0.5f * __ldg(m.inv_dx3 + kk);
+        const float h1 = 0.5f * __ldg(m.inv_dx1 + ii), h2 = 0.5f * inv_len<float, COORD, 1>(m, ii, jj, kk);
+        const float h3 = 0.5f * inv_len<float, COORD, 2>(m, ii, jj, kk);
         float g[3][3];  // g[c][a] = d v_c / d x_a
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -218,6 +219,18 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
           g[c][2] = (vp[oc] - vm[oc]) * h3;
         }
         const float tt = 2.f / 3.f;
+        if constexpr (COORD != COORD_CART) {
+          // the metric terms of the diagonal gradients and of the off-diagonal sums
+          const float ir = __ldg(m.inv_r + ii), v1 = v0[o], v2 = v0[PL + o], v3 = v0[2 * PL + o];
+          g[1][1] = fmaf(v1, ir, g[1][1]);
+          g[0][1] = fmaf(-v2, ir, g[0][1]);
+          if constexpr (COORD == COORD_SPH) {
+            const float lc = ir * __ldg(m.cot_c2 + jj);
+            g[2][2] = fmaf(v1, ir, fmaf(v2, lc, g[2][2]));
+            g[0][2] = fmaf(-v3, ir, g[0][2]);
+            g[1][2] = fmaf(-v3, lc, g[1][2]);
+          }
+        }
         const float divv = (g[0][0] + g[1][1]) + g[2][2];
         t[0] = mu * (2.f * g[0][0] - tt * divv);
         t[1] = mu * (2.f * g[1][1] - tt * divv);
@@ -327,12 +340,14 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
               for (int f = 0; f < NF; ++f) qr[f] = fmaf(-0.5f, s[f], fb[f]);
               strip_flux_visc<1, RIEM>(ql, qr, gam, F);
               if (t >= 2) {
-                const float idym = __ldg(m.inv_dx2 + min(max(j - 1, 0), ny - 1));
+                const int jc = min(max(j - 1, 0), ny - 1);
+                const float idym = cm.a2(m, jc, jc + 1);
 #pragma unroll
                 for (int v = 0; v < 5; ++v) kv[t - 2][v] = fmaf(F[v], idym, kv[t - 2][v]);
               }
               if (t <= R) {
-                const float idy = __ldg(m.inv_dx2 + min(j, ny - 1));
+                const int jc = min(j, ny - 1);
+                const float idy = cm.a2(m, jc, jc);
 #pragma unroll
                 for (int v = 0; v < 5; ++v) kv[t - 1][v] = fmaf(-F[v], idy, kv[t - 1][v]);
               }
@@ -368,7 +383,8 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
               for (int v = 0; v < 5; ++v) {
                 const float fd = __shfl_down_sync(0xffffffffu, F[v], 1);
                 const float fe = lane == 31 ? fr[(par * 5 + v) * TY + ty] : fd;
-                kv[r][v] = fmaf(fe - F[v], idx, kv[r][v]);
+                if constexpr (COORD == COORD_CART) kv[r][v] = fmaf(fe - F[v], cm.a1p, kv[r][v]);
+                else kv[r][v] = fmaf(fe, cm.a1p, fmaf(-F[v], cm.a1m, kv[r][v]));
               }
             }
 #pragma unroll
@@ -494,9 +510,10 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
             if (zface) {
               float F[5];
               strip_flux_visc<2, RIEM>(qlz[r], qr, gam, F);
+              const float a3 = cm.a3(m, min(y0 + ty, ny - 1), idz);
 #pragma unroll
               for (int v = 0; v < 5; ++v) {
-                kv[r][v] = fmaf(F[v] - fzp[r][v], idz, kv[r][v]);
+                kv[r][v] = fmaf(F[v] - fzp[r][v], a3, kv[r][v]);
                 fzp[r][v] = F[v];
               }
             }
@@ -525,7 +542,11 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
               float q[5];
 #pragma unroll
               for (int v = 0; v < 5; ++v) q[v] = uK[v * PL + o];
-              const float sg[5] = {0.f, q[0] * gx, q[0] * gy, q[0] * gz, fmaf(gx, q[1], fmaf(gy, q[2], gz * q[3]))};
+              float sg[5] = {0.f, q[0] * gx, q[0] * gy, q[0] * gz, fmaf(gx, q[1], fmaf(gy, q[2], gz * q[3]))};
+              if constexpr (COORD != COORD_CART) {
+                const int op = (ty + 2) * W2 + lane + 2;
+                curvilinear_source<COORD>(cm, m, j, q, pK[op], tK + op, sg, PL2);
+              }
               const long long g = L.idx(0, K, j + 1, i + 1);
               const int so = ty * TX + lane;
 #pragma unroll
