@@ -401,6 +401,26 @@ __device__ __forceinline__ R stage_combine(const StageCoef& c, R dt, R k, R ucur
   }
 }
 
+// stage_combine and acc_update of the float32 build with the step's constants
+// formed once per launch (they are float64 in StageCoef, and dt / 6 a division):
+// every mode but MODE_SSP is base + c k.
+struct StripCoef {
+  int mode;
+  bool set;
+  float c, cb, dt, w;
+  __device__ __forceinline__ StripCoef(const StageCoef& s, float dt_) : mode(s.mode), set(s.accmode == ACC_SET), dt(dt_) {
+    c = mode == MODE_RHS ? 1.f : (mode == MODE_AXPY ? float(s.ca) * dt : (mode == MODE_FINAL ? dt / 6.f : dt));
+    cb = float(s.cb);
+    w = set ? dt / 6.f : (float(s.wacc) * dt) / 6.f;
+  }
+  __device__ __forceinline__ float combine(float k, float ucur, float u0, float acc) const {
+    if (mode == MODE_SSP) return fmaf(cb, fmaf(dt, k, ucur - u0), u0);
+    const float base = mode == MODE_AXPY ? u0 : (mode == MODE_FINAL ? acc : (mode == MODE_EULER ? ucur : 0.f));
+    return fmaf(c, k, base);
+  }
+  __device__ __forceinline__ float acc(float k, float u0, float a) const { return fmaf(w, k, set ? u0 : a); }
+};
+
 // The stage epilogue needs U0 from memory (not from the input ring)?
 template <typename R>
 __device__ __forceinline__ bool needs_u0(const StageCoef& c) {

@@ -20,10 +20,7 @@
 //      combination, stores; one block barrier.
 // The face flux F = (F_L + F_R)/2 - c (q_R - q_L)/2 is Rusanov; HLL with wave
 // speeds -c, +c is the same function for Maxwell (riemann_solvers.py:13-89).
-// The float32 MC limiter is written as copysign(k m, a + b) with
-// m = min(|a + b|/2, 2|a|, 2|b|), k = 1 when a b > 0 and 1/3 otherwise, which
-// is the reference's three-sign form (slope_limiters.py:42-73) for every sign
-// pattern.
+// Slopes and face states as in stage_ns_strip.cuh (strip_slope, strip_half).
 #pragma once
 #include "stage_ns_strip.cuh"
 #include "stage_maxwell.cuh"
@@ -63,17 +60,6 @@ struct MxStripSource {
   MaxwellParams<float> p;
 };
 
-template <int LIM>
-__device__ __forceinline__ float mx_slope(float a, float b) {
-  if constexpr (LIM == LIM_MC) {
-    const float s = a + b;
-    const float mm = fminf(0.5f * fabsf(s), 2.f * fminf(fabsf(a), fabsf(b)));
-    return copysignf(a * b > 0.f ? mm : mm * (1.f / 3.f), s);
-  } else {
-    return strip_slope<LIM>(a, b);
-  }
-}
-
 // Face flux along axis D of states q = (B1, B2, B3, D1, D2, D3):
 // (F(q_L) + F(q_R))/2 - hc (q_R - q_L) with the curl tensors of H = B/mu and
 // E = D/eps (maxwell.py:145-165); ihm = 0.5/mu, ihe = 0.5/eps, hc = c/2.
@@ -106,6 +92,7 @@ __global__ void __launch_bounds__(MxStripCfg<R, NW>::NT, MINB)
   using G = Geo<float, COORD>;
   constexpr int TX = C::TX, TY = C::TY, W = C::W, PL = C::PL, HH = C::HH, NV = C::NV;
   constexpr int WR = C::WR, PLR = C::PLR;
+  constexpr float HS = strip_half<LIM>();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   float* sm = reinterpret_cast<float*>(smem_raw);
   float* uring = sm + C::OFF_U;
@@ -135,7 +122,7 @@ __global__ void __launch_bounds__(MxStripCfg<R, NW>::NT, MINB)
   const float ihm = 0.5f / mu, ihe = 0.5f / ep, hc = 0.5f * float(p.c);
   const float imu = 1.f / mu, iep = 1.f / ep;
   const float sigma = float(p.sigma), rho_c = float(p.rho_c), chib = float(p.chi_b), chid = float(p.chi_d);
-  const float dt = float(*p.dt);
+  const StripCoef sc(p.coef, float(*p.dt));
   const bool need_u0 = needs_u0<float>(p.coef) && !p.coef.u0_is_input;
   const bool need_acc = needs_acc(p.coef);
   const unsigned stg_bytes = (need_u0 ? C::STG_BYTES : 0u) + (need_acc ? C::STG_BYTES : 0u);
@@ -271,14 +258,14 @@ __global__ void __launch_bounds__(MxStripCfg<R, NW>::NT, MINB)
             const int ty = w * R - 1 + t;
             const int j = jb - 1 + t;
             ldf(fc, ty + 1, lane);
-            const bool yghost = j < 0 || j >= ny;
+            const float hy = j < 0 || j >= ny ? 0.f : HS;  // zero slope in a ghost cell
             float s[NV];
 #pragma unroll
-            for (int f = 0; f < NV; ++f) s[f] = yghost ? 0.f : mx_slope<LIM>(fb[f] - fa[f], fc[f] - fb[f]);
+            for (int f = 0; f < NV; ++f) s[f] = strip_slope<LIM>(fb[f] - fa[f], fc[f] - fb[f]);
             if (t >= 1) {
               float qr[NV], F[NV];
 #pragma unroll
-              for (int f = 0; f < NV; ++f) qr[f] = fmaf(-0.5f, s[f], fb[f]);
+              for (int f = 0; f < NV; ++f) qr[f] = fmaf(-hy, s[f], fb[f]);
               mx_flux<1>(ql, qr, ihm, ihe, hc, F);
               if (t >= 2) {
 #pragma unroll
@@ -290,20 +277,20 @@ __global__ void __launch_bounds__(MxStripCfg<R, NW>::NT, MINB)
               }
             }
 #pragma unroll
-            for (int f = 0; f < NV; ++f) ql[f] = fmaf(0.5f, s[f], fb[f]);
+            for (int f = 0; f < NV; ++f) ql[f] = fmaf(hy, s[f], fb[f]);
             if (t >= 1 && t <= R) {
               const int r = t - 1;
               float fm[NV], fp[NV], qlx[NV], qrx[NV], F[NV];
               ldf(fm, ty, lane - 1);
               ldf(fp, ty, lane + 1);
-              const bool xghost = i >= nx;
+              const float hx = i >= nx ? 0.f : HS;
 #pragma unroll
               for (int f = 0; f < NV; ++f) {
-                const float s1 = xghost ? 0.f : mx_slope<LIM>(fb[f] - fm[f], fp[f] - fb[f]);
+                const float s1 = strip_slope<LIM>(fb[f] - fm[f], fp[f] - fb[f]);
                 const float su = __shfl_up_sync(0xffffffffu, s1, 1);
                 const float sl = lane == 0 ? hl[(par * NV + f) * TY + ty] : su;
-                qlx[f] = fmaf(0.5f, sl, fm[f]);
-                qrx[f] = fmaf(-0.5f, s1, fb[f]);
+                qlx[f] = fmaf(HS, sl, fm[f]);
+                qrx[f] = fmaf(-hx, s1, fb[f]);
               }
               mx_flux<0>(qlx, qrx, ihm, ihe, hc, F);
 #pragma unroll
@@ -336,7 +323,7 @@ __global__ void __launch_bounds__(MxStripCfg<R, NW>::NT, MINB)
             ldh(c, 0);
 #pragma unroll
             for (int f = 0; f < NV; ++f)
-              hl[(hpar * NV + f) * TY + row] = x0 == 0 ? 0.f : mx_slope<LIM>(b[f] - a[f], c[f] - b[f]);
+              hl[(hpar * NV + f) * TY + row] = x0 == 0 ? 0.f : strip_slope<LIM>(b[f] - a[f], c[f] - b[f]);
           } else {
             float F[NV] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             if (x0 + TX <= nx) {
@@ -348,10 +335,8 @@ __global__ void __launch_bounds__(MxStripCfg<R, NW>::NT, MINB)
               const bool g32 = x0 + TX >= nx;
 #pragma unroll
               for (int f = 0; f < NV; ++f) {
-                const float sm1 = mx_slope<LIM>(b[f] - a[f], c[f] - b[f]);
-                const float s0 = g32 ? 0.f : mx_slope<LIM>(c[f] - b[f], d[f] - c[f]);
-                qlh[f] = fmaf(0.5f, sm1, b[f]);
-                qrh[f] = fmaf(-0.5f, s0, c[f]);
+                qlh[f] = fmaf(HS, strip_slope<LIM>(b[f] - a[f], c[f] - b[f]), b[f]);
+                qrh[f] = fmaf(g32 ? 0.f : -HS, strip_slope<LIM>(c[f] - b[f], d[f] - c[f]), c[f]);
               }
               mx_flux<0>(qlh, qrh, ihm, ihe, hc, F);
             }
@@ -396,7 +381,7 @@ __global__ void __launch_bounds__(MxStripCfg<R, NW>::NT, MINB)
           }
         }
         // ------------------------------------------------------------ 5 ----
-        const bool zghost = K + 1 <= 0 || K + 1 >= nz + 1;
+        const float hz = K + 1 <= 0 || K + 1 >= nz + 1 ? 0.f : HS;
         const bool zface = K >= Z0 - 1;
         const float idz = outstep ? __ldg(m.inv_dx3 + (K - 1)) : 0.f;
 #pragma unroll
@@ -407,9 +392,9 @@ __global__ void __launch_bounds__(MxStripCfg<R, NW>::NT, MINB)
 #pragma unroll
           for (int f = 0; f < NV; ++f) {
             const float b0 = uK[f * PL + o], b1 = uK1[f * PL + o], b2 = uK2[f * PL + o];
-            const float s = zghost ? 0.f : mx_slope<LIM>(b1 - b0, b2 - b1);
-            qr[f] = fmaf(-0.5f, s, b1);
-            qn[f] = fmaf(0.5f, s, b1);
+            const float s = strip_slope<LIM>(b1 - b0, b2 - b1);
+            qr[f] = fmaf(-hz, s, b1);
+            qn[f] = fmaf(hz, s, b1);
           }
           if (zface) {
             float F[NV];
@@ -478,9 +463,9 @@ __global__ void __launch_bounds__(MxStripCfg<R, NW>::NT, MINB)
                 const float u0v = need_u0 ? gu0[v * TY * TX + so] : q[v];
                 const float accv = need_acc ? gacc[v * TY * TX + so] : 0.f;
                 const long long gi = g + (long long)v * L.var_stride;
-                const float o2 = stage_combine(p.coef, dt, k, q[v], u0v, accv);
+                const float o2 = sc.combine(k, q[v], u0v, accv);
                 p.out[gi] = o2;
-                if (p.coef.accmode != ACC_NONE) p.acc[gi] = acc_update(p.coef, dt, k, u0v, accv);
+                if (p.coef.accmode != ACC_NONE) p.acc[gi] = sc.acc(k, u0v, accv);
                 if (!isfinite(o2)) bad |= ST_NONFINITE;
               }
             }

@@ -78,15 +78,67 @@ struct NsStripSource {
   NsParams<float> p;
 };
 
-// Limited slope from the backward and forward differences (float32; zero
-// for piecewise constant).  minmod is the median of (a, b, 0), which equals
-// (sign a + sign b)/2 * min(|a|, |b|) (slope_limiters.py:13-39).
+// min(|a|, |b|), positive where a and b have the same sign, negative where not.
+__device__ __forceinline__ float min_xorsign(float a, float b) {
+  float d;
+  asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+  return d;
+}
+
+// Limited slope from the backward and forward differences (float32; zero for
+// piecewise constant), up to the factor 2 strip_half<LIM>: a face state is
+// f +- strip_half * strip_slope, the reference's f +- slope / 2.  The factor
+// carries the constants of the limiters (slope_limiters.py:13-105), and a ghost
+// cell's zero slope is a zero factor, one select per cell instead of one per
+// field.  The kernels are bound by issue and latency: with the limiters in
+// four to eleven instructions, a select per slope, flux vectors formed per state
+// and float64 stage constants converted per cell, the stage launches took 717 us
+// (inviscid 256^3), 1497 (viscous 256^3), 95 (97x130x61, three-sign limiter) and
+// 291 (Maxwell 128x128x256); in this form 600, 1291, 54 and 200.
+template <int LIM>
+__host__ __device__ constexpr float strip_half() {
+  return LIM == LIM_MC ? 0.25f : (LIM == LIM_VANLEER ? 1.f : 0.5f);
+}
 template <int LIM>
 __device__ __forceinline__ float strip_slope(float a, float b) {
   if constexpr (LIM == LIM_PC) return 0.f;
-  else if constexpr (LIM == LIM_MINMOD) return fmaxf(fminf(a, b), fminf(fmaxf(a, b), 0.f));
-  else if constexpr (LIM == LIM_MC) return flim_mc(a, b);
-  else return flim_vanleer(a, b);
+  else if constexpr (LIM == LIM_MINMOD) return copysignf(fmaxf(min_xorsign(a, b), 0.f), a);
+  else if constexpr (LIM == LIM_MC) {
+    // the three-sign form: opposite slopes keep a third, with the sign of a + b
+    const float s = a + b, t = min_xorsign(a, b);
+    const float m = fminf(fabsf(s), fabsf(4.f * t));
+    return copysignf(t > 0.f ? m : m * (1.f / 3.f), s);
+  } else {
+    // a b / (a + b) where a b > 0; a + b = 0 only where a b <= 0
+    const float ab = a * b;
+    return ab > 0.f ? ab * rcp_approx(a + b) : 0.f;
+  }
+}
+
+// a F(qL) + b F(qR) + c (qR - qL) of the Euler flux F along axis D, with the
+// normal velocities v and sound speeds c of the two states: F's terms all carry
+// v, so a v and b v multiply the states directly.
+template <int D, int RIEM>
+__device__ __forceinline__ void strip_combine(const float* qL, const float* qR, float vL, float vR, float cL, float cR,
+                                              float* F) {
+  float a, b, c;
+  if constexpr (RIEM == RIEM_HLL) {
+    const float sl = fminf(fminf(vL - cL, vR - cR), 0.f);
+    const float sr = fmaxf(fmaxf(vL + cL, vR + cR), 0.f);
+    const float rd = rcp_approx(fmaxf(sr - sl, 1e-30f));
+    a = sr * rd;
+    b = -sl * rd;
+    c = sl * a;
+  } else {
+    a = b = 0.5f;
+    c = -0.5f * fmaxf(fabsf(vL) + cL, fabsf(vR) + cR);
+  }
+  const float av = a * vL, bv = b * vR;
+  F[0] = fmaf(a, qL[1 + D], fmaf(b, qR[1 + D], c * (qR[0] - qL[0])));
+#pragma unroll
+  for (int k = 1; k < 4; ++k) F[k] = fmaf(av, qL[k], fmaf(bv, qR[k], c * (qR[k] - qL[k])));
+  F[1 + D] += fmaf(a, qL[5], b * qR[5]);
+  F[4] = fmaf(av, qL[4] + qL[5], fmaf(bv, qR[4] + qR[5], c * (qR[4] - qL[4])));
 }
 
 // Inviscid Riemann flux along axis D from face states q = {rho, m1, m2, m3, E, P}
@@ -96,36 +148,15 @@ __device__ __forceinline__ void strip_flux(const float* qL, const float* qR, flo
   const float irL = rcp_approx(qL[0]), irR = rcp_approx(qR[0]);
   const float vL = qL[1 + D] * irL, vR = qR[1 + D] * irR;
   const float cL = sqrt_approx((gam * qL[5]) * irL), cR = sqrt_approx((gam * qR[5]) * irR);
-  float FL[5], FR[5];
-  FL[0] = qL[1 + D];
-  FR[0] = qR[1 + D];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    FL[1 + c] = qL[1 + c] * vL;
-    FR[1 + c] = qR[1 + c] * vR;
-  }
-  FL[1 + D] += qL[5];
-  FR[1 + D] += qR[5];
-  FL[4] = (qL[4] + qL[5]) * vL;
-  FR[4] = (qR[4] + qR[5]) * vR;
-  if constexpr (RIEM == RIEM_HLL) {
-    const float sl = fminf(fminf(vL - cL, vR - cR), 0.f);
-    const float sr = fmaxf(fmaxf(vL + cL, vR + cR), 0.f);
-    const float rd = rcp_approx(fmaxf(sr - sl, 1e-30f));
-    const float a = sr * rd, b = -sl * rd, c = (sl * sr) * rd;
-#pragma unroll
-    for (int v = 0; v < 5; ++v) F[v] = fmaf(a, FL[v], fmaf(b, FR[v], c * (qR[v] - qL[v])));
-  } else {
-    const float h = 0.5f * fmaxf(fabsf(vL) + cL, fabsf(vR) + cR);
-#pragma unroll
-    for (int v = 0; v < 5; ++v) F[v] = fmaf(0.5f, FL[v] + FR[v], -h * (qR[v] - qL[v]));
-  }
+  strip_combine<D, RIEM>(qL, qR, vL, vR, cL, cR, F);
 }
 
 // P = (gamma - 1)(E - |m|^2 / (2 rho)) of one ring cell (navier_stokes.py:94-100).
+// Cells outside the ghosted grid hold zeros; the clamp keeps their P, which a
+// ghost cell's discarded slope reads, finite.
 __device__ __forceinline__ float strip_pressure(const float* u, int PL, float gm1) {
   const float rho = u[0], m1 = u[PL], m2 = u[2 * PL], m3 = u[3 * PL], E = u[4 * PL];
-  const float ke = fmaf(m1, m1, fmaf(m2, m2, m3 * m3)) * (0.5f * rcp_approx(rho));
+  const float ke = fmaf(m1, m1, fmaf(m2, m2, m3 * m3)) * (0.5f * rcp_approx(fmaxf(rho, 1e-30f)));
   return gm1 * (E - ke);
 }
 
@@ -169,6 +200,7 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
   using C = NsStripCfg<R, NW>;
   constexpr int TX = C::TX, TY = C::TY, W = C::W, PL = C::PL, HH = C::HH, NF = C::NF, W2 = C::W2;
   constexpr int PL2 = C::PL2;
+  constexpr float HS = strip_half<LIM>();
   float* sm = reinterpret_cast<float*>(smem_raw);
   float* uring = sm + C::OFF_U;
   float* pring = sm + C::OFF_P;
@@ -179,7 +211,7 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
   const Layout& L = p.lay;
   const int nx = L.nx, ny = L.ny, nz = L.nz;
   const float gam = float(p.gamma), gm1 = float(p.gamma) - 1.f;
-  const float dt = float(*p.dt);
+  const StripCoef sc(p.coef, float(*p.dt));
   const float gx = float(p.g1), gy = float(p.g2), gz = float(p.g3);
   const bool need_u0 = needs_u0<float>(p.coef) && !p.coef.u0_is_input;
   const bool need_acc = needs_acc(p.coef);
@@ -252,10 +284,8 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
             const bool g32 = x0 + TX >= nx;  // x0 + 32 is the right ghost column
 #pragma unroll
             for (int f = 0; f < NF; ++f) {
-              const float sm1 = strip_slope<LIM>(b[f] - a[f], c[f] - b[f]);
-              const float s0 = g32 ? 0.f : strip_slope<LIM>(c[f] - b[f], d[f] - c[f]);
-              ql[f] = fmaf(0.5f, sm1, b[f]);
-              qr[f] = fmaf(-0.5f, s0, c[f]);
+              ql[f] = fmaf(HS, strip_slope<LIM>(b[f] - a[f], c[f] - b[f]), b[f]);
+              qr[f] = fmaf(g32 ? 0.f : -HS, strip_slope<LIM>(c[f] - b[f], d[f] - c[f]), c[f]);
             }
             strip_flux<0, RIEM>(ql, qr, gam, F);
           }
@@ -377,14 +407,14 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
             const int ty = w * R - 1 + t;
             const int j = jb - 1 + t;
             ldf(fc, ty + 1, lane);
-            const bool yghost = j < 0 || j >= ny;
+            const float hy = j < 0 || j >= ny ? 0.f : HS;  // zero slope in a ghost cell
             float s[NF];
 #pragma unroll
-            for (int f = 0; f < NF; ++f) s[f] = yghost ? 0.f : strip_slope<LIM>(fb[f] - fa[f], fc[f] - fb[f]);
+            for (int f = 0; f < NF; ++f) s[f] = strip_slope<LIM>(fb[f] - fa[f], fc[f] - fb[f]);
             if (t >= 1) {
               float qr[NF], F[5];
 #pragma unroll
-              for (int f = 0; f < NF; ++f) qr[f] = fmaf(-0.5f, s[f], fb[f]);
+              for (int f = 0; f < NF; ++f) qr[f] = fmaf(-hy, s[f], fb[f]);
               strip_flux<1, RIEM>(ql, qr, gam, F);
               if (t >= 2) {
                 const int jc = min(max(j - 1, 0), ny - 1);
@@ -400,7 +430,7 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
               }
             }
 #pragma unroll
-            for (int f = 0; f < NF; ++f) ql[f] = fmaf(0.5f, s[f], fb[f]);
+            for (int f = 0; f < NF; ++f) ql[f] = fmaf(hy, s[f], fb[f]);
             if (t >= 1 && t <= R) {
               // x1 for own row r = t - 1 (cell i, row j): the flux through
               // the cell's left face, the right face's from the next lane
@@ -408,14 +438,14 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
               float fm[NF], fp[NF], qlx[NF], qrx[NF], F[5];
               ldf(fm, ty, lane - 1);
               ldf(fp, ty, lane + 1);
-              const bool xghost = i >= nx;  // i == nx: the right ghost column
+              const float hx = i >= nx ? 0.f : HS;  // i == nx: the right ghost column
 #pragma unroll
               for (int f = 0; f < NF; ++f) {
-                const float s1 = xghost ? 0.f : strip_slope<LIM>(fb[f] - fm[f], fp[f] - fb[f]);
+                const float s1 = strip_slope<LIM>(fb[f] - fm[f], fp[f] - fb[f]);
                 const float su = __shfl_up_sync(0xffffffffu, s1, 1);
                 const float sl = lane == 0 ? hl[(par * NF + f) * TY + ty] : su;
-                qlx[f] = fmaf(0.5f, sl, fm[f]);
-                qrx[f] = fmaf(-0.5f, s1, fb[f]);
+                qlx[f] = fmaf(HS, sl, fm[f]);
+                qrx[f] = fmaf(-hx, s1, fb[f]);
               }
               strip_flux<0, RIEM>(qlx, qrx, gam, F);
 #pragma unroll
@@ -472,7 +502,7 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
           }
           // ------------------------------------------------------------ 5 ----
           // slope of plane K+1 (zero on a ghost plane) and the flux at K+1/2
-          const bool zghost = K + 1 <= 0 || K + 1 >= nz + 1;
+          const float hz = K + 1 <= 0 || K + 1 >= nz + 1 ? 0.f : HS;
           const bool zface = K >= Z0 - 1;
           const float idz = outstep ? __ldg(p.met.inv_dx3 + (K - 1)) : 0.f;
 #pragma unroll
@@ -485,9 +515,9 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
               const float a0 = f < 5 ? uK[f * PL + o] : pK[op];
               const float a1 = f < 5 ? uK1[f * PL + o] : pK1[op];
               const float a2 = f < 5 ? uK2[f * PL + o] : pnew[r];
-              const float s = zghost ? 0.f : strip_slope<LIM>(a1 - a0, a2 - a1);
-              qr[f] = fmaf(-0.5f, s, a1);
-              qn[f] = fmaf(0.5f, s, a1);
+              const float s = strip_slope<LIM>(a1 - a0, a2 - a1);
+              qr[f] = fmaf(-hz, s, a1);
+              qn[f] = fmaf(hz, s, a1);
             }
             if (zface) {
               float F[5];
@@ -536,9 +566,9 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
                 const float u0v = need_u0 ? gu0[v * TY * TX + so] : q[v];
                 const float accv = need_acc ? gacc[v * TY * TX + so] : 0.f;
                 const long long gi = g + (long long)v * L.var_stride;
-                const float o2 = stage_combine(p.coef, dt, k, q[v], u0v, accv);
+                const float o2 = sc.combine(k, q[v], u0v, accv);
                 p.out[gi] = o2;
-                if (p.coef.accmode != ACC_NONE) p.acc[gi] = acc_update(p.coef, dt, k, u0v, accv);
+                if (p.coef.accmode != ACC_NONE) p.acc[gi] = sc.acc(k, u0v, accv);
                 if (!isfinite(o2)) bad |= ST_NONFINITE;
                 if (v == 0 && p.coef.mode != MODE_RHS && !(o2 > 0.f)) bad |= ST_DENSITY;
               }

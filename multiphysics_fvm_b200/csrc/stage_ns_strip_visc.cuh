@@ -79,30 +79,7 @@ __device__ __forceinline__ void strip_flux_visc(const float* qL, const float* qR
     vR[c] = qR[1 + c] * irR;
   }
   const float cL = sqrt_approx((gam * qL[5]) * irL), cR = sqrt_approx((gam * qR[5]) * irR);
-  float FL[5], FR[5];
-  FL[0] = qL[1 + D];
-  FR[0] = qR[1 + D];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    FL[1 + c] = qL[1 + c] * vL[D];
-    FR[1 + c] = qR[1 + c] * vR[D];
-  }
-  FL[1 + D] += qL[5];
-  FR[1 + D] += qR[5];
-  FL[4] = (qL[4] + qL[5]) * vL[D];
-  FR[4] = (qR[4] + qR[5]) * vR[D];
-  if constexpr (RIEM == RIEM_HLL) {
-    const float sl = fminf(fminf(vL[D] - cL, vR[D] - cR), 0.f);
-    const float sr = fmaxf(fmaxf(vL[D] + cL, vR[D] + cR), 0.f);
-    const float rd = rcp_approx(fmaxf(sr - sl, 1e-30f));
-    const float a = sr * rd, b = -sl * rd, c = (sl * sr) * rd;
-#pragma unroll
-    for (int v = 0; v < 5; ++v) F[v] = fmaf(a, FL[v], fmaf(b, FR[v], c * (qR[v] - qL[v])));
-  } else {
-    const float h = 0.5f * fmaxf(fabsf(vL[D]) + cL, fabsf(vR[D]) + cR);
-#pragma unroll
-    for (int v = 0; v < 5; ++v) F[v] = fmaf(0.5f, FL[v] + FR[v], -h * (qR[v] - qL[v]));
-  }
+  strip_combine<D, RIEM>(qL, qR, vL[D], vR[D], cL, cR, F);
   // diffusive flux -tau_D. and -(tau_D . v), averaged over the two states
 #pragma unroll
   for (int c = 0; c < 3; ++c) F[1 + c] -= 0.5f * (qL[6 + c] + qR[6 + c]);
@@ -117,6 +94,7 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
   using C = NsStripViscCfg<R, NW>;
   constexpr int TX = C::TX, TY = C::TY, W = C::W, PL = C::PL, HH = C::HH, NF = C::NF, W2 = C::W2;
   constexpr int PL2 = C::PL2, NT = C::NT;
+  constexpr float HS = strip_half<LIM>();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   float* sm = reinterpret_cast<float*>(smem_raw);
   float* uring = sm + C::OFF_U;
@@ -146,7 +124,7 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
   const Metric<float>& m = p.met;
   const int nx = L.nx, ny = L.ny, nz = L.nz;
   const float gam = float(p.gamma), gm1 = float(p.gamma) - 1.f, mu = float(p.mu);
-  const float dt = float(*p.dt);
+  const StripCoef sc(p.coef, float(*p.dt));
   const float gx = float(p.g1), gy = float(p.g2), gz = float(p.g3);
   const bool need_u0 = needs_u0<float>(p.coef) && !p.coef.u0_is_input;
   const bool need_acc = needs_acc(p.coef);
@@ -330,14 +308,14 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
             const int ty = w * R - 1 + t;
             const int j = jb - 1 + t;
             ldf1(fc, ty + 1, lane);
-            const bool yghost = j < 0 || j >= ny;
+            const float hy = j < 0 || j >= ny ? 0.f : HS;  // zero slope in a ghost cell
             float s[NF];
 #pragma unroll
-            for (int f = 0; f < NF; ++f) s[f] = yghost ? 0.f : strip_slope<LIM>(fb[f] - fa[f], fc[f] - fb[f]);
+            for (int f = 0; f < NF; ++f) s[f] = strip_slope<LIM>(fb[f] - fa[f], fc[f] - fb[f]);
             if (t >= 1) {
               float qr[NF], F[5];
 #pragma unroll
-              for (int f = 0; f < NF; ++f) qr[f] = fmaf(-0.5f, s[f], fb[f]);
+              for (int f = 0; f < NF; ++f) qr[f] = fmaf(-hy, s[f], fb[f]);
               strip_flux_visc<1, RIEM>(ql, qr, gam, F);
               if (t >= 2) {
                 const int jc = min(max(j - 1, 0), ny - 1);
@@ -353,7 +331,7 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
               }
             }
 #pragma unroll
-            for (int f = 0; f < NF; ++f) ql[f] = fmaf(0.5f, s[f], fb[f]);
+            for (int f = 0; f < NF; ++f) ql[f] = fmaf(hy, s[f], fb[f]);
             if (t >= 1 && t <= R) {
               // x1 for own row r = t - 1: fields with the stress row of axis 1
               const int r = t - 1;
@@ -369,14 +347,14 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
               ldf0(fm, lane - 1);
               ldf0(f0, lane);
               ldf0(fp, lane + 1);
-              const bool xghost = i >= nx;
+              const float hx = i >= nx ? 0.f : HS;
 #pragma unroll
               for (int f = 0; f < NF; ++f) {
-                const float s1 = xghost ? 0.f : strip_slope<LIM>(f0[f] - fm[f], fp[f] - f0[f]);
+                const float s1 = strip_slope<LIM>(f0[f] - fm[f], fp[f] - f0[f]);
                 const float su = __shfl_up_sync(0xffffffffu, s1, 1);
                 const float sl = lane == 0 ? hl[(par * NF + f) * TY + ty] : su;
-                qlx[f] = fmaf(0.5f, sl, fm[f]);
-                qrx[f] = fmaf(-0.5f, s1, f0[f]);
+                qlx[f] = fmaf(HS, sl, fm[f]);
+                qrx[f] = fmaf(-hx, s1, f0[f]);
               }
               strip_flux_visc<0, RIEM>(qlx, qrx, gam, F);
 #pragma unroll
@@ -425,10 +403,8 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
               const bool g32 = x0 + TX >= nx;
 #pragma unroll
               for (int f = 0; f < NF; ++f) {
-                const float sm1 = strip_slope<LIM>(b[f] - a[f], c[f] - b[f]);
-                const float s0 = g32 ? 0.f : strip_slope<LIM>(c[f] - b[f], d[f] - c[f]);
-                qlh[f] = fmaf(0.5f, sm1, b[f]);
-                qrh[f] = fmaf(-0.5f, s0, c[f]);
+                qlh[f] = fmaf(HS, strip_slope<LIM>(b[f] - a[f], c[f] - b[f]), b[f]);
+                qrh[f] = fmaf(g32 ? 0.f : -HS, strip_slope<LIM>(c[f] - b[f], d[f] - c[f]), c[f]);
               }
               strip_flux_visc<0, RIEM>(qlh, qrh, gam, F);
             }
@@ -477,7 +453,7 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
       bool step_ok = true;
       if (is_out) {
         // ------------------------------------------------------------ 5 ----
-        const bool zghost = K + 1 <= 0 || K + 1 >= nz + 1;
+        const float hz = K + 1 <= 0 || K + 1 >= nz + 1 ? 0.f : HS;
         const bool zslope = K >= Z0 - 2, zface = K >= Z0 - 1;
         const float idz = outstep ? __ldg(m.inv_dx3 + (K - 1)) : 0.f;
         if (zslope) {
@@ -503,9 +479,9 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
                 a1 = tK1[c * PL2 + op];
                 a2 = own[r][f - 5];
               }
-              const float s = zghost ? 0.f : strip_slope<LIM>(a1 - a0, a2 - a1);
-              qr[f] = fmaf(-0.5f, s, a1);
-              qn[f] = fmaf(0.5f, s, a1);
+              const float s = strip_slope<LIM>(a1 - a0, a2 - a1);
+              qr[f] = fmaf(-hz, s, a1);
+              qn[f] = fmaf(hz, s, a1);
             }
             if (zface) {
               float F[5];
@@ -555,9 +531,9 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
                 const float u0v = need_u0 ? gu0[v * TY * TX + so] : q[v];
                 const float accv = need_acc ? gacc[v * TY * TX + so] : 0.f;
                 const long long gi = g + (long long)v * L.var_stride;
-                const float o2 = stage_combine(p.coef, dt, k, q[v], u0v, accv);
+                const float o2 = sc.combine(k, q[v], u0v, accv);
                 p.out[gi] = o2;
-                if (p.coef.accmode != ACC_NONE) p.acc[gi] = acc_update(p.coef, dt, k, u0v, accv);
+                if (p.coef.accmode != ACC_NONE) p.acc[gi] = sc.acc(k, u0v, accv);
                 if (!isfinite(o2)) bad |= ST_NONFINITE;
                 if (v == 0 && p.coef.mode != MODE_RHS && !(o2 > 0.f)) bad |= ST_DENSITY;
               }
