@@ -296,16 +296,16 @@ cudaError_t launch_heat_any(int lim, int coord, const Src& src, long long ntiles
   return cudaErrorInvalidValue;
 }
 
-// Float32 piecewise-constant heat (stage_heat_pc.cuh): 4 rows per thread,
-// TY = 16 (4 warps) or 8 (2 warps); mixed-batch members also run 20 (4 x 5
-// warps) and 10 (2-row strips, 5 warps).
+// Float32 piecewise-constant heat (stage_heat_pc.cuh): 4 columns per thread,
+// TY = 16 (4 warps) or 8 (2 warps); mixed-batch members also run 20 (5 warps)
+// and 10 (2 columns per thread, 5 warps).
 constexpr int HEAT_PC_TY = 16, HEAT_PC_TY_ALT = 8;
 
 template <int COORD, int TY>
 cudaError_t launch_heat_pc_ty(const CUtensorMap& map, const HeatParams<float>& p, cudaStream_t s, int nsm) {
-  constexpr int R = TY % 4 == 0 ? 4 : 2, NW = TY / R;
-  using C = HeatPcCfg<R, NW>;
-  auto kern = heat_pc_kernel<COORD, R, NW>;
+  constexpr int VX = TY % 4 == 0 ? 4 : 2, NW = TY / VX;
+  using C = HeatPcCfg<VX, NW>;
+  auto kern = heat_pc_kernel<COORD, VX, NW>;
   static int bps = 0;
   if (bps == 0 || nsm < 0) {
     cudaError_t e = prepare_kernel(kern, C::NT, C::BYTES, &bps);

@@ -16,14 +16,14 @@
 namespace fvm {
 
 constexpr int MIX_NS_R = 2, MIX_NS_NW = 4;  // Navier-Stokes: 2-row strips, 8-row tiles
-constexpr int MIX_HEAT_NW = 5;              // heat: 4-row strips (20-row tiles) or 2-row (10-row tiles)
+constexpr int MIX_HEAT_NW = 5;              // heat: 4 columns per thread (20-row tiles) or 2 (10-row tiles)
 constexpr int MIX_NT = 160;
 constexpr int MIX_NBAR = 7;
 // Relative cost of a unit in the balanced split of the launch: a Navier-Stokes
 // plane (or row tile) of 32 x 8 cells against a heat plane of 32 x 20 (or 32 x
-// 10).  Step of 64 + 32 grids (12,275 and 40,085 units) at 1:1, 3:2, 2:1, 5:2,
-// 3:1 and 4:1: 2112, 1731, 1533, 1484, 1560 and 1728 us.
-constexpr int MIX_NS_COST = 5, MIX_HEAT_COST = 2, MIX_HEAT_COST_ALT = 1;
+// 10).  Step of 64 + 32 grids (12,275 and 40,085 units) at 5:2, 3:1, 7:2, 4:1
+// and 5:1: 1195, 1178, 1197, 1235 and 1333 us.
+constexpr int MIX_NS_COST = 6, MIX_HEAT_COST = 2, MIX_HEAT_COST_ALT = 1;
 constexpr int MIX_NS_TY = MIX_NS_R * MIX_NS_NW, MIX_HEAT_TY = 4 * MIX_HEAT_NW, MIX_HEAT_TY_ALT = 2 * MIX_HEAT_NW;
 static_assert(NsStripCfg<MIX_NS_R, MIX_NS_NW>::NT == MIX_NT && HeatPcCfg<4, MIX_HEAT_NW>::NT == MIX_NT,
               "both bodies run on the same block");
@@ -62,8 +62,8 @@ struct MixedSource {
   __device__ __forceinline__ int weight(int i) const { return inst[i].weight; }
 };
 
-// HR: heat rows per strip (4: 20-row heat tiles, 2: 10-row).
-template <int LIM, int RIEM, int HCOORD, int HR>
+// HVX: heat columns per thread (4: 20-row heat tiles, 2: 10-row).
+template <int LIM, int RIEM, int HCOORD, int HVX>
 __global__ void __launch_bounds__(MIX_NT, 3) batch_mixed_kernel(const __grid_constant__ MixedSource src) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + src.bar_off);
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(MIX_NT, 3) batch_mixed_kernel(const __grid_con
                                                          bars + 6, 6, phase_bits, pending);
     } else {
       if (in.heat.active && !*in.heat.active) continue;
-      ok = heat_pc_tile<HCOORD, HR, MIX_HEAT_NW, true>(in.heat, &in.tmap, pc, smem_raw, bars, phase_bits, pending);
+      ok = heat_pc_tile<HCOORD, HVX, MIX_HEAT_NW>(in.heat, &in.tmap, pc, smem_raw, bars, phase_bits, pending);
     }
   }
   // On a timeout, wait (bounded) for every copy this block may still have in flight.

@@ -13,17 +13,34 @@
 // cell column are formed once per tile in registers; only 1/dx3 of the plane
 // varies along the z-march.
 //
-// Tile: 32 columns x TY = NW*R rows; warp w owns rows w*R .. w*R+R-1, lane l
-// column l.  Each step reads the TMA ring (tile + 2 halo, planes K..K+2) and
-// keeps phi3 of planes K-1 and K in registers; one block barrier per step.
+// Written out per cell, each direction is three products of a coefficient and a
+// difference d_a = U_+1 - U_-1 at the cell and its two neighbours, so every
+// coefficient is formed once per tile column and the differences are shared:
+//   x1: a1+ g(i+1) d(i+1) + (a1+ - a1-) g(i) d(i) - a1- g(i-1) d(i-1), and x2 alike.
+//
+// Tile: 32 columns x TY = NW*VX rows.  A thread owns VX consecutive columns of
+// one row and reads the TMA ring (tile + 2 halo, planes K..K+2) with VX-wide
+// loads: own, left and right group, the four neighbour rows and the plane above,
+// 8 wide loads per VX cells; with one column and four rows per thread (10 loads
+// per cell, 2 barriers a plane) a 192x256x128 stage took 37.7 us, this takes
+// 24.5.  phi3 of planes K-1 and K stay in registers; one block barrier a plane.
 #pragma once
 #include "stage_heat.cuh"
 
 namespace fvm {
 
-template <int R, int NW>
+template <int VX>
+struct alignas(VX * 4) FloatVec {
+  float v[VX];
+};
+template <int VX>
+__device__ __forceinline__ FloatVec<VX> vload(const float* p) {
+  return *reinterpret_cast<const FloatVec<VX>*>(p);
+}
+
+template <int VX, int NW>
 struct HeatPcCfg {
-  static constexpr int TX = 32, TY = R * NW, NT = 32 * NW, HH = 2;
+  static constexpr int TX = 32, TY = VX * NW, NT = 32 * NW, HH = 2;
   static constexpr int W = 40;  // ring column c <-> tile x offset c - 4
   static constexpr int ROWS = TY + 2 * HH, PL = ROWS * W;
   static constexpr int NSLOT = 6;  // planes K..K+2 in use, K+3..K+5 in flight
@@ -33,213 +50,186 @@ struct HeatPcCfg {
   static_assert((SLOT * 4) % 128 == 0, "TMA destinations need 128-byte alignment");
 };
 
-// One piece of the stage (a run of planes of one tile column) with the ring barriers
-// `bars` (phase bits 0..5); `phase_bits` and `pending` carry over from tile to
-// tile.  Returns false when a wait ran out: the block must stop and drain.
-// MERGED: the two warm-up steps of the z-march (phi3 of planes Z0-1 and Z0)
-// are one prologue step.  It pays where z-chunks are short and many (the
-// batched launch); a single-grid launch of one wave of long chunks ran 2 %
-// slower with it.
-template <int COORD, int R, int NW, bool MERGED = false>
+// One piece of the stage (a run of planes of one tile column) with the ring
+// barriers `bars` (phase bits 0..5); `phase_bits` and `pending` carry over from
+// piece to piece.  Returns false when a wait ran out: the block must stop and drain.
+template <int COORD, int VX, int NW>
 __device__ __forceinline__ bool heat_pc_tile(const HeatParams<float>& p, const CUtensorMap* tmap, const Piece& pc,
                                              unsigned char* smem_raw, uint64_t* bars, unsigned& phase_bits,
                                              unsigned& pending) {
-  using C = HeatPcCfg<R, NW>;
-  using G = Geo<float, COORD>;
-  constexpr int TX = C::TX, TY = C::TY, W = C::W, HH = C::HH;
+  using C = HeatPcCfg<VX, NW>;
+  using V = FloatVec<VX>;
+  constexpr int TX = C::TX, TY = C::TY, W = C::W, HH = C::HH, LX = TX / VX;  // LX lanes per row
   float* uring = reinterpret_cast<float*>(smem_raw);
   const int tid = threadIdx.x;
   const Layout& L = p.lay;
   const Metric<float>& m = p.met;
   const int nx = L.nx, ny = L.ny, nz = L.nz;
-  const float qsrc = float(p.q), dt = float(*p.dt);
-  const float kap = float(p.k * p.inv_rho_cp);  // k / (rho cp)
+  const float qsrc = float(p.q);
+  const StripCoef sc(p.coef, float(*p.dt));
+  const float gk = -0.5f * float(p.k * p.inv_rho_cp);  // phi = gk / L * (U_+1 - U_-1)
   const bool need_u0 = needs_u0<float>(p.coef) && !p.coef.u0_is_input;
   const bool need_acc = needs_acc(p.coef);
   const int w = tid >> 5, lane = tid & 31;
-  {
-    const int x0 = (pc.col % p.ntx) * TX, y0 = (pc.col / p.ntx) * TY;
-    const int Z0 = 1 + pc.u0, Zl = pc.u1;
-    const int Kfirst = Z0 - 2, Plast = Zl + 2;
-    const int i = x0 + lane, jb = y0 + w * R;
-    const bool icol = i < nx;
-    const int ic = min(i, nx - 1);  // metric index of this column (garbage lanes clamp)
+  const int x0 = (pc.col % p.ntx) * TX, y0 = (pc.col / p.ntx) * TY;
+  const int Z0 = 1 + pc.u0, Zl = pc.u1;
+  const int Kfirst = Z0 - 2, Plast = Zl + 2;
+  const int ty = w * VX + lane / LX, tx = (lane % LX) * VX;
+  const int i0 = x0 + tx, j = y0 + ty;
 
-    auto issue = [&](int pl) {
-      const int s = pmod(pl, C::NSLOT);
+  int next_pl = Kfirst;  // the next plane to issue (thread 0)
+  auto issue_to = [&](int last) {
+    for (; next_pl <= last && next_pl <= Plast; ++next_pl) {
+      const int s = pmod(next_pl, C::NSLOT);
       pending |= 1u << s;
       fence_proxy_async();
       mbar_arrive_expect_tx(&bars[s], C::TX_BYTES + p.extra_tx);
-      tma_load_4d(&uring[s * C::SLOT], tmap, &bars[s], x0 - 3 + L.padx, y0 + 1 - HH, pl, 0);
-    };
-    if (tid == 0)
-      for (int pl = Kfirst; pl <= Kfirst + C::NSLOT - 1 && pl <= Plast; ++pl) issue(pl);
+      tma_load_4d(&uring[s * C::SLOT], tmap, &bars[s], x0 - 3 + L.padx, y0 + 1 - HH, next_pl, 0);
+    }
+  };
+  if (tid == 0) issue_to(Kfirst + C::NSLOT - 1);
 
-    // per-column and per-row metric factors (zero g in ghost cells: phi is
-    // zero-padded there)
-    const float g1m = (i - 1 >= 0 && i - 1 < nx) ? -0.5f * kap * __ldg(m.inv_dx1 + i - 1) : 0.f;
-    const float g10 = icol ? -0.5f * kap * __ldg(m.inv_dx1 + i) : 0.f;
-    const float g1p = (i + 1 < nx) ? -0.5f * kap * __ldg(m.inv_dx1 + i + 1) : 0.f;
-    float g2[R + 2];  // rows jb-1 .. jb+R
+  // coefficients of the own cells (clamped indices in lanes outside the grid;
+  // zero where a neighbour is a ghost cell: phi is zero-padded there)
+  const int jc = min(j, ny - 1);
+  auto gx = [&](int i) { return i >= 0 && i < nx ? gk * __ldg(m.inv_dx1 + i) : 0.f; };
+  auto gy = [&](int jj) { return jj >= 0 && jj < ny ? gk * __ldg(m.inv_dx2 + jj) : 0.f; };
+  float cxm[VX], cx0[VX], cxp[VX], cy[VX], cz[VX];
 #pragma unroll
-    for (int t = 0; t < R + 2; ++t) {
-      const int j = jb - 1 + t;
-      g2[t] = (icol && j >= 0 && j < ny) ? -0.5f * kap * inv_len<float, COORD, 1>(m, i, j, 0) : 0.f;
-    }
-    float a1p[R], a1m[R], a2p[R], a2m[R], a3[R], g3[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int jc = min(jb + r, ny - 1);
-      // V and the face areas at plane 0; their x3 factor dx3 cancels in S1/V
-      // and S2/V, and S3/V scales with 1/dx3 of the plane
-      const float iv = 0.5f / G::V(m, ic, jc, 0);
-      a1p[r] = G::S1(m, ic + 1, jc, 0) * iv;
-      a1m[r] = G::S1(m, ic, jc, 0) * iv;
-      a2p[r] = G::S2(m, ic, jc + 1, 0) * iv;
-      a2m[r] = G::S2(m, ic, jc, 0) * iv;
-      a3[r] = G::S3(m, ic, jc) * iv * __ldg(m.dx3);
-      g3[r] = -0.5f * kap;
-      if constexpr (COORD == COORD_SPH) g3[r] *= __ldg(m.inv_r + ic) * __ldg(m.inv_sin_c2 + jc);
-    }
-    // phi3 of plane P at the own cells from the ring planes P-1 (um) and P+1
-    // (up); zero on a ghost plane
-    auto phi3 = [&](int P, const float* um, const float* up, float* out) {
-      const bool zg = P <= 0 || P >= nz + 1;
-      const float idz1 = zg ? 0.f : __ldg(m.inv_dx3 + min(max(P - 1, 0), nz - 1));
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int o = (w * R + r + HH) * W + lane + 4;
-        out[r] = (g3[r] * idz1) * (up[o] - um[o]);
-      }
-    };
-    float phz0[R], phz1[R];  // phi3 of planes K-1 and K at the own cells
-#pragma unroll
-    for (int r = 0; r < R; ++r) { phz0[r] = 0.f; phz1[r] = 0.f; }
-    if constexpr (MERGED) {
-      // prologue: planes Z0-2 .. Z0+1 give phi3 of planes Z0-1 and Z0 in one
-      // step (one set of waits and one barrier pair for both)
-      bool got = true;
-      for (int pl = Kfirst; pl <= Kfirst + 3; ++pl) {
-        const int s = pmod(pl, C::NSLOT);
-        const bool g = got && mbar_wait_bounded(&bars[s], (phase_bits >> s) & 1u, p.wait_ns);
-        if (g) {
-          phase_bits ^= 1u << s;
-          if (tid == 0) pending &= ~(1u << s);
-        }
-        got = g;
-      }
-      if (!__syncthreads_and(got)) {
-        if (tid == 0) atomicOr(p.status, ST_TMA_TIMEOUT);
-        return false;
-      }
-      phi3(Z0 - 1, uring + pmod(Kfirst, C::NSLOT) * C::SLOT, uring + pmod(Kfirst + 2, C::NSLOT) * C::SLOT, phz0);
-      phi3(Z0, uring + pmod(Kfirst + 1, C::NSLOT) * C::SLOT, uring + pmod(Kfirst + 3, C::NSLOT) * C::SLOT, phz1);
-      __syncthreads();  // planes Z0-2 and Z0-1 are refilled at the first step
-    }
+  for (int c = 0; c < VX; ++c) {
+    const int ic = min(i0 + c, nx - 1);
+    ColMetric<COORD> cm;
+    cm.load(m, ic);
+    const float c1 = COORD == COORD_CART ? 1.f : cm.c1;
+    cxp[c] = 0.5f * cm.a1p * gx(i0 + c + 1);
+    cxm[c] = -0.5f * cm.a1m * gx(i0 + c - 1);
+    cx0[c] = 0.5f * (cm.a1p - cm.a1m) * gx(ic);
+    cy[c] = 0.5f * c1 * (COORD == COORD_CART ? 1.f : cm.ir);
+    cz[c] = 0.5f * gk;
+    if constexpr (COORD == COORD_SPH)
+      cz[c] *= (c1 * __ldg(m.dx2 + jc)) * rcp_approx(__ldg(m.c2 + jc)) * (cm.ir * __ldg(m.inv_sin_c2 + jc));
+  }
+  // S2 / V without its column factor, at the upper and lower x2 face
+  float pu, pl_;
+  if constexpr (COORD == COORD_SPH) {
+    const float ic2 = rcp_approx(__ldg(m.c2 + jc));
+    pu = __ldg(m.sin_f2 + jc + 1) * ic2;
+    pl_ = __ldg(m.sin_f2 + jc) * ic2;
+  } else {
+    pu = pl_ = __ldg(m.inv_dx2 + jc);
+  }
+  const float cyp = pu * gy(j + 1), cy0 = (pu - pl_) * gy(jc), cym = -pl_ * gy(j - 1);
 
-    const int K0 = MERGED ? Z0 : Kfirst;
-    int next_pl = Kfirst + C::NSLOT;  // MERGED: the next plane to issue (thread 0)
-    for (int K = K0, sK = pmod(K0, C::NSLOT); K <= Zl; ++K, sK = (sK == C::NSLOT - 1 ? 0 : sK + 1)) {
-      if constexpr (MERGED) {
-        // the prologue freed two slots: the first step refills both
-        if (tid == 0)
-          for (; next_pl <= K + C::NSLOT - 1 && next_pl <= Plast; ++next_pl) issue(next_pl);
-      } else {
-        if (tid == 0 && K > Kfirst && K + C::NSLOT - 1 <= Plast) issue(K + C::NSLOT - 1);
+  const int o = (ty + HH) * W + tx + 4;
+  auto ring = [&](int pl) { return uring + pmod(pl, C::NSLOT) * C::SLOT; };
+  auto wait_planes = [&](int first, int last) {
+    bool got = true;
+    for (int pl = first; pl <= last; ++pl) {
+      const int s = pmod(pl, C::NSLOT);
+      const bool g = got && mbar_wait_bounded(&bars[s], (phase_bits >> s) & 1u, p.wait_ns);
+      if (g) {
+        phase_bits ^= 1u << s;
+        if (tid == 0) pending &= ~(1u << s);
       }
-      const bool outstep = MERGED || K >= Z0;  // the merged loop starts at Z0
-      // U0 / acc of the plane's own cells, loaded before anything is stored
-      // in this step so that the step hides their latency
-      float eu0[R], eacc[R];
+      got = g;
+    }
+    if (!__syncthreads_and(got)) {
+      if (tid == 0) atomicOr(p.status, ST_TMA_TIMEOUT);
+      return false;
+    }
+    return true;
+  };
+  // 1/dx3 of ghosted plane P, zero on a ghost plane
+  auto idz_of = [&](int P) { return P <= 0 || P >= nz + 1 ? 0.f : __ldg(m.inv_dx3 + P - 1); };
+  V ph0, ph1;  // d3 / dx3 of planes K-1 and K
+  if (!wait_planes(Kfirst, Kfirst + 3)) return false;
+  {
+    const V um = vload<VX>(ring(Z0 - 2) + o), u0 = vload<VX>(ring(Z0 - 1) + o), u1 = vload<VX>(ring(Z0) + o),
+            u2 = vload<VX>(ring(Z0 + 1) + o);
+    const float za = idz_of(Z0 - 1), zb = idz_of(Z0);
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        eu0[r] = 0.f;
-        eacc[r] = 0.f;
-        if (outstep && icol && jb + r < ny) {
-          const long long g = L.idx(0, K, jb + r + 1, i + 1);
-          if (need_u0) eu0[r] = p.u0[g];
-          if (need_acc) eacc[r] = p.acc[g];
-        }
-      }
-      {
-        bool got = true;
-        for (int pl = (!MERGED && K == Kfirst ? Kfirst : K + 2); pl <= K + 2; ++pl) {
-          const int s = pmod(pl, C::NSLOT);
-          const bool g = got && mbar_wait_bounded(&bars[s], (phase_bits >> s) & 1u, p.wait_ns);
-          if (g) {
-            phase_bits ^= 1u << s;
-            if (tid == 0) pending &= ~(1u << s);
-          }
-          got = g;
-        }
-        if (!__syncthreads_and(got)) {
-          if (tid == 0) atomicOr(p.status, ST_TMA_TIMEOUT);
-          return false;
-        }
-      }
-      const int s2 = sK + 2 >= C::NSLOT ? sK + 2 - C::NSLOT : sK + 2;
-      const float* uK = uring + sK * C::SLOT;
-      const float* uK2 = uring + s2 * C::SLOT;
-      float phz2[R];  // phi3 of plane K+1 at the own cells (zero on a ghost plane)
-      if constexpr (MERGED) {
-        phi3(K + 1, uK, uK2, phz2);
-      } else {
-        // 1/dx3 of interior plane K (ghosted K+1)
-        const bool zg = K + 1 <= 0 || K + 1 >= nz + 1;
-        const float idz1 = zg ? 0.f : __ldg(m.inv_dx3 + min(max(K, 0), nz - 1));
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int o = (w * R + r + HH) * W + lane + 4;
-          phz2[r] = (g3[r] * idz1) * (uK2[o] - uK[o]);
-        }
-      }
-      if (outstep) {
-        const float idz = __ldg(m.inv_dx3 + (K - 1));
-        // x2: phi2 along the strip (rows jb-1 .. jb+R) from the ring
-        float ph2[R + 2];
-#pragma unroll
-        for (int t = 0; t < R + 2; ++t) {
-          const int o = (w * R - 1 + t + HH) * W + lane + 4;
-          ph2[t] = g2[t] * (uK[o + W] - uK[o - W]);
-        }
-        unsigned bad = 0;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int o = (w * R + r + HH) * W + lane + 4;
-          const float um2 = uK[o - 2], um1 = uK[o - 1], u0c = uK[o], up1 = uK[o + 1], up2 = uK[o + 2];
-          const float p1m = g1m * (u0c - um2), p10 = g10 * (up1 - um1), p1p = g1p * (up2 - u0c);
-          float div = a1p[r] * (p10 + p1p) - a1m[r] * (p1m + p10);
-          div = fmaf(a2p[r], ph2[r + 1] + ph2[r + 2], div);
-          div = fmaf(-a2m[r], ph2[r] + ph2[r + 1], div);
-          div = fmaf(a3[r] * idz, phz2[r] - phz0[r], div);
-          const int j = jb + r;
-          if (icol && j < ny) {
-            const float k = qsrc - div;
-            const long long gi = L.idx(0, K, j + 1, i + 1);
-            const float u0v = need_u0 ? eu0[r] : u0c;
-            const float o2 = stage_combine(p.coef, dt, k, u0c, u0v, eacc[r]);
-            p.out[gi] = o2;
-            if (p.coef.accmode != ACC_NONE) p.acc[gi] = acc_update(p.coef, dt, k, u0v, eacc[r]);
-            if (!isfinite(o2)) bad |= ST_NONFINITE;
-          }
-        }
-        if (bad) atomicOr(p.status, bad);
-      }
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        phz0[r] = phz1[r];
-        phz1[r] = phz2[r];
-      }
-      __syncthreads();  // plane K's slot is refilled at the next step
+    for (int c = 0; c < VX; ++c) {
+      ph0.v[c] = za * (u1.v[c] - um.v[c]);
+      ph1.v[c] = zb * (u2.v[c] - u0.v[c]);
     }
   }
+  const bool in_y = j < ny, full = i0 + VX <= nx;
+  for (int K = Z0, sK = pmod(Z0, C::NSLOT); K <= Zl; ++K, sK = (sK == C::NSLOT - 1 ? 0 : sK + 1)) {
+    // U0 / acc of the own cells, before anything is stored in this step (rows
+    // are padded to whole 16-byte groups, so the wide load stays in its row)
+    V u0v, accv;
+    const long long g = L.idx(0, K, j + 1, i0 + 1);
+    const bool in = in_y && i0 < nx;
+    if (in && need_u0) u0v = vload<VX>(p.u0 + g);
+    if (in && need_acc) accv = vload<VX>(p.acc + g);
+    if (!wait_planes(K + 2, K + 2)) return false;
+    // every thread has left step K-1: its slot (on the first step, both planes
+    // below Z0) takes the next copies
+    if (tid == 0) issue_to(K + C::NSLOT - 1);
+    const int s2 = sK + 2 >= C::NSLOT ? sK + 2 - C::NSLOT : sK + 2;
+    const float* uK = uring + sK * C::SLOT + o;
+    const V uc = vload<VX>(uK), up = vload<VX>(uring + s2 * C::SLOT + o);
+    float ux[VX + 4];  // columns i0-2 .. i0+VX+1
+    {
+      const V l = vload<VX>(uK - VX), r = vload<VX>(uK + VX);
+      ux[0] = l.v[VX - 2];
+      ux[1] = l.v[VX - 1];
+#pragma unroll
+      for (int c = 0; c < VX; ++c) ux[2 + c] = uc.v[c];
+      ux[VX + 2] = r.v[0];
+      ux[VX + 3] = r.v[1];
+    }
+    float d[VX + 2];  // x1 differences at columns i0-1 .. i0+VX
+#pragma unroll
+    for (int c = 0; c < VX + 2; ++c) d[c] = ux[c + 2] - ux[c];
+    const V r1 = vload<VX>(uK + W), r2 = vload<VX>(uK + 2 * W), l1 = vload<VX>(uK - W), l2 = vload<VX>(uK - 2 * W);
+    const float idz = __ldg(m.inv_dx3 + (K - 1)), idz1 = idz_of(K + 1);
+    float out[VX], ac[VX];
+    bool fin = true;
+#pragma unroll
+    for (int c = 0; c < VX; ++c) {
+      float div = fmaf(cxp[c], d[c + 2], fmaf(cx0[c], d[c + 1], cxm[c] * d[c]));
+      const float dy = fmaf(cyp, r2.v[c] - uc.v[c], fmaf(cy0, r1.v[c] - l1.v[c], cym * (uc.v[c] - l2.v[c])));
+      div = fmaf(cy[c], dy, div);
+      const float ph2 = idz1 * (up.v[c] - uc.v[c]);
+      div = fmaf(cz[c] * idz, ph2 - ph0.v[c], div);
+      ph0.v[c] = ph1.v[c];
+      ph1.v[c] = ph2;
+      const float k = qsrc - div, b = need_u0 ? u0v.v[c] : uc.v[c], a = need_acc ? accv.v[c] : 0.f;
+      out[c] = sc.combine(k, uc.v[c], b, a);
+      ac[c] = sc.acc(k, b, a);
+      if (i0 + c < nx) fin = fin && isfinite(out[c]);
+    }
+    if (in) {
+      if (full) {
+        V ov;
+#pragma unroll
+        for (int c = 0; c < VX; ++c) ov.v[c] = out[c];
+        *reinterpret_cast<V*>(p.out + g) = ov;
+        if (p.coef.accmode != ACC_NONE) {
+#pragma unroll
+          for (int c = 0; c < VX; ++c) ov.v[c] = ac[c];
+          *reinterpret_cast<V*>(p.acc + g) = ov;
+        }
+      } else {
+#pragma unroll
+        for (int c = 0; c < VX; ++c)
+          if (i0 + c < nx) {
+            p.out[g + c] = out[c];
+            if (p.coef.accmode != ACC_NONE) p.acc[g + c] = ac[c];
+          }
+      }
+      if (!fin) atomicOr(p.status, ST_NONFINITE);
+    }
+  }
+  __syncthreads();  // the next piece's first copies reuse every slot
   return true;
 }
 
-template <int COORD, int R, int NW>
-__global__ void __launch_bounds__(HeatPcCfg<R, NW>::NT)
+template <int COORD, int VX, int NW>
+__global__ void __launch_bounds__(HeatPcCfg<VX, NW>::NT)
     heat_pc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ HeatParams<float> p) {
-  using C = HeatPcCfg<R, NW>;
+  using C = HeatPcCfg<VX, NW>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + C::NSLOT * C::SLOT * 4);
   if (smem_u32(smem_raw) & 127u) {
@@ -260,7 +250,7 @@ __global__ void __launch_bounds__(HeatPcCfg<R, NW>::NT)
   Piece pc;
   int inst;
   bool ok = true;
-  while (ok && walk.next(grid, inst, pc)) ok = heat_pc_tile<COORD, R, NW>(p, &tmap, pc, smem_raw, bars, phase_bits, pending);
+  while (ok && walk.next(grid, inst, pc)) ok = heat_pc_tile<COORD, VX, NW>(p, &tmap, pc, smem_raw, bars, phase_bits, pending);
   if (!ok && tid == 0)
     for (int s = 0; s < C::NSLOT; ++s)
       if ((pending >> s) & 1u) mbar_wait_bounded(&bars[s], (phase_bits >> s) & 1u, p.drain_ns);
