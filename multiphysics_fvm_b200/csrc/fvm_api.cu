@@ -139,6 +139,7 @@ namespace {
 int default_tile_ty(const fvm_desc& d);
 int alt_tile_ty(const fvm_desc& d);
 int tile_halo(const fvm_desc& d);
+bool former_tile_ty(const fvm_desc& d);
 
 // float32 Navier-Stokes grids run the register-blocked stage kernels
 // (stage_ns_strip.cuh, stage_ns_strip_visc.cuh) and float32
@@ -239,7 +240,7 @@ int validate(const fvm_desc* d) {
   if (d->limiter < 0 || d->limiter > 2) return fail(FVM_E_INVALID, "unknown slope limiter");
   if (d->riemann < 0 || d->riemann > 1) return fail(FVM_E_INVALID, "unknown riemann solver");
   if (d->integrator < 0 || d->integrator > 3) return fail(FVM_E_INVALID, "unknown time integrator");
-  if (d->tile_ty != 0 && d->tile_ty != default_tile_ty(*d) && d->tile_ty != alt_tile_ty(*d))
+  if (d->tile_ty != 0 && d->tile_ty != default_tile_ty(*d) && d->tile_ty != alt_tile_ty(*d) && !former_tile_ty(*d))
     return fail(FVM_E_INVALID, "tile_ty must be 0 (default), " + std::to_string(default_tile_ty(*d)) + " or " +
                                    std::to_string(alt_tile_ty(*d)) + " for this physics and precision");
   const int nv = d->physics == FVM_NAVIER_STOKES ? 5 : (d->physics == FVM_HEAT ? 1 : 6);
@@ -273,6 +274,12 @@ int alt_tile_ty(const fvm_desc& d) {
   if (heat_pc_desc(d)) return HEAT_PC_TY_ALT;
   if (d.physics == FVM_HEAT) return HEAT_TY_ALT;
   return d.params[1] != 0.0 ? ns_tile_ty<float, true>() : NS_STRIP_TY_ALT;
+}
+// Block shapes that earlier kernels of this library had: a descriptor that asks
+// for one is still taken and runs the default shape.
+bool former_tile_ty(const fvm_desc& d) {
+  if (d.physics != FVM_NAVIER_STOKES || d.tile_ty != 4) return false;
+  return d.precision == FVM_FP64 ? d.params[1] != 0.0 : d.coords != FVM_CARTESIAN;
 }
 // Halo rows staged on each side of a tile (TMA box height = rows + 2*halo).
 int tile_halo(const fvm_desc& d) {
@@ -697,7 +704,7 @@ int fvm_create(const fvm_desc* desc, fvm_handle** out) {
   FVM_CKC(cudaMallocHost(&h->stage_host, h->stage_elems * sizeof(double)));
   h->device_bytes += h->stage_elems * sizeof(double);
 #undef FVM_CKC
-  h->tile_ty = d.tile_ty > 0 ? d.tile_ty : default_tile_ty(d);
+  h->tile_ty = d.tile_ty > 0 && !former_tile_ty(d) ? d.tile_ty : default_tile_ty(d);
   rc = make_tmaps(h);
   if (rc) {
     fvm_destroy(h);

@@ -14,10 +14,12 @@
 namespace fvm {
 
 // Tile rows of the Navier-Stokes kernel and the blocks per SM it is built
-// for: float32 viscous 6 rows (2 blocks of 256 threads, ~109 KB each),
-// float32 inviscid 8 rows (2 blocks), float64 viscous 4 rows, inviscid 8.
+// for: viscous 6 rows (float32 2 blocks of 256 threads, ~109 KB each; float64
+// one, 215 KB: 4 rows, 6 warps per SM and twice the stress per cell took 529 us
+// where 6 rows take 372, 96^3), inviscid 8 rows (float32 3 blocks; float64 one:
+// two blocks of 4 rows ran the same, 177 us at 96^3 minmod).
 template <typename Real, bool VISC>
-constexpr int ns_tile_ty() { return std::is_same<Real, double>::value ? (VISC ? 4 : 8) : (VISC ? 6 : 8); }
+constexpr int ns_tile_ty() { return VISC ? 6 : 8; }
 template <typename Real, bool VISC>
 constexpr int ns_min_blocks() { return std::is_same<Real, double>::value ? 1 : (VISC ? 2 : 3); }
 constexpr int HEAT_TY = 8, HEAT_TY_ALT = 4;
