@@ -104,6 +104,12 @@ int fvm_upload(fvm_handle* h, const double* host_state);
  * (src/io.py:14-63). */
 int fvm_download(fvm_handle* h, double* host_state);
 
+/* The same copies from and into one array per variable, (nx1+2, nx2+2, nx3+2)
+ * each, in variable order: the reference's dict of arrays as it stands
+ * (src/solver.py:64-85 fills it, src/io.py:14-63 reads it). */
+int fvm_upload_vars(fvm_handle* h, const double* const* host_vars);
+int fvm_download_vars(fvm_handle* h, double* const* host_vars);
+
 /* Pipelined transfers: the same copies as fvm_upload / fvm_download (the
  * downloaded ghost edges and corners are averaged on the device, as
  * src/solver.py:39-61), enqueued without waiting.  Uploads run on their own

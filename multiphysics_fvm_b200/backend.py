@@ -89,10 +89,13 @@ def bc_codes(name: str, bcs: dict):
 
 
 def _key(x):
-    if isinstance(x, dict):
-        return tuple(sorted((k, _key(v)) for k, v in x.items()))
+    t = type(x)
+    if t is float or t is int or t is str:
+        return x
+    if t is dict or isinstance(x, dict):
+        return tuple([(k, _key(x[k])) for k in sorted(x)])
     if isinstance(x, (list, tuple)):
-        return tuple(_key(v) for v in x)
+        return tuple([_key(v) for v in x])
     if callable(x):
         return (getattr(x, "__module__", None), getattr(x, "__name__", None), getattr(x, "_fvm_id", None))
     return x
@@ -180,17 +183,21 @@ class Simulation:
                    precision=setup.get("precision", "fp64"), **kw)
 
     # -- state transfer ----------------------------------------------------
-    def _stack(self, U) -> np.ndarray:
-        if isinstance(U, dict):
-            arr = np.stack([np.asarray(U[k], dtype=np.float64) for k in self.variables])
-        else:
-            arr = np.asarray(U, dtype=np.float64)
-        if arr.shape != self._ghosted:
-            raise ValueError(f"state shape {arr.shape} != {self._ghosted}")
-        return np.ascontiguousarray(arr)
+    def _pointers(self, arrays):
+        """Array of the variables' data pointers (the arrays must outlive it)."""
+        return (C.c_void_p * self.nv)(*[a.ctypes.data for a in arrays])
 
     def upload(self, U):
-        arr = self._stack(U)
+        if isinstance(U, dict):
+            arrays = [np.ascontiguousarray(U[k], dtype=np.float64) for k in self.variables]
+            for a in arrays:
+                if a.shape != self._ghosted[1:]:
+                    raise ValueError(f"state shape {(len(arrays),) + a.shape} != {self._ghosted}")
+            L.check(self._lib.fvm_upload_vars(self._h, self._pointers(arrays)), "fvm_upload")
+            return
+        arr = np.ascontiguousarray(U, dtype=np.float64)
+        if arr.shape != self._ghosted:
+            raise ValueError(f"state shape {arr.shape} != {self._ghosted}")
         L.check(self._lib.fvm_upload(self._h, L.dptr(arr)), "fvm_upload")
 
     def download(self, out: np.ndarray | None = None) -> np.ndarray:
@@ -221,6 +228,12 @@ class Simulation:
         L.check(self._lib.fvm_synchronize(self._h), "fvm_synchronize")
 
     def download_into(self, U: dict):
+        arrays = [U[k] for k in self.variables]
+        if (all(type(a) is np.ndarray and a.dtype == np.float64 and a.shape == self._ghosted[1:]
+                and a.flags.c_contiguous and a.flags.writeable for a in arrays)
+                and len({a.ctypes.data for a in arrays}) == self.nv):
+            L.check(self._lib.fvm_download_vars(self._h, self._pointers(arrays)), "fvm_download")
+            return
         arr = self.download()
         for q, k in enumerate(self.variables):
             U[k][...] = arr[q]

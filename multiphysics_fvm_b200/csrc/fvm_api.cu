@@ -10,6 +10,8 @@
 #include <mutex>
 #include <string>
 #include <algorithm>
+#include <atomic>
+#include <thread>
 #include <vector>
 
 #include "../../include/fvm.h"
@@ -91,6 +93,14 @@ void host_lengths(const HostMetric& m, int coords, int i, int j, int k, double L
 
 }  // namespace
 
+// Host transfers: bytes of a pinned buffer (256 KB and 512 KB ran slower from 37
+// MB on), bytes per copying thread, threads of one transfer at most.  The DMA
+// from freshly written pinned memory runs at 20 GB/s, little above one thread's
+// copy, so an upload takes a thread per 8 MB (at 8 MB four threads took 0.74 ms,
+// none 0.57); a download takes one per 2 MB (0.33 ms against 0.59).
+constexpr size_t XF_CHUNK = 1 << 20, XF_PER_UP = 8 << 20, XF_PER_DOWN = 2 << 20;
+constexpr int XF_THREADS = 8;
+
 struct fvm_handle {
   fvm_desc d{};
   int nv = 0;
@@ -110,8 +120,13 @@ struct fvm_handle {
   double* partials = nullptr;
   double* totals_dev = nullptr;
   double* stage_dev = nullptr;   // reference-layout float64 staging on the device
-  double* stage_host = nullptr;  // pinned staging
   size_t stage_elems = 0;
+  // host transfers (host_copy): a ring of pinned buffers, two per thread, and
+  // their events
+  int xf_threads = 1;
+  size_t xf_chunk = 0;
+  unsigned char* xf_pinned = nullptr;
+  std::vector<cudaEvent_t> xf_ev;
   // pipelined host transfers (fvm_upload_async / fvm_download_async): a second
   // device staging buffer for downloads, one stream per copy direction and the
   // events that order them against the handle's stream
@@ -667,19 +682,23 @@ int fvm_create(const fvm_desc* desc, fvm_handle** out) {
   }
   // constant parts of the CFL step (navier_stokes.py:575, heat.py:331-338, maxwell.py:586-598)
   double mx = 0.0, rmax = 0.0;
-  for (int k = 0; k < d.nx3; ++k)
-    for (int j = 0; j < d.nx2; ++j)
-      for (int i = 0; i < d.nx1; ++i) {
-        double Ls[3];
-        host_lengths(hm, d.coords, i, j, k, Ls);
-        const double s = (1.0 / (Ls[0] * Ls[0]) + 1.0 / (Ls[1] * Ls[1])) + 1.0 / (Ls[2] * Ls[2]);
-        mx = std::max(mx, s);
-        if (d.physics == FVM_MAXWELL) {
-          const double c = 1 / std::sqrt(d.params[0] * d.params[1]);
-          const double ml = std::max(std::fabs(-c), std::fabs(c));
-          rmax = std::max(rmax, std::max(std::max(ml / Ls[0], ml / Ls[1]), ml / Ls[2]));
-        }
+  // (rounded products, quotients and sums are monotone: the largest of each
+  // column is at the plane of the smallest dx3)
+  const int k = (int)(std::min_element(hm.dx3.begin(), hm.dx3.end(),
+                                       [](double a, double b) { return std::fabs(a) < std::fabs(b); }) -
+                      hm.dx3.begin());
+  for (int j = 0; j < d.nx2; ++j)
+    for (int i = 0; i < d.nx1; ++i) {
+      double Ls[3];
+      host_lengths(hm, d.coords, i, j, k, Ls);
+      const double s = (1.0 / (Ls[0] * Ls[0]) + 1.0 / (Ls[1] * Ls[1])) + 1.0 / (Ls[2] * Ls[2]);
+      mx = std::max(mx, s);
+      if (d.physics == FVM_MAXWELL) {
+        const double c = 1 / std::sqrt(d.params[0] * d.params[1]);
+        const double ml = std::max(std::fabs(-c), std::fabs(c));
+        rmax = std::max(rmax, std::max(std::max(ml / Ls[0], ml / Ls[1]), ml / Ls[2]));
       }
+    }
   h->max_inv_l2 = mx;
   if (d.physics == FVM_HEAT) {
     const double nu = d.params[2] / (d.params[0] * d.params[1]);
@@ -701,7 +720,13 @@ int fvm_create(const fvm_desc* desc, fvm_handle** out) {
   FVM_CKC(cudaMalloc(&h->totals_dev, sizeof(double) * 8));
   h->stage_elems = (size_t)h->nv * (d.nx1 + 2) * (d.nx2 + 2) * (d.nx3 + 2);
   FVM_CKC(cudaMalloc(&h->stage_dev, h->stage_elems * sizeof(double)));
-  FVM_CKC(cudaMallocHost(&h->stage_host, h->stage_elems * sizeof(double)));
+  const size_t host_bytes = h->stage_elems * sizeof(double);
+  h->xf_chunk = std::min(XF_CHUNK, (host_bytes / 2 + 255) / 256 * 256 + 256);
+  h->xf_threads = (int)std::max<size_t>(
+      1, std::min({host_bytes / XF_PER_DOWN, (size_t)XF_THREADS, (size_t)std::thread::hardware_concurrency() / 2}));
+  FVM_CKC(cudaMallocHost(&h->xf_pinned, 2 * h->xf_threads * h->xf_chunk));
+  h->xf_ev.assign(2 * h->xf_threads, nullptr);
+  for (cudaEvent_t& e : h->xf_ev) FVM_CKC(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   h->device_bytes += h->stage_elems * sizeof(double);
 #undef FVM_CKC
   h->tile_ty = d.tile_ty > 0 && !former_tile_ty(d) ? d.tile_ty : default_tile_ty(d);
@@ -733,7 +758,9 @@ int fvm_destroy(fvm_handle* h) {
   if (h->partials) cudaFree(h->partials);
   if (h->totals_dev) cudaFree(h->totals_dev);
   if (h->stage_dev) cudaFree(h->stage_dev);
-  if (h->stage_host) cudaFreeHost(h->stage_host);
+  if (h->xf_pinned) cudaFreeHost(h->xf_pinned);
+  for (cudaEvent_t e : h->xf_ev)
+    if (e) cudaEventDestroy(e);
   if (h->s_in) cudaStreamSynchronize(h->s_in);
   if (h->s_out) cudaStreamSynchronize(h->s_out);
   if (h->stage_out) cudaFree(h->stage_out);
@@ -781,55 +808,177 @@ static int transpose(fvm_handle* h, bool to_device, int buf, bool interior, doub
   return FVM_OK;
 }
 
-int fvm_upload(fvm_handle* h, const double* host_state) {
-  if (!h || !host_state) return fail(FVM_E_INVALID, "null argument");
-  const size_t bytes = h->stage_elems * sizeof(double);
-  FVM_CK(cudaMemcpyAsync(h->stage_dev, host_state, bytes, cudaMemcpyHostToDevice, h->stream));
-  int rc = transpose(h, true, 0, false);
+}  // extern "C"
+
+namespace {
+
+// Copy between the device staging array and `n` host arrays of `per` bytes each
+// (pageable memory), on the handle's stream, finished on return.  The driver's
+// own pageable copy stages through pinned memory with one thread: 5 GB/s at 2.6
+// MB, 17 at 37 MB, 13 at 170 MB of the link's 55.  Here the bytes go through the
+// handle's ring of pinned buffers: this thread issues the DMA copies in order,
+// up to XF_THREADS others (for this call only; they make no CUDA calls, whose
+// first use in a new thread costs more than a chunk) copy between the ring and
+// the host arrays.  170 MB up 13.4 -> 5.1 ms, down 13.5 -> 4.8; 37 MB up 2.3 ->
+// 2.0, down 2.3 -> 1.2; a host dict of 2 MB up 0.28 -> 0.19, down 0.59 -> 0.21
+// (stacking and slicing copies included).
+int host_copy(fvm_handle* h, bool to_device, double* const* host, int n, size_t per) {
+  const size_t total = per * n, chunk = h->xf_chunk;
+  const long long nchunk = (long long)((total + chunk - 1) / chunk);
+  const int want = (int)std::min<size_t>(h->xf_threads, total / (to_device ? XF_PER_UP : XF_PER_DOWN)), ring = 2 * h->xf_threads;
+  auto buf = [&](long long c) { return h->xf_pinned + (size_t)(c % ring) * chunk; };
+  auto len = [&](long long c) { return std::min(chunk, total - (size_t)c * chunk); };
+  auto move = [&](long long c) {  // chunk c, host arrays <-> pinned buffer
+    unsigned char* pinned = buf(c);
+    size_t off = (size_t)c * chunk, left = len(c);
+    while (left) {
+      const size_t q = off / per, at = off - q * per, m = std::min(left, per - at);
+      unsigned char* p = reinterpret_cast<unsigned char*>(host[q]) + at;
+      std::memcpy(to_device ? pinned : p, to_device ? p : pinned, m);
+      off += m;
+      pinned += m;
+      left -= m;
+    }
+  };
+  auto dma = [&](long long c) -> cudaError_t {
+    unsigned char* dev = reinterpret_cast<unsigned char*>(h->stage_dev) + (size_t)c * chunk;
+    const cudaError_t e = to_device ? cudaMemcpyAsync(dev, buf(c), len(c), cudaMemcpyHostToDevice, h->stream)
+                                    : cudaMemcpyAsync(buf(c), dev, len(c), cudaMemcpyDeviceToHost, h->stream);
+    return e != cudaSuccess ? e : cudaEventRecord(h->xf_ev[c % ring], h->stream);
+  };
+  auto landed = [&](long long c) { return cudaEventSynchronize(h->xf_ev[c % ring]); };
+  // chunk counters: taken by a copying thread; open to it (upload: its buffer is
+  // free, download: its bytes have landed); moved
+  std::atomic<long long> taken{0}, open{to_device ? ring : 0};
+  std::atomic<bool> stop{false};
+  std::vector<std::atomic<unsigned char>> moved;
+  std::vector<std::thread> pool;
+  auto worker = [&] {
+    for (long long c; (c = taken.fetch_add(1)) < nchunk;) {
+      while (c >= open.load(std::memory_order_acquire)) {
+        if (stop.load(std::memory_order_relaxed)) return;
+        std::this_thread::yield();
+      }
+      move(c);
+      moved[c].store(1, std::memory_order_release);
+    }
+  };
+  if (want >= 2) {
+    try {
+      moved = std::vector<std::atomic<unsigned char>>(nchunk);
+      pool.reserve(want);
+      for (int i = 0; i < want; ++i) pool.emplace_back(worker);
+    } catch (...) {  // fewer threads, or none: this one copies
+    }
+  }
+  const bool helped = !pool.empty();
+  auto wait_moved = [&](long long c) {
+    while (!moved[c].load(std::memory_order_acquire)) std::this_thread::yield();
+  };
+  cudaError_t e = cudaSuccess;
+  if (to_device) {
+    for (long long c = 0; c < nchunk && e == cudaSuccess; ++c) {
+      if (helped) {
+        wait_moved(c);
+      } else {
+        if (c >= ring) e = landed(c);  // the buffer's previous copy
+        if (e != cudaSuccess) break;
+        move(c);
+      }
+      e = dma(c);
+      const long long k = c + 1 - ring / 2;  // keep half the ring in flight, open the rest
+      if (helped && k >= 0 && e == cudaSuccess && (e = landed(k)) == cudaSuccess)
+        open.store(k + 1 + ring, std::memory_order_release);
+    }
+  } else {
+    const long long ahead = std::min<long long>(ring / 2, nchunk);
+    for (long long c = 0; c < nchunk + ahead && e == cudaSuccess; ++c) {
+      if (c < nchunk) {
+        if (helped && c >= ring) wait_moved(c - ring);  // its buffer has been read
+        e = dma(c);
+      }
+      if (c >= ahead && e == cudaSuccess && (e = landed(c - ahead)) == cudaSuccess) {
+        if (helped) open.store(c - ahead + 1, std::memory_order_release);
+        else move(c - ahead);
+      }
+    }
+  }
+  if (e != cudaSuccess) stop = true;
+  for (std::thread& w : pool) w.join();
+  FVM_CK(e);
+  FVM_CK(cudaStreamSynchronize(h->stream));
+  return FVM_OK;
+}
+
+// A caller's page-locked array is copied from or into directly.
+bool page_locked(const void* p) {
+  cudaPointerAttributes a;
+  const bool ok = cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type == cudaMemoryTypeHost;
+  cudaGetLastError();
+  return ok;
+}
+
+// Ghosted state in the device staging array: faces from the boundary
+// conditions, edges and corners averaged (src/solver.py:39-61).
+int stage_ghosted(fvm_handle* h, double* stage) {
+  FVM_CK(launch_bc(h, 0));
+  if (int rc = transpose(h, false, 0, false, stage)) return rc;
+  const fvm_desc& d = h->d;
+  const int longest = std::max(d.nx1, std::max(d.nx2, d.nx3));
+  edges_kernel<<<dim3((longest + 255) / 256, 12 * h->nv), 256, 0, h->stream>>>(stage, d.nx1, d.nx2, d.nx3);
+  FVM_CK(cudaGetLastError());
+  corners_kernel<<<1, 64, 0, h->stream>>>(stage, d.nx1, d.nx2, d.nx3, h->nv);
+  FVM_CK(cudaGetLastError());
+  return FVM_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int fvm_upload_vars(fvm_handle* h, const double* const* host_vars) {
+  if (!h || !host_vars) return fail(FVM_E_INVALID, "null argument");
+  double* p[6] = {};
+  for (int q = 0; q < h->nv; ++q)
+    if (!(p[q] = const_cast<double*>(host_vars[q]))) return fail(FVM_E_INVALID, "null variable");
+  int rc = host_copy(h, true, p, h->nv, h->stage_elems / h->nv * sizeof(double));
+  if (!rc) rc = transpose(h, true, 0, false);
   if (rc) return rc;
   FVM_CK(cudaStreamSynchronize(h->stream));
   return FVM_OK;
 }
 
-static void fill_edges_corners(double* f, int n1, int n2, int n3) {
-  // ghost edges/corners as averages of adjacent ghost faces (src/solver.py:39-61)
-  const int N[3] = {n1 + 2, n2 + 2, n3 + 2};
-  auto at = [&](int i, int j, int k) -> double& { return f[((long long)i * N[1] + j) * N[2] + k]; };
-  for (int a = 0; a < 3; ++a)
-    for (int b = a + 1; b < 3; ++b) {
-      const int c = 3 - a - b;
-      for (int ea = 0; ea < 2; ++ea)
-        for (int eb = 0; eb < 2; ++eb)
-          for (int t = 1; t <= N[c] - 2; ++t) {
-            int idx[3], p[3], q[3];
-            idx[a] = ea ? N[a] - 1 : 0;
-            idx[b] = eb ? N[b] - 1 : 0;
-            idx[c] = t;
-            for (int z = 0; z < 3; ++z) { p[z] = idx[z]; q[z] = idx[z]; }
-            p[a] = ea ? N[a] - 2 : 1;
-            q[b] = eb ? N[b] - 2 : 1;
-            at(idx[0], idx[1], idx[2]) = 0.5 * (at(p[0], p[1], p[2]) + at(q[0], q[1], q[2]));
-          }
-    }
-  for (int ci = 0; ci < 2; ++ci)
-    for (int cj = 0; cj < 2; ++cj)
-      for (int ck = 0; ck < 2; ++ck) {
-        const int i = ci ? N[0] - 1 : 0, j = cj ? N[1] - 1 : 0, k = ck ? N[2] - 1 : 0;
-        const int ii = ci ? N[0] - 2 : 1, jj = cj ? N[1] - 2 : 1, kk = ck ? N[2] - 2 : 1;
-        at(i, j, k) = (at(ii, j, k) + at(i, jj, k) + at(i, j, kk)) / 3.0;
-      }
+int fvm_download_vars(fvm_handle* h, double* const* host_vars) {
+  if (!h || !host_vars) return fail(FVM_E_INVALID, "null argument");
+  for (int q = 0; q < h->nv; ++q)
+    if (!host_vars[q]) return fail(FVM_E_INVALID, "null variable");
+  if (int rc = stage_ghosted(h, h->stage_dev)) return rc;
+  return host_copy(h, false, host_vars, h->nv, h->stage_elems / h->nv * sizeof(double));
+}
+
+int fvm_upload(fvm_handle* h, const double* host_state) {
+  if (!h || !host_state) return fail(FVM_E_INVALID, "null argument");
+  const size_t bytes = h->stage_elems * sizeof(double);
+  int rc = FVM_OK;
+  if (page_locked(host_state)) {
+    FVM_CK(cudaMemcpyAsync(h->stage_dev, host_state, bytes, cudaMemcpyHostToDevice, h->stream));
+  } else {
+    double* p = const_cast<double*>(host_state);
+    rc = host_copy(h, true, &p, 1, bytes);
+  }
+  if (!rc) rc = transpose(h, true, 0, false);
+  if (rc) return rc;
+  FVM_CK(cudaStreamSynchronize(h->stream));
+  return FVM_OK;
 }
 
 int fvm_download(fvm_handle* h, double* host_state) {
   if (!h || !host_state) return fail(FVM_E_INVALID, "null argument");
-  FVM_CK(launch_bc(h, 0));
-  int rc = transpose(h, false, 0, false);
-  if (rc) return rc;
-  FVM_CK(cudaMemcpyAsync(host_state, h->stage_dev, h->stage_elems * sizeof(double), cudaMemcpyDeviceToHost,
-                         h->stream));
+  if (int rc = stage_ghosted(h, h->stage_dev)) return rc;
+  const size_t bytes = h->stage_elems * sizeof(double);
+  if (!page_locked(host_state)) return host_copy(h, false, &host_state, 1, bytes);
+  FVM_CK(cudaMemcpyAsync(host_state, h->stage_dev, bytes, cudaMemcpyDeviceToHost, h->stream));
   FVM_CK(cudaStreamSynchronize(h->stream));
-  const size_t per = h->stage_elems / h->nv;
-  for (int q = 0; q < h->nv; ++q) fill_edges_corners(host_state + q * per, h->d.nx1, h->d.nx2, h->d.nx3);
   return FVM_OK;
 }
 
@@ -871,16 +1020,9 @@ int fvm_download_async(fvm_handle* h, double* host_state) {
   if (!h || !host_state) return fail(FVM_E_INVALID, "null argument");
   int rc = ensure_async(h);
   if (rc) return rc;
-  FVM_CK(launch_bc(h, 0));
   // the previous download's copy must have drained the staging buffer
   FVM_CK(cudaStreamWaitEvent(h->stream, h->ev_out_free, 0));
-  if ((rc = transpose(h, false, 0, false, h->stage_out))) return rc;
-  const fvm_desc& d = h->d;
-  const int longest = std::max(d.nx1, std::max(d.nx2, d.nx3));
-  edges_kernel<<<dim3((longest + 255) / 256, 12 * h->nv), 256, 0, h->stream>>>(h->stage_out, d.nx1, d.nx2, d.nx3);
-  FVM_CK(cudaGetLastError());
-  corners_kernel<<<1, 64, 0, h->stream>>>(h->stage_out, d.nx1, d.nx2, d.nx3, h->nv);
-  FVM_CK(cudaGetLastError());
+  if ((rc = stage_ghosted(h, h->stage_out))) return rc;
   FVM_CK(cudaEventRecord(h->ev_out_ready, h->stream));
   FVM_CK(cudaStreamWaitEvent(h->s_out, h->ev_out_ready, 0));
   FVM_CK(cudaMemcpyAsync(host_state, h->stage_out, h->stage_elems * sizeof(double), cudaMemcpyDeviceToHost,
@@ -915,9 +1057,7 @@ int fvm_residual(fvm_handle* h, double* host_rhs) {
   int rc = transpose(h, false, 1, true);
   if (rc) return rc;
   const size_t n = (size_t)h->nv * h->d.nx1 * h->d.nx2 * h->d.nx3;
-  FVM_CK(cudaMemcpyAsync(host_rhs, h->stage_dev, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  FVM_CK(cudaStreamSynchronize(h->stream));
-  return FVM_OK;
+  return host_copy(h, false, &host_rhs, 1, n * sizeof(double));
 }
 
 int fvm_set_time(fvm_handle* h, double t, double t_end, double cfl) {
