@@ -8,21 +8,26 @@
 // the halo warp forms the x1 data outside the warps and the border cells of
 // the P / stress planes.  Halo HH = 3 (the stress at K+2 needs v at K+3).
 //
+// Velocities are formed where the stress needs them, six neighbours a cell.  A
+// ring of v planes, formed once per cell, costs a barrier in the middle of every
+// step (v of the newest plane before the stress): with 16 warps per SM a quarter
+// of the issue slots were lost to barriers.  256^3 stage 1291 -> 1118 us without
+// it (one block of 15 rows instead of two of 7 ran 1183).
+//
 // Per step K (ghosted output plane K; ring planes K..K+2 resident, K+3
 // arriving):
 //   1. thread 0 issues plane K+3 into the slot of plane K-1 and the staged
 //      U0 / accumulator tile of plane K;
 //   2. x2/x1 sweep of plane K in registers (U, P and the stress row of each
 //      face axis); the halo warp forms the x1 halo data of plane K+1;
-//   3. wait for plane K+3; v = m / rho of plane K+3 over the tile + 3;
-//      block barrier;
+//   3. every thread waits (bounded) for plane K+3;
 //   4. P and the stress of plane K+2 over the tile + 2 (own cells by their
 //      owners, kept in registers for x3; border cells by the halo warp);
 //   5. x3 slope of plane K+1 and the flux at K+1/2 (left state and the flux
 //      at K-1/2 carried in registers);
 //   6. divergence, gravity, stage combination, stores; block barrier.
-// The first step of a tile (K = Z0 - 3) only fills v, P and the stress of
-// planes Z0-2 and Z0-1.
+// The first step of a tile (K = Z0 - 3) only fills P and the stress of planes
+// Z0-2 and Z0-1.
 #pragma once
 #include "stage_ns_strip.cuh"
 
@@ -34,18 +39,16 @@ struct NsStripViscCfg {
   static constexpr int NO = 32 * NW;
   static constexpr int NT = NO + 32;
   static constexpr int NV = 5, NF = 9, HH = 3;
-  static constexpr int W = 40;  // U / v ring column c <-> tile x offset c - 4
+  static constexpr int W = 40;  // U ring column c <-> tile x offset c - 4
   static constexpr int ROWS = TY + 2 * HH;
   static constexpr int PL = ROWS * W;
   static constexpr int NSLOT = 4;  // planes K, K+1, K+2 resident, K+3 arriving
   static constexpr int SLOT = round_up(NV * PL, 32);
   static constexpr int W2 = TX + 4, R2 = TY + 4, PL2 = W2 * R2;  // P / stress planes: tile + 2
   static constexpr int NBORDER = 4 * W2 + 4 * TY;
-  static constexpr int VW = TX + 6, VR = TY + 6, NVC = VW * VR;  // v region: tile + 3
   static constexpr int STG = NV * TY * TX;
   static constexpr int OFF_U = 0;
-  static constexpr int OFF_V = OFF_U + NSLOT * SLOT;  // [slot][component][PL]
-  static constexpr int OFF_P = OFF_V + 3 * 3 * PL;
+  static constexpr int OFF_P = OFF_U + NSLOT * SLOT;
   static constexpr int OFF_T = OFF_P + 3 * PL2;       // [slot][component][PL2]
   static constexpr int OFF_HL = OFF_T + 3 * 6 * PL2;
   static constexpr int OFF_FR = OFF_HL + 2 * NF * TY;
@@ -93,12 +96,11 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
     ns_strip_visc_kernel(const __grid_constant__ NsStripSource src) {
   using C = NsStripViscCfg<R, NW>;
   constexpr int TX = C::TX, TY = C::TY, W = C::W, PL = C::PL, HH = C::HH, NF = C::NF, W2 = C::W2;
-  constexpr int PL2 = C::PL2, NT = C::NT;
+  constexpr int PL2 = C::PL2;
   constexpr float HS = strip_half<LIM>();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   float* sm = reinterpret_cast<float*>(smem_raw);
   float* uring = sm + C::OFF_U;
-  float* vring = sm + C::OFF_V;
   float* pring = sm + C::OFF_P;
   float* tring = sm + C::OFF_T;
   float* hl = sm + C::OFF_HL;
@@ -161,17 +163,11 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
     if (tid == 0)
       for (int pl = Kfirst; pl <= Kfirst + 3; ++pl) issue(pl);
 
-    // v = m / rho of one ring plane over the tile + 3 (all threads)
-    auto velocity = [&](int pl) {
-      const float* ub = uring + pmod(pl, C::NSLOT) * C::SLOT;
-      float* vb = vring + pmod(pl, 3) * 3 * PL;
-      for (int it = tid; it < C::NVC; it += NT) {
-        const int o = (it / C::VW) * W + 1 + it % C::VW;  // rows -3..TY+2, columns -3..TX+2
-        const float ir = rcp_approx(ub[o]);
-        vb[o] = ub[PL + o] * ir;
-        vb[PL + o] = ub[2 * PL + o] * ir;
-        vb[2 * PL + o] = ub[3 * PL + o] * ir;
-      }
+    // v = m / rho of ring cell u
+    auto velocity = [&](const float* u, float* v) {
+      const float ir = rcp_approx(u[0]);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) v[c] = u[(1 + c) * PL] * ir;
     };
     // P and the six stress components of plane pl at tile offset (x, y),
     // written to the rings; returns {P, t13, t23, t33} for the x3 phase
@@ -183,23 +179,25 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
       const int ii = x0 + x, jj = y0 + y, kk = pl - 1;
       float t[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       if (!(kk < 0 || kk >= nz || ii < 0 || ii >= nx || jj < 0 || jj >= ny)) {
-        const float* vm = vring + pmod(pl - 1, 3) * 3 * PL;
-        const float* v0 = vring + pmod(pl, 3) * 3 * PL;
-        const float* vp = vring + pmod(pl + 1, 3) * 3 * PL;
         const float h1 = 0.5f * __ldg(m.inv_dx1 + ii), h2 = 0.5f * inv_len<float, COORD, 1>(m, ii, jj, kk);
         const float h3 = 0.5f * inv_len<float, COORD, 2>(m, ii, jj, kk);
         float g[3][3];  // g[c][a] = d v_c / d x_a
+        auto gradient = [&](const float* up, const float* um, float h, int a) {
+          float vp[3], vm[3];
+          velocity(up, vp);
+          velocity(um, vm);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const int oc = c * PL + o;
-          g[c][0] = (v0[oc + 1] - v0[oc - 1]) * h1;
-          g[c][1] = (v0[oc + W] - v0[oc - W]) * h2;
-          g[c][2] = (vp[oc] - vm[oc]) * h3;
-        }
+          for (int c = 0; c < 3; ++c) g[c][a] = (vp[c] - vm[c]) * h;
+        };
+        gradient(ub + o + 1, ub + o - 1, h1, 0);
+        gradient(ub + o + W, ub + o - W, h2, 1);
+        gradient(uring + pmod(pl + 1, C::NSLOT) * C::SLOT + o, uring + pmod(pl - 1, C::NSLOT) * C::SLOT + o, h3, 2);
         const float tt = 2.f / 3.f;
         if constexpr (COORD != COORD_CART) {
           // the metric terms of the diagonal gradients and of the off-diagonal sums
-          const float ir = __ldg(m.inv_r + ii), v1 = v0[o], v2 = v0[PL + o], v3 = v0[2 * PL + o];
+          float v[3];
+          velocity(ub + o, v);
+          const float ir = __ldg(m.inv_r + ii), v1 = v[0], v2 = v[1], v3 = v[2];
           g[1][1] = fmaf(v1, ir, g[1][1]);
           g[0][1] = fmaf(-v2, ir, g[0][1]);
           if constexpr (COORD == COORD_SPH) {
@@ -414,10 +412,11 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
         }
       }
       // ------------------------------------------------------------ 3 ----
-      // each thread waits for the plane itself; the barrier after v of the
-      // new plane also takes the block out if any wait ran out
+      // Every thread waits for the plane itself; what it reads after the wait was
+      // not written by another thread in this step.  A thread whose wait ran out
+      // skips the rest of the step and the barrier at its end takes the block out.
+      bool got = true;
       {
-        bool got = true;
         for (int pl = (K == Kfirst ? Kfirst : K + 3); pl <= K + 3; ++pl) {
           const int s = pmod(pl, C::NSLOT);
           const bool g = got && mbar_wait_bounded(&bars[s], (phase_bits >> s) & 1u, p.wait_ns);
@@ -427,31 +426,16 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
           }
           got = g;
         }
-        if (K != Kfirst && got) velocity(K + 3);
-        if (!__syncthreads_and(got)) {
-          if (tid == 0) atomicOr(p.status, ST_TMA_TIMEOUT);
-          ok = false;
-          break;
-        }
+        if (!got) atomicOr(p.status, ST_TMA_TIMEOUT);
       }
       float own[R][4];  // P, t13, t23, t33 of plane K+2 at the own cells
-      if (K == Kfirst) {
-        // v of planes K..K+2, then P / stress of plane K+1; v of plane K+3
-        // (into plane K's slot), then P / stress of plane K+2
-        velocity(K);
-        velocity(K + 1);
-        velocity(K + 2);
-        __syncthreads();
-        float skip[R][4];
-        closure_plane(K + 1, skip);
-        __syncthreads();
-        velocity(K + 3);
-        __syncthreads();
-      }
       // ------------------------------------------------------------ 4 ----
-      closure_plane(K + 2, own);
-      bool step_ok = true;
-      if (is_out) {
+      if (got) {
+        if (K == Kfirst) closure_plane(K + 1, own);
+        closure_plane(K + 2, own);
+      }
+      bool step_ok = got;
+      if (is_out && got) {
         // ------------------------------------------------------------ 5 ----
         const float hz = K + 1 <= 0 || K + 1 >= nz + 1 ? 0.f : HS;
         const bool zslope = K >= Z0 - 2, zface = K >= Z0 - 1;
