@@ -152,11 +152,11 @@ cudaError_t launch_ns(int lim, int riem, int coord, bool visc, const CUtensorMap
 // 128 registers) or 16 (8 output warps, 2 blocks/SM).
 constexpr int NS_STRIP_TY = 8, NS_STRIP_TY_ALT = 16;
 
-template <int LIM, int RIEM, int COORD, int TY>
+template <int LIM, int RIEM, int COORD, int TY, bool FLAT>
 cudaError_t launch_ns_strip_ty(const NsStripSource& src, int nbuf, cudaStream_t s, int nsm) {
   constexpr int R = 2, NW = TY / R;
   using C = NsStripCfg<R, NW>;
-  auto kern = ns_strip_kernel<LIM, RIEM, R, NW, TY == 8 ? 3 : 2, COORD>;
+  auto kern = ns_strip_kernel<LIM, RIEM, R, NW, TY == 8 ? 3 : 2, COORD, FLAT>;
   static int bps[3] = {0, 0, 0};
   if (bps[0] == 0 || nsm < 0) {
     // occupancy with 0, 1 and 2 staged tiles; the attribute ends at the largest
@@ -177,8 +177,14 @@ template <int LIM, int RIEM, int COORD>
 cudaError_t launch_ns_strip_lr(NsStripSource& src, int ty, int nbuf, cudaStream_t s, int nsm) {
   NsParams<float>& p = src.p;
   set_tiles(p, ty, p.flat != 0);
-  if (ty == NS_STRIP_TY_ALT) return launch_ns_strip_ty<LIM, RIEM, COORD, NS_STRIP_TY_ALT>(src, nbuf, s, nsm);
-  return launch_ns_strip_ty<LIM, RIEM, COORD, NS_STRIP_TY>(src, nbuf, s, nsm);
+  const bool alt = ty == NS_STRIP_TY_ALT;
+  if (p.flat || nsm < 0) {  // (a handle prepares both marches: residuals run the x3 one)
+    const cudaError_t e = alt ? launch_ns_strip_ty<LIM, RIEM, COORD, NS_STRIP_TY_ALT, true>(src, nbuf, s, nsm)
+                              : launch_ns_strip_ty<LIM, RIEM, COORD, NS_STRIP_TY, true>(src, nbuf, s, nsm);
+    if (nsm >= 0 || e != cudaSuccess) return e;
+  }
+  return alt ? launch_ns_strip_ty<LIM, RIEM, COORD, NS_STRIP_TY_ALT, false>(src, nbuf, s, nsm)
+             : launch_ns_strip_ty<LIM, RIEM, COORD, NS_STRIP_TY, false>(src, nbuf, s, nsm);
 }
 
 template <int COORD>

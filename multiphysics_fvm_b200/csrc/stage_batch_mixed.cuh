@@ -89,8 +89,12 @@ __global__ void __launch_bounds__(MIX_NT, 3) batch_mixed_kernel(const __grid_con
     const MixedInst& in = src.inst[inst];
     if (in.kind == 0) {
       if (in.ns.active && !*in.ns.active) continue;  // this grid's clock passed t_end
-      ok = ns_strip_tile<LIM, RIEM, MIX_NS_R, MIX_NS_NW>(in.ns, &in.tmap, &in.u0map, &in.accmap, pc, smem_raw, bars,
-                                                         bars + 6, 6, phase_bits, pending);
+      if (in.ns.flat)
+        ok = ns_strip_tile<LIM, RIEM, MIX_NS_R, MIX_NS_NW, COORD_CART, true>(
+            in.ns, &in.tmap, &in.u0map, &in.accmap, pc, smem_raw, bars, bars + 6, 6, phase_bits, pending);
+      else
+        ok = ns_strip_tile<LIM, RIEM, MIX_NS_R, MIX_NS_NW, COORD_CART, false>(
+            in.ns, &in.tmap, &in.u0map, &in.accmap, pc, smem_raw, bars, bars + 6, 6, phase_bits, pending);
     } else {
       if (in.heat.active && !*in.heat.active) continue;
       ok = heat_pc_tile<HCOORD, HVX, MIX_HEAT_NW>(in.heat, &in.tmap, pc, smem_raw, bars, phase_bits, pending);

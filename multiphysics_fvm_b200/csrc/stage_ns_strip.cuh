@@ -192,7 +192,7 @@ __device__ __forceinline__ void curvilinear_source(const ColMetric<COORD>& cm, c
 // barriers (indices 0..2, phase bits 0..2), `gbar` the staged-tile barrier with
 // phase bit `gbit`; `phase_bits` and `pending` carry over from tile to tile.
 // Returns false when a wait ran out: the block must stop and drain.
-template <int LIM, int RIEM, int R, int NW, int COORD = COORD_CART>
+template <int LIM, int RIEM, int R, int NW, int COORD, bool flat>
 __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CUtensorMap* tmap,
                                               const CUtensorMap* u0map, const CUtensorMap* accmap, const Piece& pc,
                                               unsigned char* smem_raw, uint64_t* bars, uint64_t* gbar, int gbit,
@@ -224,8 +224,10 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
     // A one-plane grid whose x3 ghosts copy the plane ("flat") has x3 fluxes
     // that cancel exactly: plane 1 alone, no x3 pipeline.  Its piece marches
     // instead over row tiles along x2 (the steps of the march), each step's
-    // plane copy issued one step ahead into the next ring slot.
-    const bool flat = p.flat != 0;
+    // plane copy issued one step ahead into the next ring slot.  A
+    // template argument: with both marches in one body the hot loop spread over
+    // code it jumped across, and warps waited for instructions (256^3 stage
+    // 599 -> 575 us, a mixed batch's stage 340 -> 301, when they were parted).
     const int Z0 = flat ? 1 : 1 + pc.u0;  // first ghosted output plane
     const int Zl = flat ? 1 : pc.u1;      // last ghosted output plane
     const int x0 = (pc.col % p.ntx) * TX, ybase = flat ? pc.u0 * TY : (pc.col / p.ntx) * TY;
@@ -362,7 +364,7 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
       for (int r = 0; r < R; ++r)
 #pragma unroll
         for (int v = 0; v < 5; ++v) kv[r][v] = 0.f;
-      if (flat) {
+      if constexpr (flat) {
         // the plane itself, its P over the tile + 2 and the halo warp's x1
         // data, before the sweep
         const bool g = mbar_wait_bounded(&bars[sK], (phase_bits >> sK) & 1u, p.wait_ns);
@@ -464,7 +466,7 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
         // --------------------------------------------------- halo warp ----
         // x1 data of plane K+1, the next output plane (a flat grid's was
         // formed before the sweep)
-        if (!flat) halo_x1(K + 1, uK1, pK1);
+        if constexpr (!flat) halo_x1(K + 1, uK1, pK1);
       }
       // ------------------------------------------------------------ 3 ----
       // Every thread waits for the plane itself; nothing read after the wait
@@ -472,7 +474,8 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
       // barrier here.  A thread whose wait ran out skips the rest of the step
       // and the barrier at its end takes the block out.
       bool got = true;
-      for (int pl = (K == Kfirst ? Kfirst : K + 2); !flat && pl <= K + 2; ++pl) {
+      if constexpr (!flat)
+      for (int pl = (K == Kfirst ? Kfirst : K + 2); pl <= K + 2; ++pl) {
         const int s = pmod(pl, C::NSLOT);
         const bool g = got && mbar_wait_bounded(&bars[s], (phase_bits >> s) & 1u, p.wait_ns);
         if (g) {
@@ -486,7 +489,7 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
       if (!got) {
         // skip to the barrier
       } else if (is_out) {
-        if (!flat) {  // x3 (a flat grid has none)
+        if constexpr (!flat) {  // x3 (a flat grid has none)
           // ------------------------------------------------------------ 4 ----
           float pnew[R];
 #pragma unroll
@@ -579,7 +582,7 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
       } else {
         // P of plane K+2 (and on the first step of K, K+1) on the cells of
         // the P plane no output thread owns
-        if (!flat) {
+        if constexpr (!flat) {
           border_p(pK2, uK2);
           if (K == Kfirst) {
             border_p(pK, uK);
@@ -594,7 +597,7 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
   return true;
 }
 
-template <int LIM, int RIEM, int R, int NW, int MINB, int COORD>
+template <int LIM, int RIEM, int R, int NW, int MINB, int COORD, bool FLAT>
 __global__ void __launch_bounds__(NsStripCfg<R, NW>::NT, MINB)
     ns_strip_kernel(const __grid_constant__ NsStripSource src) {
   using C = NsStripCfg<R, NW>;
@@ -623,8 +626,8 @@ __global__ void __launch_bounds__(NsStripCfg<R, NW>::NT, MINB)
   int inst;
   bool ok = true;
   while (ok && walk.next(grid, inst, pc))
-    ok = ns_strip_tile<LIM, RIEM, R, NW, COORD>(p, &src.tmap, &src.u0map, &src.accmap, pc, smem_raw, bars,
-                                                bars + C::NSLOT, C::NSLOT, phase_bits, pending);
+    ok = ns_strip_tile<LIM, RIEM, R, NW, COORD, FLAT>(p, &src.tmap, &src.u0map, &src.accmap, pc, smem_raw, bars,
+                                                      bars + C::NSLOT, C::NSLOT, phase_bits, pending);
   // On a timeout, wait (bounded) for every copy this block may still have in flight.
   if (!ok && tid == 0) {
     for (int s = 0; s < C::NBAR; ++s)
