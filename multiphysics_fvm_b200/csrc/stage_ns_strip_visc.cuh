@@ -45,7 +45,9 @@ struct NsStripViscCfg {
   static constexpr int NSLOT = 4;  // planes K, K+1, K+2 resident, K+3 arriving
   static constexpr int SLOT = round_up(NV * PL, 32);
   static constexpr int W2 = TX + 4, R2 = TY + 4, PL2 = W2 * R2;  // P / stress planes: tile + 2
-  static constexpr int NBORDER = 4 * W2 + 4 * TY;
+  static constexpr int NBORDER = 4 * W2 + 4 * TY;                // halo cells of a P / stress plane ...
+  static constexpr int NPASS = (NBORDER + 31) / 32;              // ... in warp-wide passes,
+  static constexpr int HALO_PASSES = 2;                          // of which the halo warp takes these
   static constexpr int STG = NV * TY * TX;
   static constexpr int OFF_U = 0;
   static constexpr int OFF_P = OFF_U + NSLOT * SLOT;
@@ -60,6 +62,7 @@ struct NsStripViscCfg {
   static constexpr unsigned STG_BYTES = STG * 4;
   static constexpr int bytes(int nbuf) { return STG_OFF_BYTES + nbuf * (int)STG_BYTES; }
   static_assert(2 * TY <= 32, "one halo lane per tile row and task");
+  static_assert(R == 1 && NPASS - HALO_PASSES <= NW, "an own row and at most one border pass per output warp");
   static_assert((SLOT * 4) % 128 == 0 && (STG_BYTES % 128) == 0, "TMA destinations need 128-byte alignment");
 };
 
@@ -223,16 +226,25 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
       out4[2] = t[5];
       out4[3] = t[2];
     };
-    // P and stress of plane pl over the tile + 2: own cells by the output
-    // threads (results kept in `own`), border cells by the halo warp
-    auto closure_plane = [&](int pl, float (*own)[4]) {
-      if (is_out) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) closure_at(pl, lane, w * R + r, own[r]);
-      } else {
-        for (int b = lane; b < C::NBORDER; b += 32) {
+    // P and stress of planes pa..pb over the tile + 2: own cells by the output
+    // threads (the last plane's results kept in `own`), border cells 32 at a
+    // time by the halo warp (the first HALO_PASSES) and output warps 0, 1, ...
+    // (one pass each): with all six passes the halo warp was the last to reach
+    // the step's barrier (cylindrical 96x128x64 stage 76.9 -> 72.3 us, 256^3 1118 ->
+    // 1108).  One loop, so one copy of the closure.
+    auto closure_planes = [&](int pa, int pb, float* own) {
+      for (int pl = pa; pl <= pb; ++pl) {
+        const int first = is_out ? C::HALO_PASSES - 1 + w : 0;
+        const int last = !is_out ? C::HALO_PASSES : (first + 1 < C::NPASS ? first + 2 : first + 1);
+#pragma unroll 1
+        for (int q = first; q < last; ++q) {
+          const bool mine = is_out && q == first;
+          const int b = q * 32 + lane;
           int x, y;
-          if (b < 2 * W2) {
+          if (mine) {
+            x = lane;
+            y = w;
+          } else if (b < 2 * W2) {
             y = b / W2 - 2;
             x = b % W2 - 2;
           } else if (b < 4 * W2) {
@@ -243,8 +255,14 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
             y = c >> 2;
             x = (c & 3) < 2 ? (c & 3) - 2 : (c & 3) + 30;
           }
-          float dummy[4];
-          closure_at(pl, x, y, dummy);
+          if (mine || b < C::NBORDER) {
+            float o4[4];
+            closure_at(pl, x, y, o4);
+            if (mine) {
+#pragma unroll
+              for (int c = 0; c < 4; ++c) own[c] = o4[c];
+            }
+          }
         }
       }
     };
@@ -428,12 +446,9 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
         }
         if (!got) atomicOr(p.status, ST_TMA_TIMEOUT);
       }
-      float own[R][4];  // P, t13, t23, t33 of plane K+2 at the own cells
+      float own[4] = {0.f, 0.f, 0.f, 0.f};  // P, t13, t23, t33 of plane K+2 at the own cell
       // ------------------------------------------------------------ 4 ----
-      if (got) {
-        if (K == Kfirst) closure_plane(K + 1, own);
-        closure_plane(K + 2, own);
-      }
+      if (got) closure_planes(K == Kfirst ? K + 1 : K + 2, K + 2, own);
       bool step_ok = got;
       if (is_out && got) {
         // ------------------------------------------------------------ 5 ----
@@ -456,12 +471,12 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
               } else if (f == 5) {
                 a0 = pK[op];
                 a1 = pK1[op];
-                a2 = own[r][0];
+                a2 = own[0];
               } else {
                 const int c = tau_row<2>(f - 6);
                 a0 = tK[c * PL2 + op];
                 a1 = tK1[c * PL2 + op];
-                a2 = own[r][f - 5];
+                a2 = own[f - 5];
               }
               const float s = strip_slope<LIM>(a1 - a0, a2 - a1);
               qr[f] = fmaf(-hz, s, a1);
