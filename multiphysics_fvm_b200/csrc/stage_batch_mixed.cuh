@@ -21,8 +21,8 @@ constexpr int MIX_NT = 160;
 constexpr int MIX_NBAR = 7;
 // Relative cost of a unit in the balanced split of the launch: a Navier-Stokes
 // plane (or row tile) of 32 x 8 cells against a heat plane of 32 x 20 (or 32 x
-// 10).  Step of 64 + 32 grids (12,275 and 40,085 units) at 5:2, 3:1, 7:2, 4:1
-// and 5:1: 1195, 1178, 1197, 1235 and 1333 us.
+// 10).  Of 64 + 32 grids (12,275 and 40,085 units) the first alone take 106 us a
+// stage, the others alone 122: 2.8 to 1 per unit.
 constexpr int MIX_NS_COST = 6, MIX_HEAT_COST = 2, MIX_HEAT_COST_ALT = 1;
 constexpr int MIX_NS_TY = MIX_NS_R * MIX_NS_NW, MIX_HEAT_TY = 4 * MIX_HEAT_NW, MIX_HEAT_TY_ALT = 2 * MIX_HEAT_NW;
 static_assert(NsStripCfg<MIX_NS_R, MIX_NS_NW>::NT == MIX_NT && HeatPcCfg<4, MIX_HEAT_NW>::NT == MIX_NT,
@@ -35,7 +35,14 @@ __host__ __device__ constexpr int mixed_bar_offset(int nbuf) {
                        HeatPcCfg<4, MIX_HEAT_NW>::NSLOT * HeatPcCfg<4, MIX_HEAT_NW>::SLOT * 4),
                   8);
 }
-__host__ __device__ constexpr int mixed_bytes(int nbuf) { return mixed_bar_offset(nbuf) + MIX_NBAR * 8; }
+// ... and the parameters of the Navier-Stokes piece in work.  (Read from global
+// memory they are loaded again after every store of a step, in which the compiler
+// must suppose an alias; a heat piece, with registers to spare, copies its own
+// to them.  Stage of 64 + 32 grids 301 -> 262 us.)
+__host__ __device__ constexpr int mixed_param_offset(int bar_off) { return (bar_off + MIX_NBAR * 8 + 15) & ~15; }
+__host__ __device__ constexpr int mixed_bytes(int nbuf) {
+  return mixed_param_offset(mixed_bar_offset(nbuf)) + (int)sizeof(NsParams<float>);
+}
 
 // Per grid and stage: what a tile of that grid needs.
 struct alignas(64) MixedInst {
@@ -89,15 +96,21 @@ __global__ void __launch_bounds__(MIX_NT, 3) batch_mixed_kernel(const __grid_con
     const MixedInst& in = src.inst[inst];
     if (in.kind == 0) {
       if (in.ns.active && !*in.ns.active) continue;  // this grid's clock passed t_end
-      if (in.ns.flat)
+      NsParams<float>& ns = *reinterpret_cast<NsParams<float>*>(smem_raw + mixed_param_offset(src.bar_off));
+      // (the last piece's readers are past the barrier that ended it)
+      for (int q = tid; q < (int)sizeof(ns); q += MIX_NT)  // by bytes, which may alias every field
+        reinterpret_cast<unsigned char*>(&ns)[q] = reinterpret_cast<const unsigned char*>(&in.ns)[q];
+      __syncthreads();
+      if (ns.flat)
         ok = ns_strip_tile<LIM, RIEM, MIX_NS_R, MIX_NS_NW, COORD_CART, true>(
-            in.ns, &in.tmap, &in.u0map, &in.accmap, pc, smem_raw, bars, bars + 6, 6, phase_bits, pending);
+            ns, &in.tmap, &in.u0map, &in.accmap, pc, smem_raw, bars, bars + 6, 6, phase_bits, pending);
       else
         ok = ns_strip_tile<LIM, RIEM, MIX_NS_R, MIX_NS_NW, COORD_CART, false>(
-            in.ns, &in.tmap, &in.u0map, &in.accmap, pc, smem_raw, bars, bars + 6, 6, phase_bits, pending);
+            ns, &in.tmap, &in.u0map, &in.accmap, pc, smem_raw, bars, bars + 6, 6, phase_bits, pending);
     } else {
       if (in.heat.active && !*in.heat.active) continue;
-      ok = heat_pc_tile<HCOORD, HVX, MIX_HEAT_NW>(in.heat, &in.tmap, pc, smem_raw, bars, phase_bits, pending);
+      const HeatParams<float> heat = in.heat;
+      ok = heat_pc_tile<HCOORD, HVX, MIX_HEAT_NW>(heat, &in.tmap, pc, smem_raw, bars, phase_bits, pending);
     }
   }
   // On a timeout, wait (bounded) for every copy this block may still have in flight.
