@@ -213,6 +213,39 @@ struct ColMetric {
   }
 };
 
+// ------------------------------------------------------- packed float32 ----
+// Two float32 values in one 64-bit register, with the packed add, subtract,
+// multiply and fused multiply-add of sm_100a: each half rounds as the scalar
+// instruction does, and one issue slot does two cells' work.
+struct F2 {
+  unsigned long long v;
+  __device__ __forceinline__ F2() {}
+  __device__ __forceinline__ F2(float lo, float hi) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi)); }
+  __device__ __forceinline__ explicit F2(float a) : F2(a, a) {}
+  __device__ __forceinline__ float lo() const { return __uint_as_float((unsigned)v); }
+  __device__ __forceinline__ float hi() const { return __uint_as_float((unsigned)(v >> 32)); }
+};
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) {
+  F2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+  return d;
+}
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) {
+  F2 d;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+  return d;
+}
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) {
+  F2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+  return d;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return d;
+}
+
 // ------------------------------------------------------------ limiters ----
 __device__ __forceinline__ float sgn(float x) { return x > 0.f ? 1.f : (x < 0.f ? -1.f : 0.f); }
 

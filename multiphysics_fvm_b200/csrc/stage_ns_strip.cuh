@@ -15,11 +15,11 @@
 //   1. thread 0 issues the TMA of plane K+2 into the slot that plane K-1 left,
 //      and of this plane's U0 / k-accumulator tile when the stage combination
 //      reads them;
-//   2. x2 and x1 for plane K in one sweep up the strip: x2 slopes and face
-//      fluxes in registers (the strip computes its R+1 faces itself), x1 slopes
-//      per row with the left slope and the right-face flux from neighbouring
-//      lanes by shuffle (lane 0 / lane 31 from the halo warp's data).  The halo
-//      warp meanwhile forms that data for plane K+1;
+//   2. x1 and x2 for plane K: x1 slopes of both rows with the left slope and the
+//      right-face flux from neighbouring lanes by shuffle (lane 0 / lane 31 from
+//      the halo warp's data), then x2 slopes and fluxes in registers (the strip
+//      computes its three faces itself).  The halo warp meanwhile forms that data
+//      for plane K+1;
 //   3. every thread waits (bounded) for plane K+2;
 //   4. P of plane K+2: own cells by their owners (kept in registers), halo
 //      cells by the halo warp (navier_stokes.py:94-100);
@@ -67,6 +67,7 @@ struct NsStripCfg {
   static constexpr unsigned STG_BYTES = STG * 4;
   // dynamic shared memory with `nbuf` staged tiles (0: none, 1: U0 or acc, 2: both)
   static constexpr int bytes(int nbuf) { return STG_OFF_BYTES + nbuf * (int)STG_BYTES; }
+  static_assert(R == 2, "the two rows of a thread's strip share packed registers");
   static_assert(2 * TY <= 32, "one halo lane per tile row and task");
   static_assert((SLOT * 4) % 128 == 0 && (STG_BYTES % 128) == 0, "TMA destinations need 128-byte alignment");
 };
@@ -149,6 +150,52 @@ __device__ __forceinline__ void strip_flux(const float* qL, const float* qR, flo
   const float vL = qL[1 + D] * irL, vR = qR[1 + D] * irR;
   const float cL = sqrt_approx((gam * qL[5]) * irL), cR = sqrt_approx((gam * qR[5]) * irR);
   strip_combine<D, RIEM>(qL, qR, vL, vR, cL, cR, F);
+}
+
+// strip_slope, strip_flux of two faces at once, one in each half of the packed
+// registers: the kernel is bound by issue and latency, and the x1 and x3 faces of a
+// strip's two rows, and two of its three x2 faces, cost their adds and multiplies
+// once (837 -> 700 thread instructions per cell; 256^3 stage 575 -> 541 us,
+// 97x130x61 51.6 -> 48.4, one-plane 64x64 5.99 -> 5.0).
+template <int LIM>
+__device__ __forceinline__ F2 strip_slope2(F2 a, F2 b) {
+  return F2(strip_slope<LIM>(a.lo(), b.lo()), strip_slope<LIM>(a.hi(), b.hi()));
+}
+template <int LIM>
+__device__ __forceinline__ F2 strip_state2(F2 h, F2 s, F2 q) {
+  if constexpr (LIM == LIM_PC) return q;
+  else return fma2(h, s, q);
+}
+template <int D, int RIEM>
+__device__ __forceinline__ void strip_flux2(const F2* qL, const F2* qR, float gam, F2* F) {
+  const F2 g2(gam);
+  const F2 irL(rcp_approx(qL[0].lo()), rcp_approx(qL[0].hi())), irR(rcp_approx(qR[0].lo()), rcp_approx(qR[0].hi()));
+  const F2 vL = qL[1 + D] * irL, vR = qR[1 + D] * irR;
+  const F2 c2L = (g2 * qL[5]) * irL, c2R = (g2 * qR[5]) * irR;
+  const F2 cL(sqrt_approx(c2L.lo()), sqrt_approx(c2L.hi())), cR(sqrt_approx(c2R.lo()), sqrt_approx(c2R.hi()));
+  // c below is -c of strip_combine, with the states' difference turned round
+  F2 a, b, c;
+  if constexpr (RIEM == RIEM_HLL) {
+    const F2 lL = cL - vL, lR = cR - vR, uL = vL + cL, uR = vR + cR;
+    const F2 sl(fmaxf(fmaxf(lL.lo(), lR.lo()), 0.f), fmaxf(fmaxf(lL.hi(), lR.hi()), 0.f));  // -s-
+    const F2 sr(fmaxf(fmaxf(uL.lo(), uR.lo()), 0.f), fmaxf(fmaxf(uL.hi(), uR.hi()), 0.f));
+    const F2 dd = sr + sl;
+    const F2 rd(rcp_approx(fmaxf(dd.lo(), 1e-30f)), rcp_approx(fmaxf(dd.hi(), 1e-30f)));
+    a = sr * rd;
+    b = sl * rd;
+    c = sl * a;
+  } else {
+    const F2 h(0.5f);
+    const F2 uL = F2(fabsf(vL.lo()), fabsf(vL.hi())) + cL, uR = F2(fabsf(vR.lo()), fabsf(vR.hi())) + cR;
+    a = b = h;
+    c = h * F2(fmaxf(uL.lo(), uR.lo()), fmaxf(uL.hi(), uR.hi()));
+  }
+  const F2 av = a * vL, bv = b * vR;
+  F[0] = fma2(a, qL[1 + D], fma2(b, qR[1 + D], c * (qL[0] - qR[0])));
+#pragma unroll
+  for (int k = 1; k < 4; ++k) F[k] = fma2(av, qL[k], fma2(bv, qR[k], c * (qL[k] - qR[k])));
+  F[1 + D] = F[1 + D] + fma2(a, qL[5], b * qR[5]);
+  F[4] = fma2(av, qL[4] + qL[5], fma2(bv, qR[4] + qR[5], c * (qL[4] - qR[4])));
 }
 
 // P = (gamma - 1)(E - |m|^2 / (2 rho)) of one ring cell (navier_stokes.py:94-100).
@@ -319,20 +366,28 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
     // x3 state carried from step to step, per own cell: the left state of the
     // face above the last slope plane and the flux of the face below the
     // output plane
-    float qlz[R][NF], fzp[R][5];
+    F2 qlz[NF], fzp[5];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
+    for (int f = 0; f < NF; ++f) qlz[f] = F2(0.f);
 #pragma unroll
-      for (int f = 0; f < NF; ++f) qlz[r][f] = 0.f;
-#pragma unroll
-      for (int v = 0; v < 5; ++v) fzp[r][v] = 0.f;
-    }
+    for (int v = 0; v < 5; ++v) fzp[v] = F2(0.f);
+    // P of plane u at the thread's two cells, into P plane pp
+    auto pressure2 = [&](const float* u, float* pp) {
+      const int o = (w * R + HH) * W + lane + 4, op = (w * R + 2) * W2 + lane + 2;
+      const F2 P(strip_pressure(u + o, PL, gm1), strip_pressure(u + o + W, PL, gm1));
+      pp[op] = P.lo();
+      pp[op + W2] = P.hi();
+      return P;
+    };
 
+    static_assert(C::NSLOT == 3, "the U and P rings turn together");
+    int slot = flat ? 0 : pmod(Kfirst, C::NSLOT);
     const int nstep = flat ? nsteps : Zl - Kfirst + 1;
     for (int st = 0; st < nstep; ++st) {
       const int K = flat ? Kfirst : Kfirst + st;
       if (flat) y0 = ybase + st * TY;
-      const int sK = flat ? st % C::NSLOT : pmod(K, C::NSLOT), pK0 = flat ? 0 : pmod(K, 3);
+      const int sK = slot, pK0 = flat ? 0 : slot;
+      slot = slot == C::NSLOT - 1 ? 0 : slot + 1;
       const bool outstep = K >= Z0;
       const int sK1 = sK == C::NSLOT - 1 ? 0 : sK + 1, sK2 = sK1 == C::NSLOT - 1 ? 0 : sK1 + 1;
       const int pK1i = pK0 == 2 ? 0 : pK0 + 1, pK2i = pK1i == 2 ? 0 : pK1i + 1;
@@ -359,11 +414,9 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
           if (need_acc) tma_load_4d(gst + (need_u0 ? C::STG : 0), accmap, gbar, gxc, y0 + 1, K, 0);
         }
       }
-      float kv[R][5];
+      F2 kv[5];  // flux differences of the two rows
 #pragma unroll
-      for (int r = 0; r < R; ++r)
-#pragma unroll
-        for (int v = 0; v < 5; ++v) kv[r][v] = 0.f;
+      for (int v = 0; v < 5; ++v) kv[v] = F2(0.f);
       if constexpr (flat) {
         // the plane itself, its P over the tile + 2 and the halo warp's x1
         // data, before the sweep
@@ -372,11 +425,7 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
           phase_bits ^= 1u << sK;
           if (tid == 0) pending &= ~(1u << sK);
           if (is_out) {
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-              const int ty = w * R + r;
-              pK[(ty + 2) * W2 + lane + 2] = strip_pressure(uK + (ty + HH) * W + lane + 4, PL, gm1);
-            }
+            pressure2(uK, pK);
           } else {
             border_p(pK, uK);
           }
@@ -392,74 +441,62 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
         if (outstep) {
           const int par = K & 1;
           const int jb = y0 + w * R;  // first row of the strip
-          auto ldf = [&](float* f, int ty, int tx) {
-            const int o = (ty + HH) * W + tx + 4;
-#pragma unroll
-            for (int v = 0; v < 5; ++v) f[v] = uK[v * PL + o];
-            f[5] = pK[(ty + 2) * W2 + tx + 2];
+          auto ld = [&](int f, int ty, int tx) {
+            return f < 5 ? uK[f * PL + (ty + HH) * W + tx + 4] : pK[(ty + 2) * W2 + tx + 2];
           };
-          float fa[NF], fb[NF], fc[NF], ql[NF];
-          ldf(fa, w * R - 2, lane);
-          ldf(fb, w * R - 1, lane);
+          auto ld2 = [&](int f, int ty, int tx) { return F2(ld(f, ty, tx), ld(f, ty + 1, tx)); };
+          const int ty = w * R;  // first row of the strip
+          {
+            // x1 of both rows (cells i, rows jb and jb + 1): the flux through
+            // the cells' left faces, the right faces' from the next lane
+            F2 qlx[NF], qrx[NF], F[5];
+            const F2 hx(i >= nx ? 0.f : -HS);  // i == nx: the right ghost column
 #pragma unroll
-          for (int t = 0; t <= R + 1; ++t) {
-            // row ty = w*R - 1 + t: its x2 slope; for t >= 1 the x2 face
-            // below it (the upper face of own row t - 2, the lower face of
-            // own row t - 1); for 1 <= t <= R (own rows) its x1 work
-            const int ty = w * R - 1 + t;
-            const int j = jb - 1 + t;
-            ldf(fc, ty + 1, lane);
-            const float hy = j < 0 || j >= ny ? 0.f : HS;  // zero slope in a ghost cell
-            float s[NF];
-#pragma unroll
-            for (int f = 0; f < NF; ++f) s[f] = strip_slope<LIM>(fb[f] - fa[f], fc[f] - fb[f]);
-            if (t >= 1) {
-              float qr[NF], F[5];
-#pragma unroll
-              for (int f = 0; f < NF; ++f) qr[f] = fmaf(-hy, s[f], fb[f]);
-              strip_flux<1, RIEM>(ql, qr, gam, F);
-              if (t >= 2) {
-                const int jc = min(max(j - 1, 0), ny - 1);
-                const float idym = cm.a2(p.met, jc, jc + 1);
-#pragma unroll
-                for (int v = 0; v < 5; ++v) kv[t - 2][v] = fmaf(F[v], idym, kv[t - 2][v]);
-              }
-              if (t <= R) {
-                const int jc = min(j, ny - 1);
-                const float idy = cm.a2(p.met, jc, jc);
-#pragma unroll
-                for (int v = 0; v < 5; ++v) kv[t - 1][v] = fmaf(-F[v], idy, kv[t - 1][v]);
-              }
+            for (int f = 0; f < NF; ++f) {
+              const F2 fm = ld2(f, ty, lane - 1), f0 = ld2(f, ty, lane), fp = ld2(f, ty, lane + 1);
+              const F2 s1 = strip_slope2<LIM>(f0 - fm, fp - f0);
+              const float ua = __shfl_up_sync(0xffffffffu, s1.lo(), 1), ub = __shfl_up_sync(0xffffffffu, s1.hi(), 1);
+              const float* h = hl + (par * NF + f) * TY + ty;
+              qlx[f] = strip_state2<LIM>(F2(HS), lane == 0 ? F2(h[0], h[1]) : F2(ua, ub), fm);
+              qrx[f] = strip_state2<LIM>(hx, s1, f0);
             }
+            strip_flux2<0, RIEM>(qlx, qrx, gam, F);
 #pragma unroll
-            for (int f = 0; f < NF; ++f) ql[f] = fmaf(hy, s[f], fb[f]);
-            if (t >= 1 && t <= R) {
-              // x1 for own row r = t - 1 (cell i, row j): the flux through
-              // the cell's left face, the right face's from the next lane
-              const int r = t - 1;
-              float fm[NF], fp[NF], qlx[NF], qrx[NF], F[5];
-              ldf(fm, ty, lane - 1);
-              ldf(fp, ty, lane + 1);
-              const float hx = i >= nx ? 0.f : HS;  // i == nx: the right ghost column
-#pragma unroll
-              for (int f = 0; f < NF; ++f) {
-                const float s1 = strip_slope<LIM>(fb[f] - fm[f], fp[f] - fb[f]);
-                const float su = __shfl_up_sync(0xffffffffu, s1, 1);
-                const float sl = lane == 0 ? hl[(par * NF + f) * TY + ty] : su;
-                qlx[f] = fmaf(HS, sl, fm[f]);
-                qrx[f] = fmaf(-hx, s1, fb[f]);
-              }
-              strip_flux<0, RIEM>(qlx, qrx, gam, F);
-#pragma unroll
-              for (int v = 0; v < 5; ++v) {
-                const float fd = __shfl_down_sync(0xffffffffu, F[v], 1);
-                const float fe = lane == 31 ? fr[(par * 5 + v) * TY + ty] : fd;
-                if constexpr (COORD == COORD_CART) kv[r][v] = fmaf(fe - F[v], cm.a1p, kv[r][v]);
-                else kv[r][v] = fmaf(fe, cm.a1p, fmaf(-F[v], cm.a1m, kv[r][v]));
-              }
+            for (int v = 0; v < 5; ++v) {
+              const float da = __shfl_down_sync(0xffffffffu, F[v].lo(), 1), db = __shfl_down_sync(0xffffffffu, F[v].hi(), 1);
+              const float* e = fr + (par * 5 + v) * TY + ty;
+              const F2 fe = lane == 31 ? F2(e[0], e[1]) : F2(da, db);
+              if constexpr (COORD == COORD_CART) kv[v] = (fe - F[v]) * F2(cm.a1p);
+              else kv[v] = fma2(fe, F2(cm.a1p), F[v] * F2(-cm.a1m));
             }
+          }
+          {
+            // x2: slopes of rows jb - 1 .. jb + 2 (zero in a ghost cell), the
+            // faces below rows jb and jb + 1 as a pair and the one above
+            F2 ql[NF], qr[NF], F[5];
+            float ql1[NF], qr1[NF], F1[5];
+            float hy[4];
 #pragma unroll
-            for (int f = 0; f < NF; ++f) { fa[f] = fb[f]; fb[f] = fc[f]; }
+            for (int r = 0; r < 4; ++r) hy[r] = jb + r - 1 < 0 || jb + r - 1 >= ny ? 0.f : HS;
+#pragma unroll
+            for (int f = 0; f < NF; ++f) {
+              float g[6], s[4];
+#pragma unroll
+              for (int r = 0; r < 6; ++r) g[r] = ld(f, ty - 2 + r, lane);
+#pragma unroll
+              for (int r = 0; r < 4; ++r) s[r] = strip_slope<LIM>(g[r + 1] - g[r], g[r + 2] - g[r + 1]);
+              ql[f] = strip_state2<LIM>(F2(hy[0], hy[1]), F2(s[0], s[1]), F2(g[1], g[2]));
+              qr[f] = strip_state2<LIM>(F2(-hy[1], -hy[2]), F2(s[1], s[2]), F2(g[2], g[3]));
+              ql1[f] = fmaf(hy[2], s[2], g[3]);
+              qr1[f] = fmaf(-hy[3], s[3], g[4]);
+            }
+            strip_flux2<1, RIEM>(ql, qr, gam, F);
+            strip_flux<1, RIEM>(ql1, qr1, gam, F1);
+            const int ja = min(jb, ny - 1), jc = min(jb + 1, ny - 1);
+            const F2 lower(-cm.a2(p.met, ja, ja), -cm.a2(p.met, jc, jc));
+            const F2 upper(cm.a2(p.met, ja, ja + 1), cm.a2(p.met, jc, jc + 1));
+#pragma unroll
+            for (int v = 0; v < 5; ++v) kv[v] = fma2(F2(F[v].hi(), F1[v]), upper, fma2(F[v], lower, kv[v]));
           }
         }
       } else {
@@ -474,9 +511,8 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
       // barrier here.  A thread whose wait ran out skips the rest of the step
       // and the barrier at its end takes the block out.
       bool got = true;
-      if constexpr (!flat)
-      for (int pl = (K == Kfirst ? Kfirst : K + 2); pl <= K + 2; ++pl) {
-        const int s = pmod(pl, C::NSLOT);
+      for (int pl = (flat ? K + 3 : (K == Kfirst ? Kfirst : K + 2)); pl <= K + 2; ++pl) {
+        const int s = pl == K + 2 ? sK2 : pl == K + 1 ? sK1 : sK;
         const bool g = got && mbar_wait_bounded(&bars[s], (phase_bits >> s) & 1u, p.wait_ns);
         if (g) {
           phase_bits ^= 1u << s;
@@ -491,50 +527,42 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
       } else if (is_out) {
         if constexpr (!flat) {  // x3 (a flat grid has none)
           // ------------------------------------------------------------ 4 ----
-          float pnew[R];
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            const int ty = w * R + r;
-            const int o = (ty + HH) * W + lane + 4, op = (ty + 2) * W2 + lane + 2;
-            pnew[r] = strip_pressure(uK2 + o, PL, gm1);
-            pK2[op] = pnew[r];
-            if (K == Kfirst) {
-              pK[op] = strip_pressure(uK + o, PL, gm1);
-              pK1[op] = strip_pressure(uK1 + o, PL, gm1);
-            }
+          const int ty = w * R;
+          const int o = (ty + HH) * W + lane + 4, op = (ty + 2) * W2 + lane + 2;
+          const F2 pnew = pressure2(uK2, pK2);
+          if (K == Kfirst) {
+            pressure2(uK, pK);
+            pressure2(uK1, pK1);
           }
           // ------------------------------------------------------------ 5 ----
           // slope of plane K+1 (zero on a ghost plane) and the flux at K+1/2
           const float hz = K + 1 <= 0 || K + 1 >= nz + 1 ? 0.f : HS;
           const bool zface = K >= Z0 - 1;
           const float idz = outstep ? __ldg(p.met.inv_dx3 + (K - 1)) : 0.f;
+          F2 qr[NF], qn[NF];
 #pragma unroll
-          for (int r = 0; r < R; ++r) {
-            const int ty = w * R + r;
-            const int o = (ty + HH) * W + lane + 4, op = (ty + 2) * W2 + lane + 2;
-            float qr[NF], qn[NF];
-#pragma unroll
-            for (int f = 0; f < NF; ++f) {
-              const float a0 = f < 5 ? uK[f * PL + o] : pK[op];
-              const float a1 = f < 5 ? uK1[f * PL + o] : pK1[op];
-              const float a2 = f < 5 ? uK2[f * PL + o] : pnew[r];
-              const float s = strip_slope<LIM>(a1 - a0, a2 - a1);
-              qr[f] = fmaf(-hz, s, a1);
-              qn[f] = fmaf(hz, s, a1);
-            }
-            if (zface) {
-              float F[5];
-              strip_flux<2, RIEM>(qlz[r], qr, gam, F);
-              const float a3 = cm.a3(p.met, min(y0 + ty, ny - 1), idz);
-#pragma unroll
-              for (int v = 0; v < 5; ++v) {
-                kv[r][v] = fmaf(F[v] - fzp[r][v], a3, kv[r][v]);
-                fzp[r][v] = F[v];
-              }
-            }
-#pragma unroll
-            for (int f = 0; f < NF; ++f) qlz[r][f] = qn[f];
+          for (int f = 0; f < NF; ++f) {
+            const float* b0 = f < 5 ? uK + f * PL + o : pK + op;
+            const float* b1 = f < 5 ? uK1 + f * PL + o : pK1 + op;
+            const int up = f < 5 ? W : W2;  // one row up
+            const F2 a0(b0[0], b0[up]), a1(b1[0], b1[up]);
+            const F2 a2 = f < 5 ? F2(uK2[f * PL + o], uK2[f * PL + o + W]) : pnew;
+            const F2 s = strip_slope2<LIM>(a1 - a0, a2 - a1);
+            qr[f] = strip_state2<LIM>(F2(-hz), s, a1);
+            qn[f] = strip_state2<LIM>(F2(hz), s, a1);
           }
+          if (zface) {
+            F2 F[5];
+            strip_flux2<2, RIEM>(qlz, qr, gam, F);
+            const F2 a3(cm.a3(p.met, min(y0 + ty, ny - 1), idz), cm.a3(p.met, min(y0 + ty + 1, ny - 1), idz));
+#pragma unroll
+            for (int v = 0; v < 5; ++v) {
+              kv[v] = fma2(F[v] - fzp[v], a3, kv[v]);
+              fzp[v] = F[v];
+            }
+          }
+#pragma unroll
+          for (int f = 0; f < NF; ++f) qlz[f] = qn[f];
         }
         // ------------------------------------------------------------ 6 ----
         if (outstep) {
@@ -548,34 +576,78 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
           }
           step_ok = step_ok && staged_ok;
           unsigned bad = staged_ok ? 0u : ST_TMA_TIMEOUT;
-          const int jb = y0 + w * R;
+          const int ty = w * R, jb = y0 + ty;
+          if (i < nx && jb < ny && staged_ok) {
+            const bool two = jb + 1 < ny;  // the strip's second row is inside the grid
+            // where the combination reads U, U0 and the accumulator of the two
+            // cells: first cell, next variable, next row
+            struct Src {
+              const float* q;
+              int var, row;
+              __device__ __forceinline__ F2 operator[](int v) const { return F2(q[v * var], q[v * var + row]); }
+            };
+            const Src cur{uK + (ty + HH) * W + lane + 4, PL, W};
+            const Src u0 = need_u0 ? Src{gu0 + ty * TX + lane, TY * TX, TX} : cur;
+            const Src ac = need_acc ? Src{gacc + ty * TX + lane, TY * TX, TX} : cur;
+            const Src base = sc.mode == MODE_AXPY ? u0 : (sc.mode == MODE_FINAL ? ac : cur);
+            const Src abase = sc.set ? u0 : ac;
+            F2 q[5];
 #pragma unroll
-          for (int r = 0; r < R; ++r) {
-            const int ty = w * R + r, j = jb + r;
-            if (i < nx && j < ny && staged_ok) {
-              const int o = (ty + HH) * W + lane + 4;
-              float q[5];
+            for (int v = 0; v < 5; ++v) q[v] = cur[v];
+            // gravity (navier_stokes.py:499-504): rho g and rho g.v = g.m
+            const F2 gx2(gx), gy2(gy), gz2(gz);
+            F2 k[5];
+            k[0] = F2(0.f) - kv[0];
+            k[1] = q[0] * gx2 - kv[1];
+            k[2] = q[0] * gy2 - kv[2];
+            k[3] = q[0] * gz2 - kv[3];
+            k[4] = fma2(gx2, q[1], fma2(gy2, q[2], gz2 * q[3])) - kv[4];
+            if constexpr (COORD != COORD_CART) {
+              float s[2][4], qs[2][5];
 #pragma unroll
-              for (int v = 0; v < 5; ++v) q[v] = uK[v * PL + o];
-              // gravity (navier_stokes.py:499-504): rho g and rho g.v = g.m
-              float sg[5] = {0.f, q[0] * gx, q[0] * gy, q[0] * gz, fmaf(gx, q[1], fmaf(gy, q[2], gz * q[3]))};
-              if constexpr (COORD != COORD_CART)
-                curvilinear_source<COORD>(cm, p.met, j, q, pK[(ty + 2) * W2 + lane + 2], nullptr, sg);
-              const long long g = L.idx(0, K, j + 1, i + 1);
-              const int so = ty * TX + lane;
+              for (int v = 0; v < 5; ++v) qs[0][v] = q[v].lo(), qs[1][v] = q[v].hi();
 #pragma unroll
-              for (int v = 0; v < 5; ++v) {
-                const float k = sg[v] - kv[r][v];
-                const float u0v = need_u0 ? gu0[v * TY * TX + so] : q[v];
-                const float accv = need_acc ? gacc[v * TY * TX + so] : 0.f;
-                const long long gi = g + (long long)v * L.var_stride;
-                const float o2 = sc.combine(k, q[v], u0v, accv);
-                p.out[gi] = o2;
-                if (p.coef.accmode != ACC_NONE) p.acc[gi] = sc.acc(k, u0v, accv);
-                if (!isfinite(o2)) bad |= ST_NONFINITE;
-                if (v == 0 && p.coef.mode != MODE_RHS && !(o2 > 0.f)) bad |= ST_DENSITY;
+              for (int r = 0; r < 2; ++r) {
+                s[r][1] = s[r][2] = s[r][3] = 0.f;
+                curvilinear_source<COORD>(cm, p.met, min(jb + r, ny - 1), qs[r], pK[(ty + r + 2) * W2 + lane + 2],
+                                          nullptr, s[r]);
               }
+#pragma unroll
+              for (int v = 1; v < 4; ++v) k[v] = k[v] + F2(s[0][v], s[1][v]);
             }
+            // (read once: a batch's parameters lie in global memory, and a load
+            // between the stores would have to be repeated after each)
+            const long long g = L.idx(0, K, jb + 1, i + 1), pitch = L.pitch, var_stride = L.var_stride;
+            const F2 dt2(sc.dt), c2(sc.c), cb2(sc.cb), w2(sc.w);
+            bool fin0 = true, fin1 = true;
+            float* po = p.out + g;
+            float* pa = p.acc + g;
+            const bool wacc = p.coef.accmode != ACC_NONE, ssp = sc.mode == MODE_SSP, rhs = sc.mode == MODE_RHS;
+#pragma unroll
+            for (int v = 0; v < 5; ++v) {
+              F2 o;
+              if (ssp) {
+                const F2 b = u0[v];
+                o = fma2(cb2, fma2(dt2, k[v], q[v] - b), b);
+              } else {
+                o = fma2(c2, k[v], rhs ? F2(0.f) : base[v]);
+              }
+              po[0] = o.lo();
+              if (two) po[pitch] = o.hi();
+              fin0 = fin0 && isfinite(o.lo());
+              fin1 = fin1 && isfinite(o.hi());
+              if (v == 0 && !rhs) {
+                if (!(o.lo() > 0.f) || (two && !(o.hi() > 0.f))) bad |= ST_DENSITY;
+              }
+              if (wacc) {
+                const F2 na = fma2(w2, k[v], abase[v]);
+                pa[0] = na.lo();
+                if (two) pa[pitch] = na.hi();
+              }
+              po += var_stride;
+              pa += var_stride;
+            }
+            if (!fin0 || (two && !fin1)) bad |= ST_NONFINITE;
           }
           if (bad) atomicOr(p.status, bad);
         }
