@@ -160,10 +160,13 @@ cudaError_t launch_ns_strip_ty(const NsStripSource& src, int nbuf, cudaStream_t 
   static int bps[3] = {0, 0, 0};
   if (bps[0] == 0 || nsm < 0) {
     // occupancy with 0, 1 and 2 staged tiles; the attribute ends at the largest
+    // (bps[0] is set last: another thread takes it as the sign that all are there)
+    int b[3];
     for (int nb = 0; nb < 3; ++nb) {
-      cudaError_t e = prepare_kernel(kern, C::NT, C::bytes(nb), &bps[nb]);
+      cudaError_t e = prepare_kernel(kern, C::NT, C::bytes(nb), &b[nb]);
       if (e != cudaSuccess) return e;
     }
+    bps[1] = b[1], bps[2] = b[2], bps[0] = b[0];
   }
   if (nsm < 0) return cudaSuccess;
   const long long ntiles = tile_total(src.p);
@@ -178,11 +181,11 @@ cudaError_t launch_ns_strip_lr(NsStripSource& src, int ty, int nbuf, cudaStream_
   NsParams<float>& p = src.p;
   set_tiles(p, ty, p.flat != 0);
   const bool alt = ty == NS_STRIP_TY_ALT;
-  if (p.flat || nsm < 0) {  // (a handle prepares both marches: residuals run the x3 one)
-    const cudaError_t e = alt ? launch_ns_strip_ty<LIM, RIEM, COORD, NS_STRIP_TY_ALT, true>(src, nbuf, s, nsm)
-                              : launch_ns_strip_ty<LIM, RIEM, COORD, NS_STRIP_TY, true>(src, nbuf, s, nsm);
-    if (nsm >= 0 || e != cudaSuccess) return e;
-  }
+  // (a handle prepares the march of its steps; a residual of a one-plane grid runs
+  // the x3 march and prepares it on its first call)
+  if (p.flat)
+    return alt ? launch_ns_strip_ty<LIM, RIEM, COORD, NS_STRIP_TY_ALT, true>(src, nbuf, s, nsm)
+               : launch_ns_strip_ty<LIM, RIEM, COORD, NS_STRIP_TY, true>(src, nbuf, s, nsm);
   return alt ? launch_ns_strip_ty<LIM, RIEM, COORD, NS_STRIP_TY_ALT, false>(src, nbuf, s, nsm)
              : launch_ns_strip_ty<LIM, RIEM, COORD, NS_STRIP_TY, false>(src, nbuf, s, nsm);
 }
