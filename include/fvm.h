@@ -68,7 +68,8 @@ extern "C" {
  * bc_kind/bc_value: [variable][side], sides ordered left,right,bottom,top,front,back
  * (src/solver.py:36).  tile_ty: tile rows, 0 = the default shape (or the alternative
  * one that fvm_tiling reports after fvm_autotune); zchunk: planes per tile, 0 = an
- * equal run of planes for every resident block. */
+ * equal run of planes for every resident block.  The depth never changes a result;
+ * in a batch of which some grids ask for a depth, 0 means 64 planes. */
 typedef struct fvm_desc {
   int physics, precision, coords;
   int nx1, nx2, nx3;

@@ -1345,6 +1345,20 @@ struct fvm_batch {
 
 namespace {
 
+// A launch's work is walked in one order (tile_walk.cuh): a group is balanced
+// where every member has depth 0; as soon as one asks for a depth of its own all
+// pieces are of fixed depth, and the members with depth 0 take this one.
+constexpr int BATCH_DEPTH = 64;
+int group_balanced(const fvm_batch* b, const fvm_batch::Group& g) {
+  for (int i : g.members)
+    if (b->h[i]->zchunk > 0) return 0;
+  return 1;
+}
+// The depth of a member's pieces in its group's launches.
+int member_depth(const fvm_batch::Group& g, const fvm_handle* h) {
+  return g.bal ? 0 : (h->zchunk > 0 ? h->zchunk : BATCH_DEPTH);
+}
+
 // Per-stage instance tables of the mixed group (float32 only).
 int build_mixed_arrays(fvm_batch* b, fvm_batch::Group& g) {
   const std::vector<StageDef> st = stage_table(b->integrator);
@@ -1354,7 +1368,7 @@ int build_mixed_arrays(fvm_batch* b, fvm_batch::Group& g) {
   g.nbuf.clear();
   g.starts = nullptr;
   g.ntiles = 0;
-  g.bal = b->h[g.members[0]]->zchunk == 0;
+  g.bal = group_balanced(b, g);
   std::vector<long long> starts(1, 0);
   for (size_t si = 0; si < st.size(); ++si) {
     std::vector<MixedInst> mi(g.members.size());
@@ -1367,6 +1381,7 @@ int build_mixed_arrays(fvm_batch* b, fvm_batch::Group& g) {
         m.u0map = h->smap;
         m.accmap = h->amap;
         m.ns = make_ns_params<float>(h, st[si], false);
+        m.ns.zchunk = member_depth(g, h);
         set_tiles(m.ns, MIX_NS_TY, m.ns.flat != 0);
         m.ncol = m.ns.ncol;
         m.nunit = m.ns.nunit;
@@ -1375,6 +1390,7 @@ int build_mixed_arrays(fvm_batch* b, fvm_batch::Group& g) {
       } else {
         m.kind = 1;
         m.heat = make_heat_params<float>(h, st[si], false);
+        m.heat.zchunk = member_depth(g, h);
         set_tiles(m.heat, g.heat_ty);
         m.ncol = m.heat.ncol;
         m.nunit = m.heat.nunit;
@@ -1408,7 +1424,7 @@ int build_group_arrays(fvm_batch* b, fvm_batch::Group& g) {
   g.maps.clear();
   g.starts = nullptr;
   g.ntiles = 0;
-  g.bal = b->h[g.members[0]]->zchunk == 0;
+  g.bal = group_balanced(b, g);
   std::vector<long long> starts(1, 0);
   for (size_t si = 0; si < st.size(); ++si) {
     std::vector<CUtensorMap> maps;
@@ -1417,6 +1433,7 @@ int build_group_arrays(fvm_batch* b, fvm_batch::Group& g) {
       std::vector<NsParams<Real>> ps;
       for (int i : g.members) {
         NsParams<Real> p = make_ns_params<Real>(b->h[i], st[si], false);
+        p.zchunk = member_depth(g, b->h[i]);
         set_tiles(p, g.visc ? ns_tile_ty<Real, true>() : ns_tile_ty<Real, false>());
         ps.push_back(p);
         maps.push_back(b->h[i]->tmap[st[si].in]);
@@ -1428,6 +1445,7 @@ int build_group_arrays(fvm_batch* b, fvm_batch::Group& g) {
       std::vector<HeatParams<Real>> ps;
       for (int i : g.members) {
         HeatParams<Real> p = make_heat_params<Real>(b->h[i], st[si], false);
+        p.zchunk = member_depth(g, b->h[i]);
         set_tiles(p, HEAT_TY);
         ps.push_back(p);
         maps.push_back(b->h[i]->tmap[st[si].in]);
