@@ -62,19 +62,15 @@ cudaError_t launch_ns_src(const Src& src, long long ntiles, cudaStream_t s, int 
   return cudaGetLastError();
 }
 
-// One grid: float64, and the viscous float32 grids' second block shape
-// (inviscid float32 grids always run the register-blocked kernel).
+// One grid: float64, the viscous float32 grids' second block shape, and single
+// calls on a float32 member of a batch that runs these kernels.
 template <typename Real, int LIM, int RIEM, int COORD, bool VISC>
 cudaError_t launch_ns_one(const CUtensorMap& map, NsParams<Real> p, cudaStream_t s, int nsm) {
-  if constexpr (std::is_same<Real, float>::value && !VISC) {
-    return cudaErrorInvalidValue;
-  } else {
-    SingleSource<NsParams<Real>> src;
-    src.tmap = map;
-    set_tiles(p, ns_tile_ty<Real, VISC>());
-    src.p = p;
-    return launch_ns_src<Real, LIM, RIEM, COORD, VISC>(src, tile_total(p), s, nsm);
-  }
+  SingleSource<NsParams<Real>> src;
+  src.tmap = map;
+  set_tiles(p, ns_tile_ty<Real, VISC>());
+  src.p = p;
+  return launch_ns_src<Real, LIM, RIEM, COORD, VISC>(src, tile_total(p), s, nsm);
 }
 
 template <typename Real, int COORD>
