@@ -136,6 +136,7 @@ struct fvm_handle {
   CUtensorMap tmap[3];
   CUtensorMap smap{}, amap{};  // staged U0 / accumulator tiles (staged_kernel)
   bool legacy = false;         // batch member: runs the batched (tile-list) kernels
+  bool member = false;         // batch member: its block shape is its batch's
   unsigned long long wait_ns = 2000000000ull;  // limit of each wait for a TMA plane
   unsigned long long drain_ns = 1000000000ull; // limit of the wait for copies in flight after a timeout
   unsigned extra_tx = 0;                       // test of the timeout path (fvm_set_wait_limit)
@@ -1627,6 +1628,7 @@ int fvm_batch_create(const fvm_desc* descs, int n, fvm_batch** out) {
     int rc = fvm_create(&di, &h);
     if (rc) return bail(rc);
     b->h.push_back(h);
+    h->member = true;
     if (mixed) {  // the block shapes of the mixed launch's two bodies
       h->tile_ty = heat_pc_desc(di) ? mheat_ty : MIX_NS_TY;
       if ((rc = make_tmaps(h))) return bail(rc);
@@ -1862,8 +1864,10 @@ int fvm_autotune(fvm_handle* h, int* best_zchunk, double* best_ms) {
   if (rc) return rc;
   int best = h->zchunk, best_ty = h->tile_ty;
   double bt = 1e30;
-  std::vector<int> tys{default_tile_ty(h->d)};
-  if (alt_tile_ty(h->d) != tys[0]) tys.push_back(alt_tile_ty(h->d));
+  // (a batch member keeps the shape of its batch's kernels, which read its
+  // tensor maps: a map of another shape copies more than a kernel's ring slot holds)
+  std::vector<int> tys{h->member ? h->tile_ty : default_tile_ty(h->d)};
+  if (!h->member && alt_tile_ty(h->d) != tys[0]) tys.push_back(alt_tile_ty(h->d));
   for (int ty : tys) {
     h->tile_ty = ty;
     if ((rc = make_tmaps(h))) break;
