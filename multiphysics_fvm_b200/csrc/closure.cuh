@@ -516,7 +516,7 @@ struct WgCfg {
   static constexpr int OFF_X = 0;
   static constexpr int OFF_G = NSLOT * PLANEB + PADB;
   static constexpr int OFF_BAR = OFF_G + TY * GROWB;
-  static constexpr int NBAR = 2 * NSLOT + 2;     // full, empty, accumulators done, accumulators free
+  static constexpr int NBAR = 2 * NSLOT + 3;     // full, empty, accumulators done, accumulators free, drain
   static constexpr int USED = OFF_BAR + NBAR * 8 + 16;
   static constexpr int TCOLS = 9 * COUT <= 256 ? 256 : 512;
   // as many CTAs per SM as its tensor memory holds, never more
@@ -543,7 +543,8 @@ __global__ void __launch_bounds__(WgCfg<CIN, COUT>::NT, WgCfg<CIN, COUT>::CTAS) 
   uint64_t* empty = full + C::NSLOT;
   uint64_t* done = empty + C::NSLOT;
   uint64_t* accfree = done + 1;
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(accfree + 1);
+  uint64_t* drain = accfree + 1;
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(drain + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tslot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n1 = a.n1, n2 = a.n2, n3 = a.n3, len = a.zc;
@@ -553,6 +554,7 @@ __global__ void __launch_bounds__(WgCfg<CIN, COUT>::NT, WgCfg<CIN, COUT>::CTAS) 
   if (tid == 0) {
     mbar_init(done, 1);
     mbar_init(accfree, 4);
+    mbar_init(drain, 1);
     for (int s = 0; s < C::NSLOT; ++s) {
       mbar_init(&full[s], C::NLOAD);
       mbar_init(&empty[s], 1);
@@ -694,12 +696,13 @@ __global__ void __launch_bounds__(WgCfg<CIN, COUT>::NT, WgCfg<CIN, COUT>::CTAS) 
       o0 += len;
     }
     if (!ok) {
-      // drain this CTA's MMAs (bounded) before tensor memory is freed: a slot
-      // barrier's next phase completes with them
+      // drain this CTA's MMAs (bounded) before tensor memory is freed, on a
+      // barrier of its own: which phase `done` is in depends on where the wait
+      // ran out
       give_up();
-      if (elect_one()) umma_commit(done);
+      if (elect_one()) umma_commit(drain);
       __syncwarp();
-      mbar_wait_bounded(done, it & 1, WAIT_NS);
+      mbar_wait_bounded(drain, 0, WAIT_NS);
     }
     __syncwarp();
   } else {
