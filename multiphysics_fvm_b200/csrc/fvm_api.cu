@@ -597,14 +597,18 @@ int enqueue_step(fvm_handle* h, int dt_mode, Prof* pf) {
   return close(false);
 }
 
+// Prepare the kernel that the handle's steps launch (outside any capture): a
+// step's stage, as a one-plane grid's residual runs another march.
+cudaError_t prepare_stage(fvm_handle* h) {
+  const StageDef sd = stage_table(h->d.integrator).front();
+  return h->f64 ? launch_stage<double>(h, sd, false, true) : launch_stage<float>(h, sd, false, true);
+}
+
 int ensure_graph(fvm_handle* h, int dt_mode) {
   cudaGraphExec_t& ge = h->graph[dt_mode];
   if (ge) return FVM_OK;
   cudaGraph_t g;
-  {
-    StageDef sd{0, 1, MODE_RHS, ACC_NONE, 0, 0, 0};
-    FVM_CK(h->f64 ? launch_stage<double>(h, sd, true, true) : launch_stage<float>(h, sd, true, true));
-  }
+  FVM_CK(prepare_stage(h));
   FVM_CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   int rc = enqueue_step(h, dt_mode, nullptr);
   cudaError_t ce = cudaStreamEndCapture(h->stream, &g);
@@ -1813,14 +1817,14 @@ std::vector<int> zchunk_candidates(int nz) {
 
 // The z-march depth a handle reports: its fixed one, or the longest run of
 // planes that the balanced split gives a block.
-int reported_depth(fvm_handle* h) {
-  if (h->zchunk > 0) return h->zchunk;
-  StageDef sd{0, 1, MODE_RHS, ACC_NONE, 0, 0, 0};
-  const cudaError_t e = h->f64 ? launch_stage<double>(h, sd, true, true) : launch_stage<float>(h, sd, true, true);
-  if (e != cudaSuccess) return h->d.nx3;
+int reported_depth(fvm_handle* h, int* depth) {
+  *depth = h->zchunk;
+  if (h->zchunk > 0) return FVM_OK;
+  FVM_CK(prepare_stage(h));
   const long long units = (long long)((h->lay.nx + 31) / 32) * ((h->lay.ny + h->tile_ty - 1) / h->tile_ty) * h->lay.nz;
   const long long blocks = std::max(1LL, std::min(units, (long long)prepared_blocks * h->nsm));
-  return (int)std::min<long long>(h->d.nx3, (units + blocks - 1) / blocks);
+  *depth = (int)std::min<long long>(h->d.nx3, (units + blocks - 1) / blocks);
+  return FVM_OK;
 }
 
 struct Saved {
@@ -1892,16 +1896,14 @@ int fvm_autotune(fvm_handle* h, int* best_zchunk, double* best_ms) {
   if (rc) return rc;
   if (rr) return rr;
   if (rt) return rt;
-  if (best_zchunk) *best_zchunk = reported_depth(h);
   if (best_ms) *best_ms = bt / 3.0;
-  return FVM_OK;
+  return best_zchunk ? reported_depth(h, best_zchunk) : FVM_OK;
 }
 
 int fvm_tiling(fvm_handle* h, int* tile_ty, int* zchunk) {
   if (!h) return fail(FVM_E_INVALID, "null handle");
   if (tile_ty) *tile_ty = h->tile_ty;
-  if (zchunk) *zchunk = reported_depth(h);
-  return FVM_OK;
+  return zchunk ? reported_depth(h, zchunk) : FVM_OK;
 }
 
 int fvm_batch_autotune(fvm_batch* b, int* best_zchunk, double* best_ms) {
