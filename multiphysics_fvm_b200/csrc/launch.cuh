@@ -1,6 +1,8 @@
 // Launch helpers for the fused stage kernels: persistent grids sized from the
 // occupancy of each instantiation, runtime dispatch over the scheme enums.
 #pragma once
+#include <algorithm>
+#include <atomic>
 #include <type_traits>
 #include "stage_ns.cuh"
 #include "stage_ns_strip.cuh"
@@ -28,20 +30,40 @@ constexpr int HEAT_TY = 8, HEAT_TY_ALT = 4;
 // this thread (of a kernel with several shared-memory sizes, its largest).
 inline thread_local int prepared_blocks = 0;
 
-template <typename K>
-static cudaError_t prepare_kernel(K kern, int threads, int bytes, int* blocks_per_sm) {
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+// Resident blocks per SM of one kernel with each of its N shared-memory sizes.
+// The launchers' are process-wide and handles may be made and stepped from
+// several threads: blocks[0], written last, says that all are there.
+template <int N>
+struct Residency {
+  std::atomic<int> blocks[N] = {};
+  bool known() const { return blocks[0].load(std::memory_order_acquire) != 0; }
+  long long operator[](int k) const { return blocks[k].load(std::memory_order_relaxed); }
+};
+
+// Prepare a kernel that runs with bytes[0] < bytes[1] < ... of dynamic shared
+// memory: its limit goes to the largest at once, and never below what another
+// thread may be launching with.
+template <typename K, int N>
+static cudaError_t prepare_kernel(K kern, int threads, const int (&bytes)[N], Residency<N>& res) {
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes[N - 1]);
   if (e != cudaSuccess) return e;
   // all of the unified L1/shared array as shared memory: the ring planes are
   // the blocks' working set, so more resident blocks beat a larger L1
   e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kern, threads, bytes);
-  if (e != cudaSuccess) return e;
-  if (*blocks_per_sm < 1) return cudaErrorInvalidConfiguration;
-  prepared_blocks = *blocks_per_sm;
+  int blocks[N];
+  for (int k = 0; k < N; ++k) {
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[k], kern, threads, bytes[k]);
+    if (e != cudaSuccess) return e;
+    if (blocks[k] < 1) return cudaErrorInvalidConfiguration;
+  }
+  for (int k = N - 1; k > 0; --k) res.blocks[k].store(blocks[k], std::memory_order_relaxed);
+  res.blocks[0].store(blocks[0], std::memory_order_release);
+  prepared_blocks = blocks[N - 1];
   return cudaSuccess;
 }
+// Blocks of a persistent launch over `ntiles` tiles.
+inline int grid_blocks(long long ntiles, long long resident, int nsm) { return (int)std::min(ntiles, resident * nsm); }
 
 // nsm < 0: only set the kernel's shared-memory attribute and query its
 // occupancy (done once, outside any stream capture).
@@ -50,14 +72,14 @@ cudaError_t launch_ns_src(const Src& src, long long ntiles, cudaStream_t s, int 
   constexpr int TY = ns_tile_ty<Real, VISC>();
   using C = NsCfg<Real, VISC, TY>;
   auto kern = ns_stage_kernel<Real, LIM, RIEM, COORD, VISC, TY, ns_min_blocks<Real, VISC>(), Src>;
-  static int bps = 0;
-  if (bps == 0 || nsm < 0) {
-    cudaError_t e = prepare_kernel(kern, C::NT, C::BYTES, &bps);
+  static Residency<1> res;
+  if (nsm < 0 || !res.known()) {
+    const cudaError_t e = prepare_kernel(kern, C::NT, {C::BYTES}, res);
     if (e != cudaSuccess) return e;
   }
   if (nsm < 0) return cudaSuccess;
   if (ntiles <= 0) return cudaSuccess;
-  const int grid = (int)(ntiles < (long long)bps * nsm ? ntiles : (long long)bps * nsm);
+  const int grid = grid_blocks(ntiles, res[0], nsm);
   kern<<<grid, C::NT, C::BYTES, s>>>(src);
   return cudaGetLastError();
 }
@@ -153,21 +175,15 @@ cudaError_t launch_ns_strip_ty(const NsStripSource& src, int nbuf, cudaStream_t 
   constexpr int R = 2, NW = TY / R;
   using C = NsStripCfg<R, NW>;
   auto kern = ns_strip_kernel<LIM, RIEM, R, NW, TY == 8 ? 3 : 2, COORD, FLAT>;
-  static int bps[3] = {0, 0, 0};
-  if (bps[0] == 0 || nsm < 0) {
-    // occupancy with 0, 1 and 2 staged tiles; the attribute ends at the largest
-    // (bps[0] is set last: another thread takes it as the sign that all are there)
-    int b[3];
-    for (int nb = 0; nb < 3; ++nb) {
-      cudaError_t e = prepare_kernel(kern, C::NT, C::bytes(nb), &b[nb]);
-      if (e != cudaSuccess) return e;
-    }
-    bps[1] = b[1], bps[2] = b[2], bps[0] = b[0];
+  static Residency<3> res;  // with 0, 1 and 2 staged tiles
+  if (nsm < 0 || !res.known()) {
+    const cudaError_t e = prepare_kernel(kern, C::NT, {C::bytes(0), C::bytes(1), C::bytes(2)}, res);
+    if (e != cudaSuccess) return e;
   }
   if (nsm < 0) return cudaSuccess;
   const long long ntiles = tile_total(src.p);
   if (ntiles <= 0) return cudaSuccess;
-  const int grid = (int)(ntiles < (long long)bps[nbuf] * nsm ? ntiles : (long long)bps[nbuf] * nsm);
+  const int grid = grid_blocks(ntiles, res[nbuf], nsm);
   kern<<<grid, C::NT, C::bytes(nbuf), s>>>(src);
   return cudaGetLastError();
 }
@@ -224,17 +240,15 @@ cudaError_t launch_ns_strip_visc_ty(const NsStripSource& src, int nbuf, cudaStre
   constexpr int R = 1, NW = TY / R;
   using C = NsStripViscCfg<R, NW>;
   auto kern = ns_strip_visc_kernel<LIM, RIEM, R, NW, 2, COORD>;
-  static int bps[3] = {0, 0, 0};
-  if (bps[0] == 0 || nsm < 0) {
-    for (int nb = 0; nb < 3; ++nb) {
-      cudaError_t e = prepare_kernel(kern, C::NT, C::bytes(nb), &bps[nb]);
-      if (e != cudaSuccess) return e;
-    }
+  static Residency<3> res;  // with 0, 1 and 2 staged tiles
+  if (nsm < 0 || !res.known()) {
+    const cudaError_t e = prepare_kernel(kern, C::NT, {C::bytes(0), C::bytes(1), C::bytes(2)}, res);
+    if (e != cudaSuccess) return e;
   }
   if (nsm < 0) return cudaSuccess;
   const long long ntiles = tile_total(src.p);
   if (ntiles <= 0) return cudaSuccess;
-  const int grid = (int)(ntiles < (long long)bps[nbuf] * nsm ? ntiles : (long long)bps[nbuf] * nsm);
+  const int grid = grid_blocks(ntiles, res[nbuf], nsm);
   kern<<<grid, C::NT, C::bytes(nbuf), s>>>(src);
   return cudaGetLastError();
 }
@@ -276,13 +290,13 @@ template <typename Real, int LIM, int COORD, class Src, int TY = HEAT_TY>
 cudaError_t launch_heat_src(const Src& src, long long ntiles, cudaStream_t s, int nsm) {
   using C = HeatCfg<Real, LIM, TY>;
   auto kern = heat_stage_kernel<Real, LIM, COORD, TY, Src>;
-  static int bps = 0;
-  if (bps == 0 || nsm < 0) {
-    cudaError_t e = prepare_kernel(kern, C::NT, C::BYTES, &bps);
+  static Residency<1> res;
+  if (nsm < 0 || !res.known()) {
+    const cudaError_t e = prepare_kernel(kern, C::NT, {C::BYTES}, res);
     if (e != cudaSuccess) return e;
   }
   if (nsm < 0 || ntiles <= 0) return cudaSuccess;
-  const int grid = (int)(ntiles < (long long)bps * nsm ? ntiles : (long long)bps * nsm);
+  const int grid = grid_blocks(ntiles, res[0], nsm);
   kern<<<grid, C::NT, C::BYTES, s>>>(src);
   return cudaGetLastError();
 }
@@ -313,15 +327,15 @@ cudaError_t launch_heat_pc_ty(const CUtensorMap& map, const HeatParams<float>& p
   constexpr int VX = TY % 4 == 0 ? 4 : 2, NW = TY / VX;
   using C = HeatPcCfg<VX, NW>;
   auto kern = heat_pc_kernel<COORD, VX, NW>;
-  static int bps = 0;
-  if (bps == 0 || nsm < 0) {
-    cudaError_t e = prepare_kernel(kern, C::NT, C::BYTES, &bps);
+  static Residency<1> res;
+  if (nsm < 0 || !res.known()) {
+    const cudaError_t e = prepare_kernel(kern, C::NT, {C::BYTES}, res);
     if (e != cudaSuccess) return e;
   }
   if (nsm < 0) return cudaSuccess;
   const long long ntiles = tile_total(p);
   if (ntiles <= 0) return cudaSuccess;
-  const int grid = (int)(ntiles < (long long)bps * nsm ? ntiles : (long long)bps * nsm);
+  const int grid = grid_blocks(ntiles, res[0], nsm);
   kern<<<grid, C::NT, C::BYTES, s>>>(map, p);
   return cudaGetLastError();
 }
@@ -333,15 +347,13 @@ cudaError_t launch_heat_pc(int coord, const CUtensorMap& map, HeatParams<float> 
 template <int LIM, int RIEM, int HCOORD, int HR>
 cudaError_t launch_mixed_lrc(const MixedSource& src, long long ntiles, int nbuf, cudaStream_t s, int nsm) {
   auto kern = batch_mixed_kernel<LIM, RIEM, HCOORD, HR>;
-  static int bps[3] = {0, 0, 0};
-  if (bps[0] == 0 || nsm < 0) {
-    for (int nb = 0; nb < 3; ++nb) {
-      cudaError_t e = prepare_kernel(kern, MIX_NT, mixed_bytes(nb), &bps[nb]);
-      if (e != cudaSuccess) return e;
-    }
+  static Residency<3> res;  // with 0, 1 and 2 staged tiles
+  if (nsm < 0 || !res.known()) {
+    const cudaError_t e = prepare_kernel(kern, MIX_NT, {mixed_bytes(0), mixed_bytes(1), mixed_bytes(2)}, res);
+    if (e != cudaSuccess) return e;
   }
   if (nsm < 0 || ntiles <= 0) return cudaSuccess;
-  const int grid = (int)(ntiles < (long long)bps[nbuf] * nsm ? ntiles : (long long)bps[nbuf] * nsm);
+  const int grid = grid_blocks(ntiles, res[nbuf], nsm);
   kern<<<grid, MIX_NT, mixed_bytes(nbuf), s>>>(src);
   return cudaGetLastError();
 }
@@ -398,15 +410,15 @@ cudaError_t launch_maxwell_one(const CUtensorMap& map, MaxwellParams<Real> p, cu
   constexpr int TY = maxwell_tile_ty<Real>();
   using C = MaxwellCfg<Real, TY>;
   auto kern = maxwell_stage_kernel<Real, LIM, RIEM, COORD, TY, std::is_same<Real, double>::value ? 1 : 3>;
-  static int bps = 0;
-  if (bps == 0 || nsm < 0) {
-    cudaError_t e = prepare_kernel(kern, C::NT, C::BYTES, &bps);
+  static Residency<1> res;
+  if (nsm < 0 || !res.known()) {
+    const cudaError_t e = prepare_kernel(kern, C::NT, {C::BYTES}, res);
     if (e != cudaSuccess) return e;
   }
   if (nsm < 0) return cudaSuccess;
   set_tiles(p, TY);
   const long long ntiles = tile_total(p);
-  const int grid = (int)(ntiles < (long long)bps * nsm ? ntiles : (long long)bps * nsm);
+  const int grid = grid_blocks(ntiles, res[0], nsm);
   kern<<<grid, C::NT, C::BYTES, s>>>(map, p);
   return cudaGetLastError();
 }
@@ -448,17 +460,15 @@ cudaError_t launch_mx_strip_ty(const MxStripSource& src, int nbuf, cudaStream_t 
   constexpr int R = TY == 8 ? 2 : 4, NW = TY / R;
   using C = MxStripCfg<R, NW>;
   auto kern = mx_strip_kernel<LIM, COORD, R, NW, TY == 8 ? 3 : 2>;
-  static int bps[3] = {0, 0, 0};
-  if (bps[0] == 0 || nsm < 0) {
-    for (int nb = 0; nb < 3; ++nb) {
-      cudaError_t e = prepare_kernel(kern, C::NT, C::bytes(nb), &bps[nb]);
-      if (e != cudaSuccess) return e;
-    }
+  static Residency<3> res;  // with 0, 1 and 2 staged tiles
+  if (nsm < 0 || !res.known()) {
+    const cudaError_t e = prepare_kernel(kern, C::NT, {C::bytes(0), C::bytes(1), C::bytes(2)}, res);
+    if (e != cudaSuccess) return e;
   }
   if (nsm < 0) return cudaSuccess;
   const long long ntiles = tile_total(src.p);
   if (ntiles <= 0) return cudaSuccess;
-  const int grid = (int)(ntiles < (long long)bps[nbuf] * nsm ? ntiles : (long long)bps[nbuf] * nsm);
+  const int grid = grid_blocks(ntiles, res[nbuf], nsm);
   kern<<<grid, C::NT, C::bytes(nbuf), s>>>(src);
   return cudaGetLastError();
 }
