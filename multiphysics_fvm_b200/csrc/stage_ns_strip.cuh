@@ -37,6 +37,7 @@
 // with clamped wave speeds (s- = min(s_min, 0), s+ = max(s_max, 0)), which is
 // the same function.
 #pragma once
+#include <cfloat>
 #include "stage_ns.cuh"
 
 namespace fvm {
@@ -201,11 +202,13 @@ __device__ __forceinline__ void strip_flux2(const F2* qL, const F2* qR, float ga
 }
 
 // P = (gamma - 1)(E - |m|^2 / (2 rho)) of one ring cell (navier_stokes.py:94-100).
-// Cells outside the ghosted grid hold zeros; the clamp keeps their P, which a
-// ghost cell's discarded slope reads, finite.
+// Cells outside the ghosted grid hold zeros; the clamp of the reciprocal keeps
+// their P, which a ghost cell's discarded slope reads, finite (a clamp of the
+// density would change the pressure of thin states: in units with densities of
+// 1e-31 a clamp at 1e-30 was wrong by 3 %).
 __device__ __forceinline__ float strip_pressure(const float* u, int PL, float gm1) {
   const float rho = u[0], m1 = u[PL], m2 = u[2 * PL], m3 = u[3 * PL], E = u[4 * PL];
-  const float ke = fmaf(m1, m1, fmaf(m2, m2, m3 * m3)) * (0.5f * rcp_approx(fmaxf(rho, 1e-30f)));
+  const float ke = fmaf(m1, m1, fmaf(m2, m2, m3 * m3)) * (0.5f * fminf(rcp_approx(rho), FLT_MAX));
   return gm1 * (E - ke);
 }
 
