@@ -324,10 +324,11 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
             const int ty = w * R - 1 + t;
             const int j = jb - 1 + t;
             ldf1(fc, ty + 1, lane);
-            const float hy = j < 0 || j >= ny ? 0.f : HS;  // zero slope in a ghost cell
+            const bool yghost = j < 0 || j >= ny;  // zero slope in a ghost cell
+            const float hy = strip_factor<LIM>(yghost);
             float s[NF];
 #pragma unroll
-            for (int f = 0; f < NF; ++f) s[f] = strip_slope<LIM>(fb[f] - fa[f], fc[f] - fb[f]);
+            for (int f = 0; f < NF; ++f) s[f] = strip_slope<LIM>(fb[f] - fa[f], fc[f] - fb[f], yghost);
             if (t >= 1) {
               float qr[NF], F[5];
 #pragma unroll
@@ -363,10 +364,11 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
               ldf0(fm, lane - 1);
               ldf0(f0, lane);
               ldf0(fp, lane + 1);
-              const float hx = i >= nx ? 0.f : HS;
+              const bool xghost = i >= nx;
+              const float hx = strip_factor<LIM>(xghost);
 #pragma unroll
               for (int f = 0; f < NF; ++f) {
-                const float s1 = strip_slope<LIM>(f0[f] - fm[f], fp[f] - f0[f]);
+                const float s1 = strip_slope<LIM>(f0[f] - fm[f], fp[f] - f0[f], xghost);
                 const float su = __shfl_up_sync(0xffffffffu, s1, 1);
                 const float sl = lane == 0 ? hl[(par * NF + f) * TY + ty] : su;
                 qlx[f] = fmaf(HS, sl, fm[f]);
@@ -420,7 +422,7 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
 #pragma unroll
               for (int f = 0; f < NF; ++f) {
                 qlh[f] = fmaf(HS, strip_slope<LIM>(b[f] - a[f], c[f] - b[f]), b[f]);
-                qrh[f] = fmaf(g32 ? 0.f : -HS, strip_slope<LIM>(c[f] - b[f], d[f] - c[f]), c[f]);
+                qrh[f] = fmaf(-strip_factor<LIM>(g32), strip_slope<LIM>(c[f] - b[f], d[f] - c[f], g32), c[f]);
               }
               strip_flux_visc<0, RIEM>(qlh, qrh, gam, F);
             }
@@ -452,7 +454,8 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
       bool step_ok = got;
       if (is_out && got) {
         // ------------------------------------------------------------ 5 ----
-        const float hz = K + 1 <= 0 || K + 1 >= nz + 1 ? 0.f : HS;
+        const bool zghost = K + 1 <= 0 || K + 1 >= nz + 1;
+        const float hz = strip_factor<LIM>(zghost);
         const bool zslope = K >= Z0 - 2, zface = K >= Z0 - 1;
         const float idz = outstep ? __ldg(m.inv_dx3 + (K - 1)) : 0.f;
         if (zslope) {
@@ -478,7 +481,7 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
                 a1 = tK1[c * PL2 + op];
                 a2 = own[f - 5];
               }
-              const float s = strip_slope<LIM>(a1 - a0, a2 - a1);
+              const float s = strip_slope<LIM>(a1 - a0, a2 - a1, zghost);
               qr[f] = fmaf(-hz, s, a1);
               qn[f] = fmaf(hz, s, a1);
             }

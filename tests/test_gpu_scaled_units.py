@@ -3,7 +3,10 @@ changes only float32 exponents, so a float32 residual is that of the unit state
 times a power of two, up to the rounding of a different exponent's reciprocal
 and square root (relative L-inf <= 1e-6 allowed).
 
-* thin: densities of 2^-104 (5e-32) with velocities of 2^47, energies of 2^-10."""
+* thin: densities of 2^-104 (5e-32) with velocities of 2^47, energies of 2^-10;
+* strong: nearly uniform states of 2^36 (momentum) and 2^72 (energy), 2^72 for
+  fields: the differences between cells are in range, the product of a ghost
+  cell's two differences, whose slope is not used, is above float32's largest."""
 import numpy as np
 import pytest
 
@@ -34,8 +37,11 @@ def _ns(mu):
 @pytest.mark.parametrize("n", [(40, 20, 12), (70, 33, 1)], ids=str)
 @pytest.mark.parametrize("mu", [0.0, 2.0 ** -10], ids=["inviscid", "viscous"])
 @pytest.mark.parametrize("a,b,smooth,limiter,riemann",
-                         [(-104, 47, False, "minmod", "hll"), (-104, 47, False, "monotonized_central", "rusanov")],
-                         ids=["thin-minmod", "thin-mc"])
+                         [(-104, 47, False, "minmod", "hll"), (-104, 47, False, "monotonized_central", "rusanov"),
+                          (0, 36, True, "van_leer", "hll"), (0, 36, True, "van_leer", "rusanov"),
+                          (0, 36, True, "minmod", "hll"), (0, 36, True, "monotonized_central", "hll")],
+                         ids=["thin-minmod", "thin-mc", "strong-van_leer", "strong-van_leer-rusanov",
+                              "strong-minmod", "strong-mc"])
 def test_navier_stokes(a, b, smooth, limiter, riemann, mu, n):
     """Density times 2^a, velocity times 2^b."""
     U = random_ns_state(tuple(x + 2 for x in n), np.random.default_rng(5))
@@ -49,3 +55,14 @@ def test_navier_stokes(a, b, smooth, limiter, riemann, mu, n):
     assert np.all(np.isfinite(got))
     for q in range(5):
         assert rel_linf(got[q], ref[q]) <= 1e-6
+
+
+@pytest.mark.parametrize("limiter", ["van_leer", "minmod", "monotonized_central"])
+def test_maxwell(limiter):
+    n = (40, 20, 12)
+    prm = {"magnetic_permeability": 1.0, "electric_permittivity": 1.0, "electrical_conductivity": 0.0,
+           "charge_density": 0.0, "magnetic_cleaning_coeff": 0.001, "electric_cleaning_coeff": 0.001}
+    U = to_fp32(1 + 1e-4 * np.random.default_rng(5).uniform(-1, 1, (6,) + tuple(x + 2 for x in n)))
+    ref = _residual("maxwell", n, "cartesian", limiter, "rusanov", prm, U)
+    got = _residual("maxwell", n, "cartesian", limiter, "rusanov", prm, U * 2.0 ** 72) * 2.0 ** -72
+    assert np.all(np.isfinite(got)) and rel_linf(got, ref) <= 1e-6
