@@ -253,11 +253,11 @@ __global__ void __launch_bounds__(MxStripCfg<R, NW>::NT, MINB)
             const int ty = w * R - 1 + t;
             const int j = jb - 1 + t;
             ldf(fc, ty + 1, lane);
-            const bool yghost = j < 0 || j >= ny;  // zero slope in a ghost cell
-            const float hy = strip_factor<LIM>(yghost);
+            const float ygate = strip_gate<LIM>(j < 0 || j >= ny);  // zero slope in a ghost cell
+            const float hy = strip_factor<LIM>(ygate);
             float s[NV];
 #pragma unroll
-            for (int f = 0; f < NV; ++f) s[f] = strip_slope<LIM>(fb[f] - fa[f], fc[f] - fb[f], yghost);
+            for (int f = 0; f < NV; ++f) s[f] = strip_slope<LIM>(fb[f] - fa[f], fc[f] - fb[f], ygate);
             if (t >= 1) {
               float qr[NV], F[NV];
 #pragma unroll
@@ -279,11 +279,11 @@ __global__ void __launch_bounds__(MxStripCfg<R, NW>::NT, MINB)
               float fm[NV], fp[NV], qlx[NV], qrx[NV], F[NV];
               ldf(fm, ty, lane - 1);
               ldf(fp, ty, lane + 1);
-              const bool xghost = i >= nx;
-              const float hx = strip_factor<LIM>(xghost);
+              const float xgate = strip_gate<LIM>(i >= nx);
+              const float hx = strip_factor<LIM>(xgate);
 #pragma unroll
               for (int f = 0; f < NV; ++f) {
-                const float s1 = strip_slope<LIM>(fb[f] - fm[f], fp[f] - fb[f], xghost);
+                const float s1 = strip_slope<LIM>(fb[f] - fm[f], fp[f] - fb[f], xgate);
                 const float su = __shfl_up_sync(0xffffffffu, s1, 1);
                 const float sl = lane == 0 ? hl[(par * NV + f) * TY + ty] : su;
                 qlx[f] = fmaf(HS, sl, fm[f]);
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(MxStripCfg<R, NW>::NT, MINB)
               ldh(b, TX - 1);
               ldh(c, TX);
               ldh(d, TX + 1);
-              const bool g32 = x0 + TX >= nx;
+              const float g32 = strip_gate<LIM>(x0 + TX >= nx);
 #pragma unroll
               for (int f = 0; f < NV; ++f) {
                 qlh[f] = fmaf(HS, strip_slope<LIM>(b[f] - a[f], c[f] - b[f]), b[f]);
@@ -379,8 +379,8 @@ __global__ void __launch_bounds__(MxStripCfg<R, NW>::NT, MINB)
           }
         }
         // ------------------------------------------------------------ 5 ----
-        const bool zghost = K + 1 <= 0 || K + 1 >= nz + 1;
-        const float hz = strip_factor<LIM>(zghost);
+        const float zgate = strip_gate<LIM>(K + 1 <= 0 || K + 1 >= nz + 1);
+        const float hz = strip_factor<LIM>(zgate);
         const bool zface = K >= Z0 - 1;
         const float idz = outstep ? __ldg(m.inv_dx3 + (K - 1)) : 0.f;
 #pragma unroll
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(MxStripCfg<R, NW>::NT, MINB)
 #pragma unroll
           for (int f = 0; f < NV; ++f) {
             const float b0 = uK[f * PL + o], b1 = uK1[f * PL + o], b2 = uK2[f * PL + o];
-            const float s = strip_slope<LIM>(b1 - b0, b2 - b1, zghost);
+            const float s = strip_slope<LIM>(b1 - b0, b2 - b1, zgate);
             qr[f] = fmaf(-hz, s, b1);
             qn[f] = fmaf(hz, s, b1);
           }

@@ -90,13 +90,15 @@ __device__ __forceinline__ float min_xorsign(float a, float b) {
 // Limited slope from the backward and forward differences (float32; zero for
 // piecewise constant), up to the factor 2 strip_half<LIM>: a face state is
 // f +- strip_half * strip_slope, the reference's f +- slope / 2.  The factor
-// carries the constants of the limiters (slope_limiters.py:13-105).  A ghost
-// cell's slope is zero by its factor, one select per cell instead of one per
-// field; of van Leer by the condition on the product of its differences, which
-// may overflow in a ghost cell to an infinity that a zero factor would turn into
-// NaN.  The kernels are bound by issue and latency: with the limiters in
-// four to eleven instructions, a select per slope, flux vectors formed per state
-// and float64 stage constants converted per cell, the stage launches took 717 us
+// carries the constants of the limiters (slope_limiters.py:13-105).
+// A ghost cell's slope is zero by one value per cell, its gate, instead of a
+// select per field: the factor, zero in a ghost cell, or for van Leer the bound
+// that the product of the differences has to pass, infinite in a ghost cell,
+// where the product may overflow to an infinity that a zero factor would turn into
+// NaN (a predicate in place of that bound: 256^3 stage 651 us, so 610).
+// The kernels are bound by issue and latency: with the limiters in four to
+// eleven instructions, a select per slope, flux vectors formed per state and
+// float64 stage constants converted per cell, the stage launches took 717 us
 // (inviscid 256^3), 1497 (viscous 256^3), 95 (97x130x61, three-sign limiter) and
 // 291 (Maxwell 128x128x256); in this form 600, 1291, 54 and 200 (541, 1108, 48 and
 // 186 with what the comments at strip_slope2, the flat march, the viscous and the
@@ -105,13 +107,19 @@ template <int LIM>
 __host__ __device__ constexpr float strip_half() {
   return LIM == LIM_MC ? 0.25f : (LIM == LIM_VANLEER ? 1.f : 0.5f);
 }
-// The factor of a cell's slope.
+// A cell's gate, and the factor of its slope.
 template <int LIM>
-__device__ __forceinline__ float strip_factor(bool ghost) {
-  return ghost && LIM != LIM_VANLEER ? 0.f : strip_half<LIM>();
+__device__ __forceinline__ float strip_gate(bool ghost) {
+  if constexpr (LIM == LIM_VANLEER) return ghost ? __int_as_float(0x7f800000) : 0.f;
+  else return ghost ? 0.f : strip_half<LIM>();
 }
 template <int LIM>
-__device__ __forceinline__ float strip_slope(float a, float b, bool ghost = false) {
+__device__ __forceinline__ float strip_factor(float gate) {
+  if constexpr (LIM == LIM_VANLEER) return strip_half<LIM>();
+  else return gate;
+}
+template <int LIM>
+__device__ __forceinline__ float strip_slope(float a, float b, float gate = strip_gate<LIM>(false)) {
   if constexpr (LIM == LIM_PC) return 0.f;
   else if constexpr (LIM == LIM_MINMOD) return copysignf(fmaxf(min_xorsign(a, b), 0.f), a);
   else if constexpr (LIM == LIM_MC) {
@@ -122,7 +130,7 @@ __device__ __forceinline__ float strip_slope(float a, float b, bool ghost = fals
   } else {
     // a b / (a + b) where a b > 0; a + b = 0 only where a b <= 0
     const float ab = a * b;
-    return ab > 0.f && !ghost ? ab * rcp_approx(a + b) : 0.f;
+    return ab > gate ? ab * rcp_approx(a + b) : 0.f;
   }
 }
 
@@ -168,8 +176,8 @@ __device__ __forceinline__ void strip_flux(const float* qL, const float* qR, flo
 // once (837 -> 700 thread instructions per cell; 256^3 stage 575 -> 541 us,
 // 97x130x61 51.6 -> 48.4, one-plane 64x64 5.99 -> 5.0).
 template <int LIM>
-__device__ __forceinline__ F2 strip_slope2(F2 a, F2 b, bool ghost) {
-  return F2(strip_slope<LIM>(a.lo(), b.lo(), ghost), strip_slope<LIM>(a.hi(), b.hi(), ghost));
+__device__ __forceinline__ F2 strip_slope2(F2 a, F2 b, float gate) {
+  return F2(strip_slope<LIM>(a.lo(), b.lo(), gate), strip_slope<LIM>(a.hi(), b.hi(), gate));
 }
 template <int LIM>
 __device__ __forceinline__ F2 strip_state2(F2 h, F2 s, F2 q) {
@@ -342,7 +350,7 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
             ldh(b, TX - 1);
             ldh(c, TX);
             ldh(d, TX + 1);
-            const bool g32 = x0 + TX >= nx;  // x0 + 32 is the right ghost column
+            const float g32 = strip_gate<LIM>(x0 + TX >= nx);  // x0 + 32 is the right ghost column
 #pragma unroll
             for (int f = 0; f < NF; ++f) {
               ql[f] = fmaf(HS, strip_slope<LIM>(b[f] - a[f], c[f] - b[f]), b[f]);
@@ -462,12 +470,12 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
             // x1 of both rows (cells i, rows jb and jb + 1): the flux through
             // the cells' left faces, the right faces' from the next lane
             F2 qlx[NF], qrx[NF], F[5];
-            const bool xghost = i >= nx;  // i == nx: the right ghost column
-            const F2 hx(-strip_factor<LIM>(xghost));
+            const float xgate = strip_gate<LIM>(i >= nx);  // i == nx: the right ghost column
+            const F2 hx(-strip_factor<LIM>(xgate));
 #pragma unroll
             for (int f = 0; f < NF; ++f) {
               const F2 fm = ld2(f, ty, lane - 1), f0 = ld2(f, ty, lane), fp = ld2(f, ty, lane + 1);
-              const F2 s1 = strip_slope2<LIM>(f0 - fm, fp - f0, xghost);
+              const F2 s1 = strip_slope2<LIM>(f0 - fm, fp - f0, xgate);
               const float ua = __shfl_up_sync(0xffffffffu, s1.lo(), 1), ub = __shfl_up_sync(0xffffffffu, s1.hi(), 1);
               const float* h = hl + (par * NF + f) * TY + ty;
               qlx[f] = strip_state2<LIM>(F2(HS), lane == 0 ? F2(h[0], h[1]) : F2(ua, ub), fm);
@@ -488,12 +496,12 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
             // faces below rows jb and jb + 1 as a pair and the one above
             F2 ql[NF], qr[NF], F[5];
             float ql1[NF], qr1[NF], F1[5];
-            bool yghost[4];
+            float ygate[4];
             float hy[4];
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
-              yghost[r] = jb + r - 1 < 0 || jb + r - 1 >= ny;
-              hy[r] = strip_factor<LIM>(yghost[r]);
+              ygate[r] = strip_gate<LIM>(jb + r - 1 < 0 || jb + r - 1 >= ny);
+              hy[r] = strip_factor<LIM>(ygate[r]);
             }
 #pragma unroll
             for (int f = 0; f < NF; ++f) {
@@ -501,7 +509,7 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
 #pragma unroll
               for (int r = 0; r < 6; ++r) g[r] = ld(f, ty - 2 + r, lane);
 #pragma unroll
-              for (int r = 0; r < 4; ++r) s[r] = strip_slope<LIM>(g[r + 1] - g[r], g[r + 2] - g[r + 1], yghost[r]);
+              for (int r = 0; r < 4; ++r) s[r] = strip_slope<LIM>(g[r + 1] - g[r], g[r + 2] - g[r + 1], ygate[r]);
               ql[f] = strip_state2<LIM>(F2(hy[0], hy[1]), F2(s[0], s[1]), F2(g[1], g[2]));
               qr[f] = strip_state2<LIM>(F2(-hy[1], -hy[2]), F2(s[1], s[2]), F2(g[2], g[3]));
               ql1[f] = fmaf(hy[2], s[2], g[3]);
@@ -553,8 +561,8 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
           }
           // ------------------------------------------------------------ 5 ----
           // slope of plane K+1 (zero on a ghost plane) and the flux at K+1/2
-          const bool zghost = K + 1 <= 0 || K + 1 >= nz + 1;
-          const float hz = strip_factor<LIM>(zghost);
+          const float zgate = strip_gate<LIM>(K + 1 <= 0 || K + 1 >= nz + 1);
+          const float hz = strip_factor<LIM>(zgate);
           const bool zface = K >= Z0 - 1;
           const float idz = outstep ? __ldg(p.met.inv_dx3 + (K - 1)) : 0.f;
           F2 qr[NF], qn[NF];
@@ -565,7 +573,7 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
             const int up = f < 5 ? W : W2;  // one row up
             const F2 a0(b0[0], b0[up]), a1(b1[0], b1[up]);
             const F2 a2 = f < 5 ? F2(uK2[f * PL + o], uK2[f * PL + o + W]) : pnew;
-            const F2 s = strip_slope2<LIM>(a1 - a0, a2 - a1, zghost);
+            const F2 s = strip_slope2<LIM>(a1 - a0, a2 - a1, zgate);
             qr[f] = strip_state2<LIM>(F2(-hz), s, a1);
             qn[f] = strip_state2<LIM>(F2(hz), s, a1);
           }

@@ -324,11 +324,11 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
             const int ty = w * R - 1 + t;
             const int j = jb - 1 + t;
             ldf1(fc, ty + 1, lane);
-            const bool yghost = j < 0 || j >= ny;  // zero slope in a ghost cell
-            const float hy = strip_factor<LIM>(yghost);
+            const float ygate = strip_gate<LIM>(j < 0 || j >= ny);  // zero slope in a ghost cell
+            const float hy = strip_factor<LIM>(ygate);
             float s[NF];
 #pragma unroll
-            for (int f = 0; f < NF; ++f) s[f] = strip_slope<LIM>(fb[f] - fa[f], fc[f] - fb[f], yghost);
+            for (int f = 0; f < NF; ++f) s[f] = strip_slope<LIM>(fb[f] - fa[f], fc[f] - fb[f], ygate);
             if (t >= 1) {
               float qr[NF], F[5];
 #pragma unroll
@@ -364,11 +364,11 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
               ldf0(fm, lane - 1);
               ldf0(f0, lane);
               ldf0(fp, lane + 1);
-              const bool xghost = i >= nx;
-              const float hx = strip_factor<LIM>(xghost);
+              const float xgate = strip_gate<LIM>(i >= nx);
+              const float hx = strip_factor<LIM>(xgate);
 #pragma unroll
               for (int f = 0; f < NF; ++f) {
-                const float s1 = strip_slope<LIM>(f0[f] - fm[f], fp[f] - f0[f], xghost);
+                const float s1 = strip_slope<LIM>(f0[f] - fm[f], fp[f] - f0[f], xgate);
                 const float su = __shfl_up_sync(0xffffffffu, s1, 1);
                 const float sl = lane == 0 ? hl[(par * NF + f) * TY + ty] : su;
                 qlx[f] = fmaf(HS, sl, fm[f]);
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
               ldh(b, TX - 1);
               ldh(c, TX);
               ldh(d, TX + 1);
-              const bool g32 = x0 + TX >= nx;
+              const float g32 = strip_gate<LIM>(x0 + TX >= nx);
 #pragma unroll
               for (int f = 0; f < NF; ++f) {
                 qlh[f] = fmaf(HS, strip_slope<LIM>(b[f] - a[f], c[f] - b[f]), b[f]);
@@ -454,8 +454,8 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
       bool step_ok = got;
       if (is_out && got) {
         // ------------------------------------------------------------ 5 ----
-        const bool zghost = K + 1 <= 0 || K + 1 >= nz + 1;
-        const float hz = strip_factor<LIM>(zghost);
+        const float zgate = strip_gate<LIM>(K + 1 <= 0 || K + 1 >= nz + 1);
+        const float hz = strip_factor<LIM>(zgate);
         const bool zslope = K >= Z0 - 2, zface = K >= Z0 - 1;
         const float idz = outstep ? __ldg(m.inv_dx3 + (K - 1)) : 0.f;
         if (zslope) {
@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
                 a1 = tK1[c * PL2 + op];
                 a2 = own[f - 5];
               }
-              const float s = strip_slope<LIM>(a1 - a0, a2 - a1, zghost);
+              const float s = strip_slope<LIM>(a1 - a0, a2 - a1, zgate);
               qr[f] = fmaf(-hz, s, a1);
               qn[f] = fmaf(hz, s, a1);
             }
