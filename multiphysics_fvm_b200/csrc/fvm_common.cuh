@@ -167,31 +167,51 @@ __device__ __forceinline__ float sqrt_approx(float x) {
   return y;
 }
 
+// 1 / x of a metric factor: the approximate reciprocal and one Newton step, which
+// leaves little more than the rounding of the result, at two operations (a
+// correctly rounded division per column made a heat stage of short pieces 2 to 5 %
+// longer).
+__device__ __forceinline__ float rcp_newton(float x) {
+  const float r = rcp_approx(x);
+  return fmaf(fmaf(-x, r, 1.f), r, r);
+}
+
 // float32 metric factors of a cell for the register-blocked kernels, as
 // products of one per-column value c1 and table entries: the divergence takes
 // face areas over the cell volume, S_a / V (the x3 length cancels in S1 / V and
 // S2 / V), and the curvilinear terms the three non-zero d_a ln h_b / h_a of the
 // supported coordinates, la = dl01/h0, lb = dl02/h0, lc = dl12/h1.
+//
+// The x1 faces come as half sum and half difference of S1 / V,
+//   S1+ F+ - S1- F- = V (s1 (F+ - F-) + d1 (F+ + F-)):
+// with the two quotients themselves the pressure, the largest term of both
+// fluxes, left a residue of their rounding, an acceleration of the column that
+// stays from step to step (cylindrical 96x128x64, error after ten steps 5.55e-8,
+// so 3.94e-8).
 template <int COORD>
 struct ColMetric {
   float a1p, a1m;  // S1 / V of the upper and lower x1 face
+  float s1, d1;    // half their sum and half their difference
   float c1;        // cylindrical dx1 / a1, spherical a1 / b1
   float ir;        // 1 / r
   __device__ __forceinline__ void load(const Metric<float>& m, int i) {
     if constexpr (COORD == COORD_CART) {
-      a1p = a1m = __ldg(m.inv_dx1 + i);
-      c1 = ir = 0.f;
+      a1p = a1m = s1 = __ldg(m.inv_dx1 + i);
+      d1 = c1 = ir = 0.f;
     } else if constexpr (COORD == COORD_CYL) {
-      const float ia = rcp_approx(__ldg(m.a1 + i));
+      const float ia = rcp_newton(__ldg(m.a1 + i));
       a1p = __ldg(m.r_f + i + 1) * ia;
       a1m = __ldg(m.r_f + i) * ia;
       c1 = __ldg(m.dx1 + i) * ia;
+      s1 = __ldg(m.inv_dx1 + i);
+      d1 = 0.5f * c1;
       ir = __ldg(m.inv_r + i);
     } else {
-      const float ib = rcp_approx(__ldg(m.b1 + i));
-      a1p = __ldg(m.r_f2 + i + 1) * ib;
-      a1m = __ldg(m.r_f2 + i) * ib;
-      c1 = __ldg(m.a1 + i) * ib;
+      const float ib = rcp_newton(__ldg(m.b1 + i)), rp = __ldg(m.r_f2 + i + 1), rm = __ldg(m.r_f2 + i);
+      a1p = rp * ib;
+      a1m = rm * ib;
+      d1 = c1 = __ldg(m.a1 + i) * ib;
+      s1 = 0.5f * (rp + rm) * ib;
       ir = __ldg(m.inv_r + i);
     }
   }

@@ -94,6 +94,7 @@ __device__ __forceinline__ bool heat_pc_tile(const HeatParams<float>& p, const C
   const int jc = min(j, ny - 1);
   auto gx = [&](int i) { return i >= 0 && i < nx ? gk * __ldg(m.inv_dx1 + i) : 0.f; };
   auto gy = [&](int jj) { return jj >= 0 && jj < ny ? gk * __ldg(m.inv_dx2 + jj) : 0.f; };
+  const float ic2 = COORD == COORD_SPH ? rcp_newton(__ldg(m.c2 + jc)) : 1.f;
   float cxm[VX], cx0[VX], cxp[VX], cy[VX], cz[VX];
 #pragma unroll
   for (int c = 0; c < VX; ++c) {
@@ -103,16 +104,15 @@ __device__ __forceinline__ bool heat_pc_tile(const HeatParams<float>& p, const C
     const float c1 = COORD == COORD_CART ? 1.f : cm.c1;
     cxp[c] = 0.5f * cm.a1p * gx(i0 + c + 1);
     cxm[c] = -0.5f * cm.a1m * gx(i0 + c - 1);
-    cx0[c] = 0.5f * (cm.a1p - cm.a1m) * gx(ic);
+    cx0[c] = cm.d1 * gx(ic);
     cy[c] = 0.5f * c1 * (COORD == COORD_CART ? 1.f : cm.ir);
     cz[c] = 0.5f * gk;
     if constexpr (COORD == COORD_SPH)
-      cz[c] *= (c1 * __ldg(m.dx2 + jc)) * rcp_approx(__ldg(m.c2 + jc)) * (cm.ir * __ldg(m.inv_sin_c2 + jc));
+      cz[c] *= (c1 * __ldg(m.dx2 + jc)) * ic2 * (cm.ir * __ldg(m.inv_sin_c2 + jc));
   }
   // S2 / V without its column factor, at the upper and lower x2 face
   float pu, pl_;
   if constexpr (COORD == COORD_SPH) {
-    const float ic2 = rcp_approx(__ldg(m.c2 + jc));
     pu = __ldg(m.sin_f2 + jc + 1) * ic2;
     pl_ = __ldg(m.sin_f2 + jc) * ic2;
   } else {

@@ -503,8 +503,8 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
               const float da = __shfl_down_sync(0xffffffffu, F[v].lo(), 1), db = __shfl_down_sync(0xffffffffu, F[v].hi(), 1);
               const float* e = fr + (par * 5 + v) * TY + ty;
               const F2 fe = lane == 31 ? F2(e[0], e[1]) : F2(da, db);
-              if constexpr (COORD == COORD_CART) kv[v] = (fe - F[v]) * F2(cm.a1p);
-              else kv[v] = fma2(fe, F2(cm.a1p), F[v] * F2(-cm.a1m));
+              kv[v] = (fe - F[v]) * F2(cm.s1);
+              if constexpr (COORD != COORD_CART) kv[v] = fma2(fe + F[v], F2(cm.d1), kv[v]);
             }
           }
           {

@@ -379,8 +379,8 @@ __global__ void __launch_bounds__(NsStripViscCfg<R, NW>::NT, MINB)
               for (int v = 0; v < 5; ++v) {
                 const float fd = __shfl_down_sync(0xffffffffu, F[v], 1);
                 const float fe = lane == 31 ? fr[(par * 5 + v) * TY + ty] : fd;
-                if constexpr (COORD == COORD_CART) kv[r][v] = fmaf(fe - F[v], cm.a1p, kv[r][v]);
-                else kv[r][v] = fmaf(fe, cm.a1p, fmaf(-F[v], cm.a1m, kv[r][v]));
+                kv[r][v] = fmaf(fe - F[v], cm.s1, kv[r][v]);
+                if constexpr (COORD != COORD_CART) kv[r][v] = fmaf(fe + F[v], cm.d1, kv[r][v]);
               }
             }
 #pragma unroll

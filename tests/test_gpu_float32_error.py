@@ -47,3 +47,14 @@ def error(coords, n, lo, hi, mu, limiter, steps, dt):
 
 def test_cartesian():
     assert error("cartesian", (64, 64, 64), (0, 0, 0), (1, 1, 1), 0.0, "minmod", 5, 2.0 ** -10) <= 3.8525e-8
+
+
+ANNULUS = ((96, 128, 8), (0.5, 0, 0), (1.5, 2 * np.pi, 0.125))
+SHELL = ((96, 64, 16), (0.5, 0.25 * np.pi, 0), (1.5, 0.75 * np.pi, 0.4))
+
+
+@pytest.mark.parametrize("coords,grid,mu,before",
+                         [("cylindrical", ANNULUS, 0.0, 5.0740e-8), ("cylindrical", ANNULUS, 1e-4, 5.1096e-8),
+                          ("spherical", SHELL, 0.0, 5.1520e-8), ("spherical", SHELL, 1e-4, 5.1562e-8)])
+def test_curvilinear(coords, grid, mu, before):
+    assert error(coords, *grid, mu, "van_leer", 10, 2.0 ** -10) <= before
