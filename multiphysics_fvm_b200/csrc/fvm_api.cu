@@ -817,6 +817,16 @@ static int transpose(fvm_handle* h, bool to_device, int buf, bool interior, doub
 
 namespace {
 
+// The kind of a caller's memory (cudaMemoryTypeHost: page-locked).
+cudaMemoryType memory_kind(const void* p) {
+  cudaPointerAttributes a;
+  const bool known = cudaPointerGetAttributes(&a, p) == cudaSuccess;
+  cudaGetLastError();
+  return known ? a.type : cudaMemoryTypeUnregistered;
+}
+// A caller's page-locked array is copied from or into directly.
+bool page_locked(const void* p) { return memory_kind(p) == cudaMemoryTypeHost; }
+
 // Copy between the device staging array and `n` host arrays of `per` bytes each
 // (pageable memory), on the handle's stream, finished on return.  The driver's
 // own pageable copy stages through pinned memory with one thread: 5 GB/s at 2.6
@@ -828,6 +838,9 @@ namespace {
 // 2.0, down 2.3 -> 1.2; a host dict of 2 MB up 0.28 -> 0.19, down 0.59 -> 0.21
 // (stacking and slicing copies included).
 int host_copy(fvm_handle* h, bool to_device, double* const* host, int n, size_t per) {
+  for (int q = 0; q < n; ++q)  // the copying threads would fault on one
+    if (memory_kind(host[q]) == cudaMemoryTypeDevice)
+      return fail(FVM_E_INVALID, "a device pointer in place of a host array");
   const size_t total = per * n, chunk = h->xf_chunk;
   const long long nchunk = (long long)((total + chunk - 1) / chunk);
   const int want = (int)std::min<size_t>(h->xf_threads, total / (to_device ? XF_PER_UP : XF_PER_DOWN)), ring = 2 * h->xf_threads;
@@ -913,14 +926,6 @@ int host_copy(fvm_handle* h, bool to_device, double* const* host, int n, size_t 
   FVM_CK(e);
   FVM_CK(cudaStreamSynchronize(h->stream));
   return FVM_OK;
-}
-
-// A caller's page-locked array is copied from or into directly.
-bool page_locked(const void* p) {
-  cudaPointerAttributes a;
-  const bool ok = cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type == cudaMemoryTypeHost;
-  cudaGetLastError();
-  return ok;
 }
 
 // Ghosted state in the device staging array: faces from the boundary
