@@ -824,13 +824,11 @@ cudaMemoryType memory_kind(const void* p) {
   cudaGetLastError();
   return known ? a.type : cudaMemoryTypeUnregistered;
 }
-// A caller's page-locked array is copied from or into directly.
-bool page_locked(const void* p) { return memory_kind(p) == cudaMemoryTypeHost; }
-
-// Copy between the device staging array and `n` host arrays of `per` bytes each
-// (pageable memory), on the handle's stream, finished on return.  The driver's
-// own pageable copy stages through pinned memory with one thread: 5 GB/s at 2.6
-// MB, 17 at 37 MB, 13 at 170 MB of the link's 55.  Here the bytes go through the
+// Copy between the device staging array and `n` host arrays of `per` bytes each,
+// on the handle's stream, finished on return (an upload from page-locked arrays
+// with the stream's next synchronisation).  The driver's copy of pageable memory
+// stages through pinned memory with one thread: 5 GB/s at 2.6 MB, 17 at 37 MB, 13
+// at 170 MB of the link's 55.  Here such bytes go through the
 // handle's ring of pinned buffers: this thread issues the DMA copies in order,
 // up to XF_THREADS others (for this call only; they make no CUDA calls, whose
 // first use in a new thread costs more than a chunk) copy between the ring and
@@ -838,9 +836,22 @@ bool page_locked(const void* p) { return memory_kind(p) == cudaMemoryTypeHost; }
 // 2.0, down 2.3 -> 1.2; a host dict of 2 MB up 0.28 -> 0.19, down 0.59 -> 0.21
 // (stacking and slicing copies included).
 int host_copy(fvm_handle* h, bool to_device, double* const* host, int n, size_t per) {
-  for (int q = 0; q < n; ++q)  // the copying threads would fault on one
-    if (memory_kind(host[q]) == cudaMemoryTypeDevice)
+  bool locked = true;
+  for (int q = 0; q < n; ++q) {
+    const cudaMemoryType kind = memory_kind(host[q]);
+    if (kind == cudaMemoryTypeDevice)  // the copying threads would fault on one
       return fail(FVM_E_INVALID, "a device pointer in place of a host array");
+    locked = locked && kind == cudaMemoryTypeHost;
+  }
+  if (locked) {  // copied from or into directly
+    for (int q = 0; q < n; ++q) {
+      unsigned char* dev = reinterpret_cast<unsigned char*>(h->stage_dev) + q * per;
+      FVM_CK(to_device ? cudaMemcpyAsync(dev, host[q], per, cudaMemcpyHostToDevice, h->stream)
+                       : cudaMemcpyAsync(host[q], dev, per, cudaMemcpyDeviceToHost, h->stream));
+    }
+    if (!to_device) FVM_CK(cudaStreamSynchronize(h->stream));
+    return FVM_OK;
+  }
   const size_t total = per * n, chunk = h->xf_chunk;
   const long long nchunk = (long long)((total + chunk - 1) / chunk);
   const int want = (int)std::min<size_t>(h->xf_threads, total / (to_device ? XF_PER_UP : XF_PER_DOWN)), ring = 2 * h->xf_threads;
@@ -968,14 +979,8 @@ int fvm_download_vars(fvm_handle* h, double* const* host_vars) {
 
 int fvm_upload(fvm_handle* h, const double* host_state) {
   if (!h || !host_state) return fail(FVM_E_INVALID, "null argument");
-  const size_t bytes = h->stage_elems * sizeof(double);
-  int rc = FVM_OK;
-  if (page_locked(host_state)) {
-    FVM_CK(cudaMemcpyAsync(h->stage_dev, host_state, bytes, cudaMemcpyHostToDevice, h->stream));
-  } else {
-    double* p = const_cast<double*>(host_state);
-    rc = host_copy(h, true, &p, 1, bytes);
-  }
+  double* p = const_cast<double*>(host_state);
+  int rc = host_copy(h, true, &p, 1, h->stage_elems * sizeof(double));
   if (!rc) rc = transpose(h, true, 0, false);
   if (rc) return rc;
   FVM_CK(cudaStreamSynchronize(h->stream));
@@ -985,11 +990,7 @@ int fvm_upload(fvm_handle* h, const double* host_state) {
 int fvm_download(fvm_handle* h, double* host_state) {
   if (!h || !host_state) return fail(FVM_E_INVALID, "null argument");
   if (int rc = stage_ghosted(h, h->stage_dev)) return rc;
-  const size_t bytes = h->stage_elems * sizeof(double);
-  if (!page_locked(host_state)) return host_copy(h, false, &host_state, 1, bytes);
-  FVM_CK(cudaMemcpyAsync(host_state, h->stage_dev, bytes, cudaMemcpyDeviceToHost, h->stream));
-  FVM_CK(cudaStreamSynchronize(h->stream));
-  return FVM_OK;
+  return host_copy(h, false, &host_state, 1, h->stage_elems * sizeof(double));
 }
 
 namespace {

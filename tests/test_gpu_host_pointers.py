@@ -1,6 +1,9 @@
 """Which memory the host transfers take: a device pointer in place of a host
 array is refused with an error (in a child process, which an access to it from
-the host would end)."""
+the host would end), page-locked results are written by one copy, without the
+staging ring."""
+import ctypes as C
+import json
 import os
 import subprocess
 import sys
@@ -53,3 +56,23 @@ print("refused")
 def test_device_pointers_are_refused():
     r = subprocess.run([sys.executable, "-c", DEVICE_POINTER], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "refused" in r.stdout, (r.returncode, r.stderr[-2000:])
+
+
+@pytest.mark.parametrize("call", ["upload", "download", "residual"])
+def test_page_locked_arrays_are_copied_directly(tmp_path, call):
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    from multiphysics_fvm_b200 import _lib as L
+    sim, lib = make_sim(), L.load()
+    want = sim.residual() if call == "residual" else sim.download()
+    pinned = torch.empty(want.shape, dtype=torch.float64, pin_memory=True)
+    if call == "upload":
+        pinned.numpy()[...] = want
+    ptr = C.cast(pinned.data_ptr(), C.POINTER(C.c_double))
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
+        L.check(getattr(lib, "fvm_" + call)(sim._h, ptr), call)
+    p.export_chrome_trace(str(tmp_path / "trace.json"))
+    copies = [e["name"] for e in json.load(open(tmp_path / "trace.json"))["traceEvents"]
+              if e.get("cat") == "gpu_memcpy" and ("HtoD" in e["name"] or "DtoH" in e["name"])]
+    assert len(copies) == 1
+    assert np.array_equal(sim.download() if call == "upload" else pinned.numpy(), want)
