@@ -194,8 +194,8 @@ int fvm_profile_steps(fvm_handle* h, int n_steps, int dt_mode, double* stage_ker
  * the reference has no tuning. */
 int fvm_autotune(fvm_handle* h, int* best_zchunk, double* best_ms_per_step);
 /* The handle's block shape: tile rows (fvm_desc.tile_ty, or the autotuner's
- * choice) and z-march depth (of the balanced split, the longest run of planes
- * that a block marches).  New: the reference has no tuning. */
+ * choice) and z-march depth (of the balanced split, the depth to ask for that comes
+ * nearest to it).  New: the reference has no tuning. */
 int fvm_tiling(fvm_handle* h, int* tile_ty, int* zchunk);
 
 /* Sharp Kelvin-Helmholtz initial state written on the device (the host

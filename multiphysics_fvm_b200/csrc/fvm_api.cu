@@ -143,6 +143,7 @@ struct fvm_handle {
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   double max_inv_l2 = 0.0, const_rate = 0.0;
   int zchunk = 0;   // z-march depth, 0: balanced pieces (tile_walk.cuh)
+  int fixed_depth = 0;  // the autotuner's best depth > 0 for tile_ty (reported_depth)
   int tile_ty = 0;  // tile rows of the stage kernel (its tensor maps are built for it)
   long long device_bytes = 0;
   fvm_closure* closure = nullptr;  // learned flux correction run inside every step
@@ -1821,15 +1822,28 @@ std::vector<int> zchunk_candidates(int nz) {
   return c;
 }
 
-// The z-march depth a handle reports: its fixed one, or the longest run of
-// planes that the balanced split gives a block.
+// The z-march depth a handle reports: its fixed one or, of the balanced split, the
+// fixed depth nearest to it in time, so that a caller who keeps the figure and asks
+// for it later gets about the same steps.  That is the autotuner's best or, where it
+// has not run, the depth of the fewest plane steps per block: rounds of pieces times
+// the depth and its warm-up planes.  (The longest run of the balanced split, asked
+// for as a depth, ran up to 1.29 times its time: 128^3, 19 planes, a second round
+// for 4 of 448 pieces.)
 int reported_depth(fvm_handle* h, int* depth) {
-  *depth = h->zchunk;
-  if (h->zchunk > 0) return FVM_OK;
+  *depth = h->zchunk > 0 ? h->zchunk : h->fixed_depth;
+  if (*depth > 0) return FVM_OK;
   FVM_CK(prepare_stage(h));
-  const long long units = (long long)((h->lay.nx + 31) / 32) * ((h->lay.ny + h->tile_ty - 1) / h->tile_ty) * h->lay.nz;
-  const long long blocks = std::max(1LL, std::min(units, (long long)prepared_blocks * h->nsm));
-  *depth = (int)std::min<long long>(h->d.nx3, (units + blocks - 1) / blocks);
+  const long long ncol = (long long)((h->lay.nx + 31) / 32) * ((h->lay.ny + h->tile_ty - 1) / h->tile_ty);
+  const long long blocks = std::max(1LL, (long long)prepared_blocks * h->nsm);
+  const int nz = h->d.nx3, warm = tile_halo(h->d);
+  long long least = 0;
+  for (int z = nz; z >= 1; --z) {
+    const long long pieces = ncol * ((nz + z - 1) / z), steps = (pieces + blocks - 1) / blocks * (z + warm);
+    if (z == nz || steps < least) {
+      least = steps;
+      *depth = z;
+    }
+  }
   return FVM_OK;
 }
 
@@ -1872,7 +1886,7 @@ int fvm_autotune(fvm_handle* h, int* best_zchunk, double* best_ms) {
   Saved sv;
   int rc = save_states({h}, sv);
   if (rc) return rc;
-  int best = h->zchunk, best_ty = h->tile_ty;
+  int best = h->zchunk, best_ty = h->tile_ty, best_fixed = 0;
   double bt = 1e30;
   // (a batch member keeps the shape of its batch's kernels, which read its
   // tensor maps: a map of another shape copies more than a kernel's ring slot holds)
@@ -1881,6 +1895,8 @@ int fvm_autotune(fvm_handle* h, int* best_zchunk, double* best_ms) {
   for (int ty : tys) {
     h->tile_ty = ty;
     if ((rc = make_tmaps(h))) break;
+    int fixed = 0;  // this shape's best depth > 0
+    double ft = 1e30;
     for (int z : zchunk_candidates(h->d.nx3)) {
       h->zchunk = z;
       for (auto& g : h->graph)
@@ -1889,13 +1905,16 @@ int fvm_autotune(fvm_handle* h, int* best_zchunk, double* best_ms) {
       if ((rc = fvm_time_steps(h, 1, 0, &ms))) break;  // warm-up (builds the graph)
       if ((rc = fvm_time_steps(h, 3, 0, &ms))) break;
       if (ms < bt) { bt = ms; best = z; best_ty = ty; }
+      if (z > 0 && ms < ft) { ft = ms; fixed = z; }
       if ((rc = restore_states({h}, sv, false))) break;
     }
     if (rc) break;
+    if (best_ty == ty) best_fixed = fixed;
   }
   const int rr = restore_states({h}, sv, true);
   h->zchunk = best;
   h->tile_ty = best_ty;
+  h->fixed_depth = best_fixed;
   const int rt = make_tmaps(h);
   for (auto& g : h->graph)
     if (g) { cudaGraphExecDestroy(g); g = nullptr; }
@@ -1920,8 +1939,8 @@ int fvm_batch_autotune(fvm_batch* b, int* best_zchunk, double* best_ms) {
   Saved sv;
   int rc = save_states(b->h, sv);
   if (rc) return rc;
-  int best = b->h[0]->zchunk;
-  double bt = 1e30;
+  int best = b->h[0]->zchunk, fixed = nzmax;  // the best depth, the best depth > 0
+  double bt = 1e30, ft = 1e30;
   // heat tile rows of the mixed group (the other bodies have one shape)
   fvm_batch::Group* mg = nullptr;
   for (auto& g : b->groups)
@@ -1957,6 +1976,7 @@ int fvm_batch_autotune(fvm_batch* b, int* best_zchunk, double* best_ms) {
       if ((rc = fvm_batch_time_steps(b, 1, 0, &ms))) break;
       if ((rc = fvm_batch_time_steps(b, 3, 0, &ms))) break;
       if (ms < bt) { bt = ms; best = z; best_hty = hty; }
+      if (z > 0 && ms < ft) { ft = ms; fixed = z; }
       if ((rc = restore_states(b->h, sv, false))) break;
     }
     if (rc) break;
@@ -1966,7 +1986,7 @@ int fvm_batch_autotune(fvm_batch* b, int* best_zchunk, double* best_ms) {
   if (rc) return rc;
   if (rr) return rr;
   if (ra) return ra;
-  if (best_zchunk) *best_zchunk = best ? best : nzmax;
+  if (best_zchunk) *best_zchunk = best ? best : fixed;
   if (best_ms) *best_ms = bt / 3.0;
   return FVM_OK;
 }
