@@ -282,7 +282,7 @@ int default_tile_ty(const fvm_desc& d) {
   if (strip_desc(d)) return visc ? NS_STRIP_VISC_TY : NS_STRIP_TY;
   if (heat_pc_desc(d)) return HEAT_PC_TY;
   if (d.physics == FVM_HEAT) return HEAT_TY;
-  if (d.physics == FVM_MAXWELL) return f64 ? maxwell_tile_ty<double>() : MX_STRIP_TY;
+  if (d.physics == FVM_MAXWELL) return f64 ? MAXWELL_TY : MX_STRIP_TY;
   return visc ? ns_tile_ty<double, true>() : ns_tile_ty<double, false>();
 }
 int alt_tile_ty(const fvm_desc& d) {

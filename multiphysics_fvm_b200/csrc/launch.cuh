@@ -401,15 +401,15 @@ extern template cudaError_t launch_heat_batch<double>(int, int, const BatchSourc
                                                       cudaStream_t, int);
 
 // ------------------------------------------------------------- maxwell ----
-// Maxwell: 6 rows x 32 columns, 2 blocks of 256 threads per SM (float32).
-template <typename Real>
-constexpr int maxwell_tile_ty() { return std::is_same<Real, double>::value ? 8 : 6; }
+// Float64 Maxwell: 8 rows x 32 columns, one block per SM.
+constexpr int MAXWELL_TY = 8;
 
 template <typename Real, int LIM, int RIEM, int COORD>
 cudaError_t launch_maxwell_one(const CUtensorMap& map, MaxwellParams<Real> p, cudaStream_t s, int nsm) {
-  constexpr int TY = maxwell_tile_ty<Real>();
+  static_assert(std::is_same<Real, double>::value, "float32 grids run stage_maxwell_strip.cuh");
+  constexpr int TY = MAXWELL_TY;
   using C = MaxwellCfg<Real, TY>;
-  auto kern = maxwell_stage_kernel<Real, LIM, RIEM, COORD, TY, std::is_same<Real, double>::value ? 1 : 3>;
+  auto kern = maxwell_stage_kernel<Real, LIM, RIEM, COORD, TY>;
   static Residency<1> res;
   if (nsm < 0 || !res.known()) {
     const cudaError_t e = prepare_kernel(kern, C::NT, {C::BYTES}, res);

@@ -1,4 +1,5 @@
-// Fused Maxwell stage kernel: residual (maxwell.py:603-729) + Runge-Kutta stage.
+// Fused Maxwell stage kernel, float64 (float32: stage_maxwell_strip.cuh):
+// residual (maxwell.py:603-729) + Runge-Kutta stage.
 //
 // Conserved B (3) and D (3); face fluxes are the antisymmetric curl tensors of
 // H = B/mu and E = D/eps (maxwell.py:145-181) evaluated on reconstructed face
@@ -52,13 +53,7 @@ struct MaxwellCfg {
   static constexpr int OFF_FL = OFF_R + 3 * 2 * PL;
   static constexpr int OFF_FR = OFF_FL + NV * XB;
   static constexpr int OFF_FB = OFF_FR + NV * XB;
-  // U0 and acc of the plane's output cells copied in by cp.async at the start
-  // of each step ([U0 | acc][variable][output thread]).  Off: with the extra
-  // 9 KB per block the three float32 blocks per SM leave too little L1 for
-  // the metric tables, and the step was slower (2.48 -> 2.53 ms on C2a).
-  static constexpr bool STAGED = false;
-  static constexpr int OFF_G = OFF_FB + NV * FB;
-  static constexpr int END = OFF_G + (STAGED ? 2 * NV * TX * TY : 0);
+  static constexpr int END = OFF_FB + NV * FB;
   static constexpr int BYTES = round_up(END * (int)sizeof(Real), 16) + NSLOT * 8;
   static constexpr unsigned TX_BYTES = NV * PL * sizeof(Real);
 };
@@ -100,8 +95,8 @@ __device__ __forceinline__ void maxwell_flux(const R* qL, const R* qR, const Quo
   }
 }
 
-template <typename Real, int LIM, int RIEM, int COORD, int TY, int MINB>
-__global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, MINB)
+template <typename Real, int LIM, int RIEM, int COORD, int TY>
+__global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, 1)
     maxwell_stage_kernel(const __grid_constant__ CUtensorMap tmap, const MaxwellParams<Real> p) {
   using C = MaxwellCfg<Real, TY>;
   using G = Geo<Real, COORD>;
@@ -113,9 +108,6 @@ __global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, MINB)
   Real* fL = sm + C::OFF_FL;
   Real* fR = sm + C::OFF_FR;
   Real* fb = sm + C::OFF_FB;
-  Real* gst = sm + C::OFF_G;
-  constexpr bool STAGED = C::STAGED;
-  constexpr int NO = TX * TY;  // output threads
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + (C::BYTES - C::NSLOT * 8));
   if (p.active && !*p.active) return;
   if (smem_u32(smem_raw) & 127u) {
@@ -179,18 +171,11 @@ __global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, MINB)
       // barrier above, which every thread reaches only after its last read of
       // the previous step, so the steps need no barrier at their end.
       if (tid == 0 && K + HH + 1 <= Plast) issue(K + HH + 1);
-      // U0 and acc of this plane's output cells, fetched now so that the
-      // step hides their latency: copied into this thread's shared-memory
-      // slots (STAGED), or lane 0 of each row asks L2 for them
+      // U0 and acc of this plane's output cells: lane 0 of each row asks L2 for
+      // them now, so that the step hides their latency
       if (K >= Z0 && out_valid) {
         const long long g0 = L.idx(0, K, oj + 1, oi + 1);
-        if constexpr (STAGED) {
-#pragma unroll
-          for (int v = 0; v < NV; ++v) {
-            if (needs_u0<Real>(p.coef) && !p.coef.u0_is_input) cp_async4(&gst[v * NO + tid], p.u0 + g0 + v * L.var_stride);
-            if (needs_acc(p.coef)) cp_async4(&gst[(NV + v) * NO + tid], p.acc + g0 + v * L.var_stride);
-          }
-        } else if (otx == 0) {
+        if (otx == 0) {
           for (int v = 0; v < NV; ++v) {
             if (needs_u0<Real>(p.coef) && !p.coef.u0_is_input) prefetch_l2(p.u0 + g0 + v * L.var_stride);
             if (needs_acc(p.coef)) prefetch_l2(p.acc + g0 + v * L.var_stride);
@@ -219,27 +204,14 @@ __global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, MINB)
 #pragma unroll
             for (int f = 0; f < 2; ++f) {
               const int q0 = 3 * f;
-              Real d1, d2, d3;
-              if constexpr (sizeof(Real) == 4) {
-                d1 = (UA(uK1, q0, r, c + 1) - UA(uK1, q0, r, c - 1)) * (0.5f * inv_len<Real, COORD, 0>(p.met, i, j, k));
-                d2 = (UA(uK1, q0 + 1, r + 1, c) - UA(uK1, q0 + 1, r - 1, c)) * (0.5f * inv_len<Real, COORD, 1>(p.met, i, j, k));
-                d3 = (UA(uK2, q0 + 2, r, c) - UA(uK, q0 + 2, r, c)) * (0.5f * inv_len<Real, COORD, 2>(p.met, i, j, k));
-              } else {
-                d1 = by1(UA(uK1, q0, r, c + 1) - UA(uK1, q0, r, c - 1));
-                d2 = by2(UA(uK1, q0 + 1, r + 1, c) - UA(uK1, q0 + 1, r - 1, c));
-                d3 = by3(UA(uK2, q0 + 2, r, c) - UA(uK, q0 + 2, r, c));
-              }
+              const Real d1 = by1(UA(uK1, q0, r, c + 1) - UA(uK1, q0, r, c - 1));
+              const Real d2 = by2(UA(uK1, q0 + 1, r + 1, c) - UA(uK1, q0 + 1, r - 1, c));
+              const Real d3 = by3(UA(uK2, q0 + 2, r, c) - UA(uK, q0 + 2, r, c));
               Real dv = (d1 + d2) + d3;
               if constexpr (COORD != COORD_CART) {
-                if constexpr (sizeof(Real) == 4) {
-                  dv = ((dv + (UA(uK1, q0, r, c) * (lm.dl[0][1] + lm.dl[0][2])) * recip(lm.h[0])) +
-                        (UA(uK1, q0 + 1, r, c) * (lm.dl[1][0] + lm.dl[1][2])) * recip(lm.h[1])) +
-                       (UA(uK1, q0 + 2, r, c) * (lm.dl[2][0] + lm.dl[2][1])) * recip(lm.h[2]);
-                } else {
-                  dv = ((dv + ((UA(uK1, q0, r, c) * (lm.dl[0][1] + lm.dl[0][2])) / lm.h[0])) +
-                        ((UA(uK1, q0 + 1, r, c) * (lm.dl[1][0] + lm.dl[1][2])) / lm.h[1])) +
-                       ((UA(uK1, q0 + 2, r, c) * (lm.dl[2][0] + lm.dl[2][1])) / lm.h[2]);
-                }
+                dv = ((dv + ((UA(uK1, q0, r, c) * (lm.dl[0][1] + lm.dl[0][2])) / lm.h[0])) +
+                      ((UA(uK1, q0 + 1, r, c) * (lm.dl[1][0] + lm.dl[1][2])) / lm.h[1])) +
+                     ((UA(uK1, q0 + 2, r, c) * (lm.dl[2][0] + lm.dl[2][1])) / lm.h[2]);
               }
               div[f] = dv;
             }
@@ -385,20 +357,8 @@ __global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, MINB)
         const int im = max(oi - 1, 0) - oi, ip = min(oi + 1, nx - 1) - oi;
         const int jm = max(oj - 1, 0) - oj, jp = min(oj + 1, ny - 1) - oj;
         const int km = (K - 1 >= 1) ? -1 : 0, kp = (K + 1 <= nz) ? 1 : 0;
-        Real h1, h2, h3;  // 1/(2L) (float32) or 2L (float64)
-        if constexpr (sizeof(Real) == 4) {
-          h1 = 0.5f * inv_len<Real, COORD, 0>(p.met, oi, oj, kK);
-          h2 = 0.5f * inv_len<Real, COORD, 1>(p.met, oi, oj, kK);
-          h3 = 0.5f * inv_len<Real, COORD, 2>(p.met, oi, oj, kK);
-        } else {
-          h1 = Real(2) * G::L1(p.met, oi, oj, kK);
-          h2 = Real(2) * G::L2(p.met, oi, oj, kK);
-          h3 = Real(2) * G::L3(p.met, oi, oj, kK);
-        }
-        auto grad = [&](Real d, Real h) -> Real {
-          if constexpr (sizeof(Real) == 4) return d * h;
-          else return d / h;
-        };
+        const Real h1 = Real(2) * G::L1(p.met, oi, oj, kK), h2 = Real(2) * G::L2(p.met, oi, oj, kK);
+        const Real h3 = Real(2) * G::L3(p.met, oi, oj, kK);
         Real sc[NV];
 #pragma unroll
         for (int f = 0; f < 2; ++f) {
@@ -406,9 +366,9 @@ __global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, MINB)
           const Real* rb = rK + f * PL + r * W + c;
           const Real* rbp = (kp ? rK1 : rK) + f * PL + r * W + c;
           const Real* rbm = (km ? rKm : rK) + f * PL + r * W + c;
-          const Real g1 = grad(rb[ip] - rb[im], h1);
-          const Real g2 = grad(rb[jp * W] - rb[jm * W], h2);
-          const Real g3 = grad(rbp[0] - rbm[0], h3);
+          const Real g1 = (rb[ip] - rb[im]) / h1;
+          const Real g2 = (rb[jp * W] - rb[jm * W]) / h2;
+          const Real g3 = (rbp[0] - rbm[0]) / h3;
           sc[3 * f + 0] = (-chi) * g1;
           sc[3 * f + 1] = (-chi) * g2;
           sc[3 * f + 2] = (-chi) * g3;
@@ -428,17 +388,11 @@ __global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, MINB)
           kv[v] = by_V(-sum) + ((sg[v] + sp) + sc[v]);
         }
         Real u0v[NV], accv[NV];
-        if constexpr (STAGED) cp_async_wait_all();
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
           const long long gi = gidx + (long long)v * L.var_stride;
-          if constexpr (STAGED) {
-            u0v[v] = needs_u0<Real>(p.coef) ? (p.coef.u0_is_input ? q[v] : gst[v * NO + tid]) : Real(0);
-            accv[v] = needs_acc(p.coef) ? gst[(NV + v) * NO + tid] : Real(0);
-          } else {
-            u0v[v] = needs_u0<Real>(p.coef) ? (p.coef.u0_is_input ? q[v] : p.u0[gi]) : Real(0);
-            accv[v] = needs_acc(p.coef) ? p.acc[gi] : Real(0);
-          }
+          u0v[v] = needs_u0<Real>(p.coef) ? (p.coef.u0_is_input ? q[v] : p.u0[gi]) : Real(0);
+          accv[v] = needs_acc(p.coef) ? p.acc[gi] : Real(0);
         }
         unsigned bad = 0;
 #pragma unroll
@@ -454,7 +408,6 @@ __global__ void __launch_bounds__(MaxwellCfg<Real, TY>::NT, MINB)
     }
     __syncthreads();  // the next tile's first loads reuse every ring slot
   }
-  if constexpr (STAGED) cp_async_wait_all();  // none left in flight at exit
   if (!ok && tid == 0)
     for (int s = 0; s < C::NSLOT; ++s)
       if ((pending >> s) & 1u) mbar_wait_bounded(&bars[s], (phase_bits >> s) & 1u, p.drain_ns);
