@@ -21,8 +21,10 @@ constexpr int MIX_NT = 160;
 constexpr int MIX_NBAR = 7;
 // Relative cost of a unit in the balanced split of the launch: a Navier-Stokes
 // plane (or row tile) of 32 x 8 cells against a heat plane of 32 x 20 (or 32 x
-// 10).  Of 64 + 32 grids (12,275 and 40,085 units) the first alone take 106 us a
-// stage, the others alone 122: 2.8 to 1 per unit.
+// 10).  Alone, warm-up included, a unit kept a block busy for 3.95 us (one-plane
+// 256^2 grids), 4.1 to 4.5 (128^3, 64^3, 96x96x32) and 1.48 (cylindrical heat
+// 96x160x48): 2.7 to 3.1 to 1.  (5:2 ran a batch of 64 + 32 grids at 1195 us a step,
+// 3:1 at 1178, 7:2 at 1197.)
 constexpr int MIX_NS_COST = 6, MIX_HEAT_COST = 2, MIX_HEAT_COST_ALT = 1;
 constexpr int MIX_NS_TY = MIX_NS_R * MIX_NS_NW, MIX_HEAT_TY = 4 * MIX_HEAT_NW, MIX_HEAT_TY_ALT = 2 * MIX_HEAT_NW;
 static_assert(NsStripCfg<MIX_NS_R, MIX_NS_NW>::NT == MIX_NT && HeatPcCfg<4, MIX_HEAT_NW>::NT == MIX_NT,
@@ -102,10 +104,10 @@ __global__ void __launch_bounds__(MIX_NT, 3) batch_mixed_kernel(const __grid_con
         reinterpret_cast<unsigned char*>(&ns)[q] = reinterpret_cast<const unsigned char*>(&in.ns)[q];
       __syncthreads();
       if (ns.flat)
-        ok = ns_strip_tile<LIM, RIEM, MIX_NS_R, MIX_NS_NW, COORD_CART, true>(
+        ok = ns_strip_tile<LIM, RIEM, MIX_NS_R, MIX_NS_NW, COORD_CART, true, false>(
             ns, &in.tmap, &in.u0map, &in.accmap, pc, smem_raw, bars, bars + 6, 6, phase_bits, pending);
       else
-        ok = ns_strip_tile<LIM, RIEM, MIX_NS_R, MIX_NS_NW, COORD_CART, false>(
+        ok = ns_strip_tile<LIM, RIEM, MIX_NS_R, MIX_NS_NW, COORD_CART, false, false>(
             ns, &in.tmap, &in.u0map, &in.accmap, pc, smem_raw, bars, bars + 6, 6, phase_bits, pending);
     } else {
       if (in.heat.active && !*in.heat.active) continue;

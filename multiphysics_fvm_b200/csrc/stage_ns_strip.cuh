@@ -189,16 +189,16 @@ __device__ __forceinline__ F2 strip_state2(F2 h, F2 s, F2 q) {
   if constexpr (LIM == LIM_PC) return q;
   else return fma2(h, s, q);
 }
-template <int D, int RIEM>
+template <int D, int RIEM, bool EARLY>
 __device__ __forceinline__ void strip_flux2(const F2* qL, const F2* qR, float gam, F2* F) {
   const F2 g2(gam);
   const F2 irL(rcp_approx(qL[0].lo()), rcp_approx(qL[0].hi())), irR(rcp_approx(qR[0].lo()), rcp_approx(qR[0].hi()));
   const F2 vL = qL[1 + D] * irL, vR = qR[1 + D] * irR;
-  // flux of the normal momentum; formed before the wave speeds for HLL (256^3 stage
-  // 542 us, 563 where it is used), where it is used for Rusanov (533, so 558)
+  // flux of the normal momentum: formed before the wave speeds (EARLY) or where it
+  // is used, as the kernel's registers and schedule like it (ns_strip_kernel)
   auto normal = [](const F2* q, F2 v) { return fma2(v, q[1 + D], q[5]); };
   F2 nL, nR;
-  if constexpr (RIEM == RIEM_HLL) nL = normal(qL, vL), nR = normal(qR, vR);
+  if constexpr (EARLY) nL = normal(qL, vL), nR = normal(qR, vR);
   const F2 c2L = (g2 * qL[5]) * irL, c2R = (g2 * qR[5]) * irR;
   const F2 cL(sqrt_approx(c2L.lo()), sqrt_approx(c2L.hi())), cR(sqrt_approx(c2R.lo()), sqrt_approx(c2R.hi()));
   // c below is -c of strip_combine, with the states' difference turned round
@@ -223,7 +223,7 @@ __device__ __forceinline__ void strip_flux2(const F2* qL, const F2* qR, float ga
 #pragma unroll
   for (int k = 1; k < 4; ++k) {
     if (k == 1 + D) {
-      if constexpr (RIEM != RIEM_HLL) nL = normal(qL, vL), nR = normal(qR, vR);
+      if constexpr (!EARLY) nL = normal(qL, vL), nR = normal(qR, vR);
       F[k] = fma2(a, nL, fma2(b, nR, c * (qL[k] - qR[k])));
     } else {
       F[k] = fma2(av, qL[k], fma2(bv, qR[k], c * (qL[k] - qR[k])));
@@ -275,7 +275,7 @@ __device__ __forceinline__ void curvilinear_source(const ColMetric<COORD>& cm, c
 // barriers (indices 0..2, phase bits 0..2), `gbar` the staged-tile barrier with
 // phase bit `gbit`; `phase_bits` and `pending` carry over from tile to tile.
 // Returns false when a wait ran out: the block must stop and drain.
-template <int LIM, int RIEM, int R, int NW, int COORD, bool flat>
+template <int LIM, int RIEM, int R, int NW, int COORD, bool flat, bool EARLY>
 __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CUtensorMap* tmap,
                                               const CUtensorMap* u0map, const CUtensorMap* accmap, const Piece& pc,
                                               unsigned char* smem_raw, uint64_t* bars, uint64_t* gbar, int gbit,
@@ -497,7 +497,7 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
               qlx[f] = strip_state2<LIM>(F2(HS), lane == 0 ? F2(h[0], h[1]) : F2(ua, ub), fm);
               qrx[f] = strip_state2<LIM>(hx, s1, f0);
             }
-            strip_flux2<0, RIEM>(qlx, qrx, gam, F);
+            strip_flux2<0, RIEM, EARLY>(qlx, qrx, gam, F);
 #pragma unroll
             for (int v = 0; v < 5; ++v) {
               const float da = __shfl_down_sync(0xffffffffu, F[v].lo(), 1), db = __shfl_down_sync(0xffffffffu, F[v].hi(), 1);
@@ -531,7 +531,7 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
               ql1[f] = fmaf(hy[2], s[2], g[3]);
               qr1[f] = fmaf(-hy[3], s[3], g[4]);
             }
-            strip_flux2<1, RIEM>(ql, qr, gam, F);
+            strip_flux2<1, RIEM, EARLY>(ql, qr, gam, F);
             strip_flux<1, RIEM>(ql1, qr1, gam, F1);
             const int ja = min(jb, ny - 1), jc = min(jb + 1, ny - 1);
             const F2 lower(-cm.a2(p.met, ja, ja), -cm.a2(p.met, jc, jc));
@@ -595,7 +595,7 @@ __device__ __forceinline__ bool ns_strip_tile(const NsParams<float>& p, const CU
           }
           if (zface) {
             F2 F[5];
-            strip_flux2<2, RIEM>(qlz, qr, gam, F);
+            strip_flux2<2, RIEM, EARLY>(qlz, qr, gam, F);
             const F2 a3(cm.a3(p.met, min(y0 + ty, ny - 1), idz), cm.a3(p.met, min(y0 + ty + 1, ny - 1), idz));
 #pragma unroll
             for (int v = 0; v < 5; ++v) {
@@ -715,6 +715,10 @@ template <int LIM, int RIEM, int R, int NW, int MINB, int COORD, bool FLAT>
 __global__ void __launch_bounds__(NsStripCfg<R, NW>::NT, MINB)
     ns_strip_kernel(const __grid_constant__ NsStripSource src) {
   using C = NsStripCfg<R, NW>;
+  // where strip_flux2 forms its normal flux, by what was measured: 256^3 HLL stage
+  // 542 us early, 563 late, Rusanov 558 and 533, the one-plane march the same, grids
+  // of 128^3 in the mixed-batch kernel 314 and 302
+  constexpr bool EARLY = RIEM == RIEM_HLL && !FLAT;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + C::BAR_BYTES);
   const NsParams<float>& p = src.p;
@@ -740,8 +744,8 @@ __global__ void __launch_bounds__(NsStripCfg<R, NW>::NT, MINB)
   int inst;
   bool ok = true;
   while (ok && walk.next(grid, inst, pc))
-    ok = ns_strip_tile<LIM, RIEM, R, NW, COORD, FLAT>(p, &src.tmap, &src.u0map, &src.accmap, pc, smem_raw, bars,
-                                                      bars + C::NSLOT, C::NSLOT, phase_bits, pending);
+    ok = ns_strip_tile<LIM, RIEM, R, NW, COORD, FLAT, EARLY>(p, &src.tmap, &src.u0map, &src.accmap, pc, smem_raw, bars,
+                                                             bars + C::NSLOT, C::NSLOT, phase_bits, pending);
   // On a timeout, wait (bounded) for every copy this block may still have in flight.
   if (!ok && tid == 0) {
     for (int s = 0; s < C::NBAR; ++s)
