@@ -12,10 +12,18 @@
 // column boundary is two pieces.  Fixed depth (> 0): pieces of `zchunk` units
 // dealt round-robin, ceil(pieces / blocks) rounds: a 256^3 grid in 64-plane
 // pieces fills 2.3 rounds of 444 resident blocks and takes 3, and a 97x130x61
-// one occupies 68 blocks.  Measured stage launches, fixed 64 -> balanced:
-// inviscid NS 256^3 811 -> 715 us and 97x130x61 342 -> 95, viscous cylindrical
-// 96x128x64 437 -> 147, Maxwell 128x128x256 395 -> 291, heat 192x256x128
-// 89 -> 38, viscous 256^3 1547 -> 1497, 64x64x1 17.2 -> 6.6.
+// one occupies 68 blocks.  Measured stage launches, fixed 64 -> balanced, when the
+// split was introduced: inviscid NS 256^3 811 -> 715 us and 97x130x61 342 -> 95,
+// viscous cylindrical 96x128x64 437 -> 147, Maxwell 128x128x256 395 -> 291, heat
+// 192x256x128 89 -> 38, viscous 256^3 1547 -> 1497, 64x64x1 17.2 -> 6.6.
+//
+// What the balanced split costs: the warm-up is not counted, so a block whose run
+// crosses a column boundary pays it twice (two planes of a run of 9 at 97x130x61);
+// and neighbouring columns are marched at different heights, so a tile's halo is
+// seldom still in L2.  At 192^3 the launches moved 1.71 (inviscid) and 2.65
+// (viscous) times the algorithmic bytes, 1.07 and 1.10 in equal chunks.  Bandwidth
+// does not bound those kernels, but a sweep over depths finds what is left: 256^3
+// inviscid 543 us a stage, 508 at depth 48.
 #pragma once
 #include "fvm_common.cuh"
 
