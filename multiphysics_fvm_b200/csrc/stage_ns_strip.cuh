@@ -100,7 +100,7 @@ __device__ __forceinline__ float min_xorsign(float a, float b) {
 // eleven instructions, a select per slope, flux vectors formed per state and
 // float64 stage constants converted per cell, the stage launches took 717 us
 // (inviscid 256^3), 1497 (viscous 256^3), 95 (97x130x61, three-sign limiter) and
-// 291 (Maxwell 128x128x256); in this form 600, 1291, 54 and 200 (541, 1108, 48 and
+// 291 (Maxwell 128x128x256); in this form 600, 1291, 54 and 200 (542, 1092, 48 and
 // 186 with what the comments at strip_slope2, the flat march, the viscous and the
 // Maxwell kernel say).
 template <int LIM>
