@@ -319,7 +319,8 @@ class Simulation:
         return z.value, ms.value
 
     def tiling(self):
-        """(tile rows, z-march depth) the stage kernels run with."""
+        """(tile rows, z-march depth) the stage kernels run with; of the balanced
+        split (depth 0), the depth to ask for that comes nearest to it."""
         ty, z = C.c_int(), C.c_int()
         L.check(self._lib.fvm_tiling(self._h, C.byref(ty), C.byref(z)), "fvm_tiling")
         return ty.value, z.value
