@@ -187,11 +187,11 @@ int fvm_step_launches(fvm_handle* h, int dt_mode, int* launches);
 int fvm_profile_steps(fvm_handle* h, int n_steps, int dt_mode, double* stage_kernel_ms,
                       double* other_kernel_ms, int* stage_launches);
 
-/* Pick the block shape -- tile rows (the default and, for float32
- * navier_stokes and heat, a 4-row tile) and the z-march depth (planes per
- * tile) -- by timing every pair on this grid; the state and clock are restored
- * afterwards.  A batch member keeps its tile rows, which are its batch's.  New:
- * the reference has no tuning. */
+/* Pick the block shape -- tile rows (the default and, for float32 grids, a second
+ * height) and the z-march depth (planes per tile; the balanced split is one of
+ * them) -- by timing every pair on this grid; the state and clock are restored
+ * afterwards.  best_zchunk: as fvm_tiling reports it.  A batch member keeps its tile
+ * rows, which are its batch's.  New: the reference has no tuning. */
 int fvm_autotune(fvm_handle* h, int* best_zchunk, double* best_ms_per_step);
 /* The handle's block shape: tile rows (fvm_desc.tile_ty, or the autotuner's
  * choice) and z-march depth (of the balanced split, the depth to ask for that comes
